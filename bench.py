@@ -493,8 +493,8 @@ def main():
     # The contraction (k_cmap, the row sorts of every size class on several
     # streams, the count scan and the copy; CUDA events on the caller's
     # stream bracket each stage) is the larger part of the step; the matching
-    # (k_match_prep, k_match_first, the round kernel k_match, k_match_finish)
-    # is reported beside it in config.stage_roofline.
+    # (k_match_prep, k_match_first, k_match_propose, k_match_rounds,
+    # k_match_finish) is reported beside it in config.stage_roofline.
     peak, peak_kind = measured_peaks()
     lb = level_bytes(sizes)
     n0, m0 = sizes[0]
@@ -528,7 +528,7 @@ def main():
         ach = per_launch_bytes / (per_launch_ms / 1e3) / 1e9
         label = {"contraction": "contraction (k_cmap, k_tiny_units, k_class_rows, k_long_sort/merge/dedup, "
                                 "k_count_scan, k_copy_rows, k_copy_class_rows, k_long_copy)",
-                 "k_match": "k_match (with k_match_prep, k_match_first, k_match_finish)"}[dom]
+                 "k_match": "matching (k_match_prep, k_match_first, k_match_propose, k_match_rounds, k_match_finish)"}[dom]
         roof = {"kernel": label, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                 "frac": ach / peak, "peak_kind": peak_kind, "traffic": traffic if dom == "contraction" else None,
                 "bytes_per_launch": per_launch_bytes, "ms_per_launch": per_launch_ms}

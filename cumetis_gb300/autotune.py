@@ -29,10 +29,9 @@ ROOT = os.path.dirname(B.HERE)
 PARAMS = [
     ("CM_SERIAL_DEG", 16, [8, 16], "cm_match.cu"),          # rows scanned by one lane (warp-per-vertex threshold)
     ("CM_MATCH_CHUNK", 256, [128, 256, 512], "cm_match.cu"),  # entries per warp work item
-    ("CM_FIRST_MINBLOCKS", 8, [4, 6, 8], "cm_match.cu"),     # first-round kernel: blocks per SM (register cap)
-    ("CM_FIRST_KEEP_SHORT", 2, [1, 2, 4], "cm_match.cu"),    # candidates the first round keeps (lane rows)
-    ("CM_FIRST_KEEP_CHUNK", 2, [1, 2, 4], "cm_match.cu"),    # ... and per chunked row
-    ("CM_TAIL_ITEMS", 4096, [1024, 4096, 16384], "cm_match.cu"),  # rounds this small run in one block
+    ("CM_FIRST_MINBLOCKS", 8, [4, 6, 8], "cm_match.cu"),     # list kernel: blocks per SM (register cap)
+    ("CM_FIRST_KEEP_CHUNK", 4, [1, 2, 4], "cm_match.cu"),    # candidates listed for rows above CM_SERIAL_DEG
+    ("CM_TAIL_CHUNKS", 64, [32, 64, 256], "cm_match.cu"),    # rounds of this few chunks run in one block
     ("CM_TINY_MAX", 64, [16, 32, 64], "cm_contract.cu"),    # rows sorted in one-warp batches; larger rows by size class
     ("CM_CHUNK", 16384, [8192, 16384], "cm_contract.cu"),    # huge-row segment (chunk) size
     ("CM_CHUNK_THREADS", 1024, [512, 1024], "cm_contract.cu"),  # threads sorting one chunk

@@ -325,7 +325,8 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
     return release(rc);
   int32_t *sizes = (int32_t *)ws_take(ctx_, 64);
   const size_t ws_mark = ctx_->ws_used;
-  if ((rc = launch_match(ctx_, &U, min_cap, active_[grp[0]].p.match_mode, match, s, vgid, d_vbase, d_gcap)))
+  if ((rc = launch_match(ctx_, &U, min_cap, active_[grp[0]].p.match_mode, match, s, vgid, d_vbase, d_gcap,
+                         row_bound / 2)))
     return release(rc);
   ctx_->ws_used = ws_mark;
   if ((rc = launch_contract(ctx_, &U, match, cmap, &C, sizes, s, row_bound))) return release(rc);

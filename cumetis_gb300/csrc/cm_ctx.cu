@@ -493,7 +493,8 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
     cm_level C;
     if ((rc = alloc_level(C, n, m, ctx->pool, s))) return fail(rc);
     ctx->ws_used = level_ws_off;
-    if ((rc = launch_match(ctx, &F.g, h->maxvwgt, params->match_mode, F.match, s))) {
+    if ((rc = launch_match(ctx, &F.g, h->maxvwgt, params->match_mode, F.match, s, nullptr, nullptr, nullptr,
+                           row_bound / 2))) {
       cudaFreeAsync(C.block, s);
       return fail(rc);
     }

@@ -143,10 +143,11 @@ size_t contract_ws_bytes(int64_t n, int64_t m);
 // Stage launchers shared between entry points (no argument checking).
 // vgid/gbase/gcap (optional): several graphs side by side -- vertex v belongs
 // to graph vgid[v], whose first vertex is gbase[g] and whose weight cap is
-// gcap[g]; maxvwgt is then the smallest cap.
+// gcap[g]; maxvwgt is then the smallest cap.  max_deg: an upper bound of the
+// longest row (INT64_MAX when unknown); kernels for longer rows are not launched.
 int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, int32_t *d_match,
                  cudaStream_t s, const int32_t *vgid = nullptr, const int32_t *gbase = nullptr,
-                 const int32_t *gcap = nullptr);
+                 const int32_t *gcap = nullptr, int64_t max_deg = INT64_MAX);
 // Rows of more than long_threshold expanded entries are listed: up to
 // long_chunk entries by size class (class_offset(m, long_threshold, k) of
 // class_list, counts in class_ctr[k]), longer ones as chunked rows.

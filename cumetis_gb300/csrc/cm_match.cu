@@ -6,30 +6,42 @@
 // (1621).  Eligibility follows cuda_shem2: a pair (v,k) may match if
 // vwgt[v]+vwgt[k] <= maxvwgt and one end is light (3*vwgt < maxvwgt).
 //
-// Rule: every vertex prefers its heaviest eligible unmatched neighbour, ties
-// to the lower vertex id (CM_MATCH_HEM) or to the lower edge hash
-// (CM_MATCH_HEM_HASH, then lower id).  Both orders are strict total orders on
-// edges, so mutual-proposal rounds converge to the unique greedy matching of
-// that order whatever the schedule.
+// Rule: every vertex prefers its heaviest eligible neighbour, ties to the lower
+// vertex id (CM_MATCH_HEM) or to the lower edge hash (CM_MATCH_HEM_HASH, then
+// lower id).  Both orders are strict total orders on edges, so the greedy
+// matching of the order is unique, and any schedule of proposals that ends in
+// the stable state finds it.
 //
-// k_match_prep initialises the state, k_match_first runs the first round's
-// scans at high occupancy, and one persistent cooperative kernel (1024-thread
-// blocks, at most one per SM) runs the rounds; a round has three phases
-// separated by grid barriers (block barriers once a round fits one block, the
-// tail mode), and k_match_finish makes the unmatched vertices singletons:
-//   A  full scans: every vertex in the round's scan list computes its kTop
-//      best eligible unmatched candidates (cached) and points at the first.
-//      Rows of <= kSerialDeg entries: one lane each; longer rows: kChunk-entry
-//      chunks, one warp each, the last chunk of a row merging the chunk lists.
-//   B  commits: a vertex whose pointer changed this round (scanned, or updated
-//      from its cache) and whose target points back forms a pair.
-//   C  filter of the active list (unmatched vertices with a candidate): a
-//      vertex whose target got matched takes the next unmatched entry of its
-//      cached list (candidates only disappear and eligibility is fixed, so the
-//      cached order stays exact); only an exhausted, incomplete cache sends it
-//      back to phase A for a full scan.
-// m2[v] < 0 encodes "unmatched, vwgt = -1 - m2[v]": one 4-byte gather per
-// neighbour answers both "matched?" and the weight cap.
+// Proposals (the Suitor scheme of Manne and Halappanavar): best[u] is the best
+// proposal u has received; a free vertex offers itself to its most preferred
+// neighbour whose best[] it beats, and the vertex it displaces there becomes
+// free and goes on with its own next candidate.  best[u] only improves, so a
+// rejected candidate never has to be looked at again, and no vertex state is
+// read beside best[]: there are no rounds of propose / commit / filter.  When
+// nobody is free, best[u] = v and best[v] = u for every matched pair.
+//
+//   k_match_prep     zeroes best[], finds the largest vertex weight, lists the
+//                    chunks of rows longer than kSerialDeg, and gives the
+//                    vertices of shorter rows their kTop most preferred
+//                    neighbours, from weights alone.
+//   k_match_first    the same for the longer rows, kFirstKeepChunk neighbours.
+//                    The lists are not written again, so the later kernels read
+//                    them without ordering.
+//   k_match_propose  one thread a vertex follows the chain of displacements
+//                    that its vertex's offer starts: per step one list read and
+//                    one atomic.  A short row whose list is used up is rescanned
+//                    by the thread; a longer one is queued.
+//   k_match_rounds   queued rows, one warp per row of up to kChunk entries, the
+//                    warp following the chain; rows of several chunks are merged
+//                    by the last chunk's warp, and a displaced one is queued for
+//                    the next round (grid barrier; a round with few chunks runs
+//                    on one block).
+//   k_match_finish   match[v] = the partner, or v.
+//
+// Only an adjacency that is not symmetric can end with an offer that is not
+// returned (best[u] = v, best[v] != u).  k_match_finish sees that and the
+// matching is then computed again by handshakes (handshake_rounds), whose
+// result is defined for such inputs too.
 #include <climits>
 
 #include <algorithm>
@@ -39,8 +51,8 @@
 namespace cm {
 namespace {
 
-// Threads per block of the persistent round kernel and the blocks per SM it
-// is compiled for (its grid is every resident block, up to the graph's need).
+// Threads per block of the round kernel and the blocks per SM it is compiled
+// for (its grid is every resident block, up to the graph's need).
 #ifndef CM_MATCH_THREADS
 #define CM_MATCH_THREADS 1024
 #endif
@@ -61,51 +73,42 @@ constexpr int kSerialDeg = CM_SERIAL_DEG;
 constexpr int kChunk = CM_MATCH_CHUNK;
 static_assert(kSerialDeg == 8 || kSerialDeg == 16, "CM_SERIAL_DEG: 8 or 16");
 static_assert(kChunk == 128 || kChunk == 256 || kChunk == 512, "CM_MATCH_CHUNK: 128, 256 or 512");
-constexpr int kTop = 4;          // cached candidates per vertex
+constexpr int kTop = 4;          // listed candidates per vertex
 // Tail mode (one block runs the remaining rounds) once a round has at most
-// kTailItems vertices to scan, commit or filter and kTailChunks row chunks.
-#ifndef CM_TAIL_ITEMS
-#define CM_TAIL_ITEMS 4096
-#endif
+// kTailChunks row chunks.
 #ifndef CM_TAIL_CHUNKS
 #define CM_TAIL_CHUNKS 64
 #endif
-constexpr long long kTailItems = CM_TAIL_ITEMS;
 constexpr int kTailChunks = CM_TAIL_CHUNKS;
-constexpr int kNotScanned = -2;  // top[v*kTop] before the first scan
-constexpr int kUnknown = -3;     // cache slot not computed (the first scan keeps only the best)
-// Candidates the first-round scans keep when every edge is eligible: short
-// rows (one lane each) and chunked rows.  1 keeps only the best (later
-// rescans fill the cache); kTop fills the cache at once.
-#ifndef CM_FIRST_KEEP_SHORT
-#define CM_FIRST_KEEP_SHORT 2
-#endif
+constexpr int kNone = -1;        // list slot: no further candidate
+constexpr int kUnknown = -3;     // list slot not computed (more candidates may exist)
+// Candidates listed for rows of more than kSerialDeg entries (short rows: kTop).
 #ifndef CM_FIRST_KEEP_CHUNK
-#define CM_FIRST_KEEP_CHUNK 2
+#define CM_FIRST_KEEP_CHUNK 4
 #endif
-constexpr int kFirstKeepShort = CM_FIRST_KEEP_SHORT, kFirstKeepChunk = CM_FIRST_KEEP_CHUNK;
+constexpr int kFirstKeepChunk = CM_FIRST_KEEP_CHUNK;
+static_assert(kFirstKeepChunk >= 1 && kFirstKeepChunk <= kTop, "CM_FIRST_KEEP_CHUNK: 1 to 4");
 
-struct Slot {      // lists feeding one round (double-buffered by round parity)
-  int *small;      // full scans, rows <= kSerialDeg
-  int *big_v, *big_base, *big_done;  // full scans, longer rows: vertex, first chunk, chunks done
+struct Slot {      // rows to scan in one round
+  int *big_base, *big_done;  // per row: first chunk, chunks done
   int4 *desc;      // per chunk: (vertex, first entry, end entry, row index or -1 if one chunk)
-  int *upd;        // pointers already updated from the cache
-  int *act;        // active list for the round's phase C
 };
 
 struct MatchArgs {
-  int n;
+  int n, span;                   // span: vertices a warp takes at a time (multiple of 32, at most kSpan)
   const int *xadj, *adjncy, *adjwgt, *vwgt;
   long long maxvwgt;
   int mode;
-  int *m2, *ptr, *stamp, *top;
+  int *m2;                       // the matching (output)
+  unsigned long long *best;      // best proposal received: (weight, proposer), 0 = none (best_key)
+  int *top, *topw;               // kTop listed candidates per vertex: ids, weights
   Slot slot[2];
-  int *nsmall, *nupd, *nact;     // [2] each
-  unsigned long long *big;       // [2] = (rows << 32 | chunks)
+  unsigned long long *big;       // [3] = (rows << 32 | chunks) of the slots, by round
+  int *tick;                     // [3] work tickets of the round kernel, by round
   int *vmax;                     // largest vertex weight (zeroed before the launch)
-  int *tick;                     // [2 slots][phase A chunks, phase C spans] work tickets
+  int *odd;                      // [2]: an offer was not returned; blocks of k_match_finish done
   int *part;                     // per chunk: kTop x (w, h, k)
-  int max_rounds;
+  long long max_rounds;
   DevStatus *st;
   unsigned long long *trace;     // optional: row 0 header, row r+1 = round r
   int trace_rows;
@@ -117,8 +120,8 @@ struct MatchArgs {
 };
 
 // Candidates.  Lex mode (ties to the lower id) packs (weight, ~id) into one
-// 64-bit key, larger = better, 0 = none.  Hash mode compares (weight desc,
-// edge hash asc, id asc) field by field.
+// 64-bit key, larger = better, 0 = none.  Hash mode has (weight desc, edge hash
+// asc) in the key and the id, which decides between equal keys, beside it.
 template <bool H> struct Cand;
 template <> struct Cand<false> {
   unsigned long long key = 0ull;
@@ -131,6 +134,7 @@ template <> struct Cand<false> {
   }
   __device__ __forceinline__ bool valid() const { return key != 0ull; }
   __device__ __forceinline__ int id() const { return valid() ? (int)~(unsigned)key : -1; }
+  __device__ __forceinline__ int weight() const { return (int)((unsigned)(key >> 32) ^ 0x80000000u); }
   __device__ __forceinline__ bool better(const Cand &o) const { return key > o.key; }
   __device__ __forceinline__ bool same(const Cand &o) const { return key == o.key; }
   __device__ __forceinline__ Cand warp_best() const {
@@ -149,45 +153,37 @@ template <> struct Cand<false> {
   }
 };
 template <> struct Cand<true> {
-  int w = 0;
-  unsigned h = 0u;
-  int k = INT_MAX;  // INT_MAX = none
+  unsigned long long key = 0ull;  // (weight, ~hash), larger = better
+  int k = INT_MAX;                // INT_MAX = none
   __device__ __forceinline__ static Cand make(int v, int k, int w, int hb) {
     Cand c;
-    c.w = w;
+    const unsigned h = edge_hash((unsigned)(min(v, k) - hb), (unsigned)(max(v, k) - hb));
+    c.key = ((unsigned long long)((unsigned)w ^ 0x80000000u) << 32) | (unsigned)~h;
     c.k = k;
-    c.h = edge_hash((unsigned)(min(v, k) - hb), (unsigned)(max(v, k) - hb));
     return c;
   }
   __device__ __forceinline__ bool valid() const { return k != INT_MAX; }
   __device__ __forceinline__ int id() const { return valid() ? k : -1; }
-  __device__ __forceinline__ bool better(const Cand &o) const {
-    if (k == INT_MAX) return false;
-    if (o.k == INT_MAX) return true;
-    if (w != o.w) return w > o.w;
-    if (h != o.h) return h < o.h;
-    return k < o.k;
-  }
-  __device__ __forceinline__ bool same(const Cand &o) const { return k == o.k && w == o.w && h == o.h; }
+  __device__ __forceinline__ int weight() const { return (int)((unsigned)(key >> 32) ^ 0x80000000u); }
+  __device__ __forceinline__ bool better(const Cand &o) const { return key > o.key || (key == o.key && k < o.k); }
+  __device__ __forceinline__ bool same(const Cand &o) const { return key == o.key && k == o.k; }
   __device__ __forceinline__ Cand warp_best() const {
     const unsigned full = 0xffffffffu;
-    const int wmax = __reduce_max_sync(full, valid() ? w : INT_MIN);
-    const bool atw = valid() && w == wmax;
-    const unsigned hmin = __reduce_min_sync(full, atw ? h : 0xffffffffu);
-    const bool ath = atw && h == hmin;
-    const unsigned kmin = __reduce_min_sync(full, ath ? (unsigned)k : 0xffffffffu);
+    const unsigned hi = __reduce_max_sync(full, (unsigned)(key >> 32));
+    const bool top = (unsigned)(key >> 32) == hi;
+    const unsigned lo = __reduce_max_sync(full, top ? (unsigned)key : 0u);
     Cand r;
-    r.w = wmax;
-    r.h = hmin;
-    r.k = kmin == 0xffffffffu ? INT_MAX : (int)kmin;
+    r.key = ((unsigned long long)hi << 32) | lo;
+    r.k = __reduce_min_sync(full, key == r.key ? k : INT_MAX);
     return r;
   }
-  __device__ __forceinline__ void store(int *p) const { *reinterpret_cast<int4 *>(p) = make_int4(w, (int)h, k, 0); }
+  __device__ __forceinline__ void store(int *p) const {
+    *reinterpret_cast<int4 *>(p) = make_int4((int)(unsigned)(key >> 32), (int)(unsigned)key, k, 0);
+  }
   __device__ __forceinline__ static Cand load(const int *p) {
     const int4 x = __ldcg(reinterpret_cast<const int4 *>(p));
     Cand c;
-    c.w = x.x;
-    c.h = (unsigned)x.y;
+    c.key = ((unsigned long long)(unsigned)x.x << 32) | (unsigned)x.y;
     c.k = x.z;
     return c;
   }
@@ -212,7 +208,7 @@ struct TopK {
   // hb: the first vertex of v's graph (0 for one graph).
   __device__ __forceinline__ void insert_edge(int v, int k, int w, int hb) {
     if constexpr (H) {
-      if (c[KK - 1].valid() && w < c[KK - 1].w) return;
+      if (c[KK - 1].valid() && w < c[KK - 1].weight()) return;
     }
     insert(Cand<H>::make(v, k, w, hb));
   }
@@ -224,13 +220,63 @@ __device__ __forceinline__ long long weight_cap(const MatchArgs &a, int v) {
   return a.vgid ? (long long)__ldg(a.gcap + __ldg(a.vgid + v)) : a.maxvwgt;
 }
 
+// The pair (v, k) may match: both fit the cap and one of them is light.
+__device__ __forceinline__ bool pair_fits(long long cap, long long vw, long long vk) {
+  return vw + vk <= cap && (3 * vw < cap || 3 * vk < cap);
+}
+
+// Even the two heaviest vertices may pair and are light: every edge is
+// eligible, and the scans skip the neighbours' weights.
+__device__ __forceinline__ bool all_eligible(const MatchArgs &a) {
+  const long long vmax = __ldcg(a.vmax);
+  return 2 * vmax <= a.maxvwgt && 3 * vmax < a.maxvwgt;
+}
+
+// A proposal by v over an edge of weight w, as best[] holds it: 0 is none (the
+// low half, ~v, is never 0).  Between different weights, and among equal
+// weights with ties to the lower id, the larger key is the better proposal.
+__device__ __forceinline__ unsigned long long best_key(int v, int w) {
+  return ((unsigned long long)((unsigned)w ^ 0x80000000u) << 32) | (unsigned)~(unsigned)v;
+}
+__device__ __forceinline__ int best_holder(unsigned long long b) { return b == 0ull ? -1 : (int)~(unsigned)b; }
+__device__ __forceinline__ unsigned long long ld_best(const MatchArgs &a, int k) { return __ldcg(a.best + k); }
+
+// v's proposal (key) to c beats the proposal b that c holds.
 template <bool H>
-__device__ __forceinline__ bool eligible(const MatchArgs &a, long long vw, int v, int k, int s) {
-  if (k == v || s >= 0) return false;  // self or matched
-  const long long vk = -1ll - s;
-  const long long cap = weight_cap(a, v);
-  if (vw + vk > cap) return false;
-  return 3 * vw < cap || 3 * vk < cap;
+__device__ __forceinline__ bool beats(unsigned long long key, unsigned long long b, int v, int c, int hb) {
+  if constexpr (H) {
+    if (b == 0ull) return true;
+    if ((key >> 32) != (b >> 32)) return key > b;
+    const int s = best_holder(b);
+    const unsigned hv = edge_hash((unsigned)(min(v, c) - hb), (unsigned)(max(v, c) - hb));
+    const unsigned hs = edge_hash((unsigned)(min(s, c) - hb), (unsigned)(max(s, c) - hb));
+    return hv != hs ? hv < hs : v < s;
+  } else {
+    return key > b;
+  }
+}
+
+// v offers itself to c over an edge of weight w.  Returns whether c took it;
+// *out = the vertex c gave up for it (-1: none).  `seen`: a recent value of
+// best[c] (any value is allowed; a right one saves a memory trip).
+template <bool H>
+__device__ __forceinline__ bool offer(const MatchArgs &a, int v, int c, int w, unsigned long long seen, int hb,
+                                      int *out) {
+  const unsigned long long key = best_key(v, w);
+  if constexpr (H) {
+    for (;;) {  // every turn best[c] has improved since the last
+      const unsigned long long old = atomicCAS(a.best + c, seen, key);
+      if (old == seen) break;
+      if (!beats<H>(key, old, v, c, hb)) return false;
+      seen = old;
+    }
+    *out = best_holder(seen);
+  } else {
+    const unsigned long long old = atomicMax(a.best + c, key);
+    if (old >= key) return false;
+    *out = best_holder(old);
+  }
+  return true;
 }
 
 // Merges the lanes' sorted lists into the warp's best KK (all lanes get it).
@@ -270,15 +316,18 @@ __device__ __forceinline__ TopK<H, KK> merge_parts(const MatchArgs &a, int cnt, 
   return warp_topk(acc);
 }
 
-// Per-lane best KK over entries [b, e) (e - b <= kChunk) of v's row; all loads
-// of the chunk are issued before any is used.
-template <bool H, int KK>
-__device__ __forceinline__ TopK<H, KK> lane_scan(const MatchArgs &a, int v, long long vw, int b, int e,
-                                                 bool all_elig = false) {
+// Loads entries [b, e) (e - b <= kChunk) of v's row, slot u of a lane entry
+// b + lane + 32 u, all loads issued before any is used, and marks with
+// k[u] = -1 those that are no candidates: the vertex itself, pairs that do not
+// fit (`all`: every pair fits), and neighbours that hold a proposal v cannot
+// beat: by its weight alone (kWeak), or at all (kExact).
+enum : int { kStatic = 0, kWeak = 1, kExact = 2 };
+template <bool H, int FILTER>
+__device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, int e, bool all, int hb,
+                                             int (&k)[kChunk / 32], int (&w)[kChunk / 32]) {
   const int lane = threadIdx.x & 31;
   constexpr int U = kChunk / 32;
   const int nu = (e - b + 31) >> 5;  // slots holding entries (warp-uniform): the others are skipped
-  int k[U], w[U], s[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const int j = b + lane + 32 * u;
@@ -289,15 +338,35 @@ __device__ __forceinline__ TopK<H, KK> lane_scan(const MatchArgs &a, int v, long
       w[u] = a.adjwgt[j];
     }
   }
+  if (!all) {
+    const long long vw = a.vwgt[v], cap = weight_cap(a, v);
+    int vk[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) s[u] = (u < nu && k[u] >= 0 && !all_elig) ? __ldcg(a.m2 + k[u]) : -1;
-  TopK<H, KK> t;
-  const int hb = hash_base(a, v);
+    for (int u = 0; u < U; ++u) vk[u] = (u < nu && k[u] >= 0) ? a.vwgt[k[u]] : 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (!pair_fits(cap, vw, vk[u])) k[u] = -1;
+  }
+  if constexpr (FILTER == kWeak) {
+    unsigned bw[U];  // the weight half of best[]; 0 for none
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      bw[u] = (u < nu && k[u] >= 0) ? __ldcg(reinterpret_cast<const unsigned *>(a.best + k[u]) + 1) : 0u;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (((unsigned)w[u] ^ 0x80000000u) < bw[u]) k[u] = -1;
+  }
+  if constexpr (FILTER == kExact) {
+    unsigned long long bk[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) bk[u] = (u < nu && k[u] >= 0) ? ld_best(a, k[u]) : 0ull;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < nu && k[u] >= 0 && !beats<H>(best_key(v, w[u]), bk[u], v, k[u], hb)) k[u] = -1;
+  }
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (u < nu && k[u] >= 0 && (all_elig ? k[u] != v : eligible<H>(a, vw, v, k[u], s[u])))
-      t.insert_edge(v, k[u], w[u], hb);
-  return t;
+    if (k[u] == v) k[u] = -1;
 }
 
 // Inserts x into the descending list tw (the KK largest values seen, with
@@ -322,38 +391,29 @@ __device__ __forceinline__ void wlist_insert(int (&tw)[KK], int x) {
 // The qualifying entries (usually KK plus the ties at W) are packed one per
 // lane through the warp's 32-entry buffer wbuf; more than 32 of them (many
 // equal weights) take the per-lane lists instead.
-template <bool H, int KK>
-__device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, long long vw, int b, int e, bool all_elig,
-                                                  int2 *wbuf) {
+template <bool H, int KK, int FILTER>
+__device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, int b, int e, bool all, int2 *wbuf) {
+  constexpr int U = kChunk / 32;
+  const int nu = (e - b + 31) >> 5;
+  const int hb = hash_base(a, v);
+  int k[U], w[U];
+  load_entries<H, FILTER>(a, v, b, e, all, hb, k, w);
   if constexpr (!H) {
     (void)wbuf;
-    return warp_topk(lane_scan<H, KK>(a, v, vw, b, e, all_elig));
+    TopK<H, KK> t;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < nu && k[u] >= 0) t.insert_edge(v, k[u], w[u], hb);
+    return warp_topk(t);
   } else {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    constexpr int U = kChunk / 32;
-    const int nu = (e - b + 31) >> 5;  // slots holding entries (warp-uniform): the others are skipped
-    int k[U], w[U], s[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int j = b + lane + 32 * u;
-      k[u] = -1;
-      w[u] = 0;
-      if (u < nu && j < e) {
-        k[u] = a.adjncy[j];
-        w[u] = a.adjwgt[j];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) s[u] = (u < nu && k[u] >= 0 && !all_elig) ? __ldcg(a.m2 + k[u]) : -1;
-    // k[u] = -1 marks an entry that is not an eligible candidate
     int tw[KK], rem = 0;
 #pragma unroll
     for (int i = 0; i < KK; ++i) tw[i] = INT_MIN;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (u >= nu) break;
-      if (k[u] >= 0 && !(all_elig ? k[u] != v : eligible<H>(a, vw, v, k[u], s[u]))) k[u] = -1;
       if (k[u] >= 0) {
         wlist_insert(tw, w[u]);
         ++rem;
@@ -386,7 +446,6 @@ __device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, lon
       if (u >= nu) break;
       total += __popc(__ballot_sync(full, k[u] >= 0 && w[u] >= W));
     }
-    const int hb = hash_base(a, v);
     TopK<H, KK> out;
     if (total > 32) {
       TopK<H, KK> t;
@@ -434,34 +493,70 @@ __device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, lon
   }
 }
 
-// Writes v's cached candidate ids and points v at the first.  A first scan
-// (KK == 1) marks the rest of the cache unknown; a full list marks unused
-// slots "none" (the cache then holds every candidate).
+// Writes v's list.  A list of fewer than KK candidates holds them all; a full
+// one of fewer than kTop slots ends with kUnknown.
 template <bool H, int KK>
 __device__ __forceinline__ void store_top(const MatchArgs &a, int v, const TopK<H, KK> &t) {
-  int q[kTop];
+  int q[kTop], w[kTop];
 #pragma unroll
-  for (int i = 0; i < kTop; ++i) q[i] = i < KK ? t.c[i].id() : (t.c[0].valid() ? kUnknown : -1);
+  for (int i = 0; i < kTop; ++i) {
+    const Cand<H> &c = t.c[i < KK ? i : KK - 1];
+    q[i] = i < KK ? c.id() : (c.valid() ? kUnknown : kNone);
+    w[i] = c.weight();
+  }
   reinterpret_cast<int4 *>(a.top)[v] = make_int4(q[0], q[1], q[2], q[3]);
-  a.ptr[v] = q[0];
+  reinterpret_cast<int4 *>(a.topw)[v] = make_int4(w[0], w[1], w[2], w[3]);
 }
+
+// A vertex's candidates, most preferred first, and the next one to offer to.
+// Two of three candidates have a better proposal by the time they are reached,
+// so the proposals that all of them hold are read together (check) and the
+// first candidate that would take the vertex is offered to with one atomic.
+struct List {
+  int id[kTop], w[kTop];          // slot 0 is next; kNone: no other candidate, kUnknown: the list is used up
+  unsigned long long seen[kTop];  // recent best[id]
+  __device__ __forceinline__ void load(const MatchArgs &a, int v) {
+    const int4 q = reinterpret_cast<const int4 *>(a.top)[v], x = reinterpret_cast<const int4 *>(a.topw)[v];
+    id[0] = q.x; id[1] = q.y; id[2] = q.z; id[3] = q.w;
+    w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
+  }
+  __device__ __forceinline__ void drop() {  // the next candidate
+#pragma unroll
+    for (int t = 0; t + 1 < kTop; ++t) {
+      id[t] = id[t + 1];
+      w[t] = w[t + 1];
+      seen[t] = seen[t + 1];
+    }
+    id[kTop - 1] = kUnknown;
+  }
+  // Drops the candidates up to c: all when c is not listed (it came from a rescan).
+  __device__ __forceinline__ void after(int c) {
+    bool found = false;
+#pragma unroll
+    for (int t = 0; t < kTop; ++t)
+      if (!found) {
+        found = id[0] == c;
+        drop();
+      }
+  }
+  // Reads the candidates' proposals and drops those v does not beat up to the first that it does.
+  template <bool H>
+  __device__ __forceinline__ void check(const MatchArgs &a, int v, int hb) {
+#pragma unroll
+    for (int t = 0; t < kTop; ++t) seen[t] = id[t] >= 0 ? ld_best(a, id[t]) : 0ull;
+    bool go = true;
+#pragma unroll
+    for (int t = 0; t < kTop; ++t) {
+      go = go && id[0] >= 0 && !beats<H>(best_key(v, w[0]), seen[0], v, id[0], hb);
+      if (go) drop();
+    }
+  }
+};
 
 __device__ __forceinline__ unsigned long long warp_excl_scan_u64(unsigned long long v, unsigned long long *total) {
   const unsigned long long inc = warp_inclusive_scan_u64(v);
   *total = __shfl_sync(0xffffffffu, inc, 31);
   return inc - v;
-}
-
-// Warp-aggregated append of x to list[counter]; convergent call.
-__device__ __forceinline__ void warp_append(int *list, int *counter, bool take, int x) {
-  const unsigned mask = __ballot_sync(0xffffffffu, take);
-  if (!mask) return;
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(mask) - 1;
-  int base = 0;
-  if (lane == leader) base = atomicAdd(counter, __popc(mask));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (take) list[base + __popc(mask & ((1u << lane) - 1))] = x;
 }
 
 // Chunk descriptors of the rows queued by the lanes with `take` set (row x of
@@ -483,544 +578,490 @@ __device__ __forceinline__ void write_descs(int4 *desc, bool take, int x, int xs
   }
 }
 
-// Queues x (row of `deg` entries starting at xs) for a full scan in slot
-// `par`; convergent.
-__device__ __forceinline__ void append_scan(const MatchArgs &a, int par, bool take, int x, int xs, int deg) {
+// Queues x (row of deg > kSerialDeg entries starting at xs) for a scan: slot
+// `par`, counter `ctr`; convergent.
+__device__ __forceinline__ void append_scan(const MatchArgs &a, int par, int ctr, bool take, int x, int xs, int deg) {
+  if (!__any_sync(0xffffffffu, take)) return;
   const Slot &S = a.slot[par];
-  warp_append(S.small, a.nsmall + par, take && deg <= kSerialDeg, x);
-  const bool bg = take && deg > kSerialDeg;
-  if (!__any_sync(0xffffffffu, bg)) return;
   const int lane = threadIdx.x & 31;
-  const int nch = bg ? (deg + kChunk - 1) / kChunk : 0;
-  const unsigned long long mine = bg ? ((1ull << 32) | (unsigned long long)nch) : 0ull;
+  const int nch = take ? (deg + kChunk - 1) / kChunk : 0;
+  const unsigned long long mine = take ? ((1ull << 32) | (unsigned long long)nch) : 0ull;
   unsigned long long tot;
   const unsigned long long ex = warp_excl_scan_u64(mine, &tot);
   unsigned long long base = 0;
-  if (lane == 0) base = atomicAdd(a.big + par, tot);
+  if (lane == 0) base = atomicAdd(a.big + ctr, tot);
   base = __shfl_sync(0xffffffffu, base, 0) + ex;
   const int idx = (int)(base >> 32), cb = (int)(base & 0xffffffffu);
-  if (bg) {
-    S.big_v[idx] = x;
+  if (take) {
     S.big_base[idx] = cb;
     S.big_done[idx] = 0;
   }
-  write_descs(S.desc, bg, x, xs, deg, nch, idx, cb);
+  write_descs(S.desc, take, x, xs, deg, nch, idx, cb);
 }
 
-constexpr int kCU = 4;  // vertices per thread in phase C
-
-// Phase C's appends for a block (all threads call it): every thread offers
-// up to kCU vertices to the next round's active list (keep), cache-update
-// list (upd) and scan lists (scan: the short-row list or, for longer rows,
-// the chunk list with one descriptor per kChunk entries).  One block-wide
-// scan of the packed per-thread counts (four 16-bit fields, block totals
-// <= kMatchThreads * kCU) and of the chunk counts, then one atomicAdd per
-// list, issued side by side by four lanes.
-static_assert(kMatchThreads * kCU < 65536, "phase C counts are packed in 16-bit fields");
-__device__ __forceinline__ void phase_c_append(const MatchArgs &a, int np, const bool (&keep)[kCU],
-                                               const bool (&upd)[kCU], const bool (&scan)[kCU], const int (&x)[kCU],
-                                               const int (&xs)[kCU], const int (&deg)[kCU],
-                                               unsigned long long *sh_cw, int *sh_cc, unsigned long long *sh_cb) {
-  constexpr int NW = kMatchThreads / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const Slot &N = a.slot[np];
-  unsigned long long c4 = 0ull;
-  int cch = 0, nch[kCU];
+// Stores a chunk's list among the row's partial lists; true for the warp of
+// the row's last chunk (d: the chunk's descriptor, q its index).
+template <bool H, int KK>
+__device__ __forceinline__ bool part_done(const MatchArgs &a, const Slot &S, int q, const int4 &d, int nch,
+                                          const TopK<H, KK> &r) {
+  const int lane = threadIdx.x & 31;
+  if (lane < KK) {
+    Cand<H> mine = r.c[0];
 #pragma unroll
-  for (int u = 0; u < kCU; ++u) {
-    const bool sm = scan[u] && deg[u] <= kSerialDeg, bg = scan[u] && deg[u] > kSerialDeg;
-    c4 += (unsigned long long)keep[u] | ((unsigned long long)upd[u] << 16) | ((unsigned long long)sm << 32) |
-          ((unsigned long long)bg << 48);
-    nch[u] = bg ? (deg[u] + kChunk - 1) / kChunk : 0;
-    cch += nch[u];
+    for (int t = 1; t < KK; ++t)
+      if (lane == t) mine = r.c[t];
+    mine.store(a.part + ((size_t)q * kTop + lane) * kPartInts);
+    __threadfence();
   }
-  unsigned long long i4 = c4;
-  int ic = cch;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long y4 = __shfl_up_sync(0xffffffffu, i4, o);
-    const int yc = __shfl_up_sync(0xffffffffu, ic, o);
-    if (lane >= o) {
-      i4 += y4;
-      ic += yc;
-    }
-  }
-  if (lane == 31) {
-    sh_cw[warp] = i4;
-    sh_cc[warp] = ic;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    const unsigned long long v4 = lane < NW ? sh_cw[lane] : 0ull;
-    const int vc = lane < NW ? sh_cc[lane] : 0;
-    unsigned long long j4 = v4;
-    int jc = vc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long y4 = __shfl_up_sync(0xffffffffu, j4, o);
-      const int yc = __shfl_up_sync(0xffffffffu, jc, o);
-      if (lane >= o) {
-        j4 += y4;
-        jc += yc;
-      }
-    }
-    const unsigned long long t4 = __shfl_sync(0xffffffffu, j4, 31);
-    const int tc = __shfl_sync(0xffffffffu, jc, 31);
-    if (lane < NW) {
-      sh_cw[lane] = j4 - v4;
-      sh_cc[lane] = jc - vc;
-    }
-    const int f = (int)((t4 >> (16 * (lane & 3))) & 0xffffull);
-    unsigned long long gb = 0ull;
-    if (lane == 0 && f) gb = (unsigned long long)atomicAdd(a.nact + np, f);
-    if (lane == 1 && f) gb = (unsigned long long)atomicAdd(a.nupd + np, f);
-    if (lane == 2 && f) gb = (unsigned long long)atomicAdd(a.nsmall + np, f);
-    if (lane == 3 && (f || tc)) gb = atomicAdd(a.big + np, ((unsigned long long)f << 32) | (unsigned)tc);
-    if (lane < 4) sh_cb[lane] = gb;
-  }
-  __syncthreads();
-  const unsigned long long e4 = sh_cw[warp] + (i4 - c4);
-  int pk = (int)sh_cb[0] + (int)(e4 & 0xffffull);
-  int pu = (int)sh_cb[1] + (int)((e4 >> 16) & 0xffffull);
-  int ps = (int)sh_cb[2] + (int)((e4 >> 32) & 0xffffull);
-  int pb = (int)(sh_cb[3] >> 32) + (int)(e4 >> 48);
-  int pc = (int)(sh_cb[3] & 0xffffffffull) + sh_cc[warp] + (ic - cch);
-#pragma unroll
-  for (int u = 0; u < kCU; ++u) {
-    if (keep[u]) N.act[pk++] = x[u];
-    if (upd[u]) N.upd[pu++] = x[u];
-    if (scan[u] && deg[u] <= kSerialDeg) N.small[ps++] = x[u];
-    const int idx = pb, cb = pc;
-    if (nch[u] > 0) {
-      ++pb;
-      pc += nch[u];
-      N.big_v[idx] = x[u];
-      N.big_base[idx] = cb;
-      N.big_done[idx] = 0;
-    }
-    write_descs(N.desc, nch[u] > 0, x[u], xs[u], deg[u], nch[u], idx, cb);
-  }
-  __syncthreads();  // the shared counts are free for the next call
+  __syncwarp();
+  int last = 0;
+  if (lane == 0) last = atomicAdd(S.big_done + d.w, 1) == nch - 1;
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (last) __threadfence();
+  return last != 0;
 }
 
-// Phase A of a round: full scans of the rows whose candidates must be
-// recomputed -- rows of <= kSerialDeg entries one lane each (the whole vertex
-// range in the first round), longer rows as kChunk-entry warp chunks with a
-// last-chunk merge.  `first`: the first round (keeps kFirstKeep* candidates);
-// `skip_gather`: first round with every edge eligible (no neighbour state).
+constexpr int kPrepThreads = 256;
+// Resident blocks per SM the list kernel is compiled for (register cap).
+#ifndef CM_FIRST_MINBLOCKS
+#define CM_FIRST_MINBLOCKS 8
+#endif
+constexpr int kFirstMinBlocks = CM_FIRST_MINBLOCKS;
+
+// Vertices a warp takes at a time in k_match_prep and k_match_propose: it first
+// packs those it has work for (short rows; rows with entries) in shared memory,
+// so that all lanes work although half of an R-MAT graph's vertices are
+// isolated and the low ids have long rows.  Small graphs take fewer per warp.
+constexpr int kSpan = 256;
+
+// best[] = none, the largest vertex weight, the chunks of the rows longer than
+// kSerialDeg (slot 0), and the lists of the shorter rows, one lane each (from
+// the weights and the cap alone).  The counters are zeroed by the host.
 template <bool H>
-__device__ __forceinline__ void phase_a(const MatchArgs &a, const Slot &S, bool first, bool skip_gather,
-                                        long long nsmall, int nchunks, int gwarp, int nwarps, int lane, int2 *wbuf,
-                                        int *tick) {
-  for (long long b0 = (long long)gwarp * 32; b0 < nsmall; b0 += (long long)nwarps * 32) {
-    const long long i = b0 + lane;
-    if (i >= nsmall) continue;
-    const int v = first ? (int)i : __ldcg(S.small + i);
-    const int xs = a.xadj[v], deg = a.xadj[v + 1] - xs;
-    if (first && (deg == 0 || deg > kSerialDeg)) continue;
-    if (skip_gather) {  // first round, every edge eligible: ids and weights only, 8 at a time
-      constexpr int kHalf = kSerialDeg / 2;
+__global__ void __launch_bounds__(kPrepThreads) k_match_prep(MatchArgs a) {
+  __shared__ int sh_v[kPrepThreads / 32][kSpan];
+  int *list = sh_v[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  const int gwarp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
+  const int n = a.n;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.st->rounds = 1;
+  int wmax = 0;
+  for (long long b0 = (long long)gwarp * a.span; b0 < n; b0 += (long long)nwarps * a.span) {
+    int cnt = 0;
+    for (int i = 0; i < a.span; i += 32) {
+      const int v = (int)(b0 + i + lane);
+      int xs = 0, deg = 0;
+      if (v < n) {
+        wmax = max(wmax, a.vwgt[v]);
+        a.best[v] = 0ull;
+        xs = a.xadj[v];
+        deg = a.xadj[v + 1] - xs;
+      }
+      append_scan(a, 0, 0, deg > kSerialDeg, v, xs, deg);
+      const bool small = deg > 0 && deg <= kSerialDeg;
+      const unsigned m = __ballot_sync(0xffffffffu, small);
+      if (small) list[cnt + __popc(m & below)] = v;
+      cnt += __popc(m);
+    }
+    __syncwarp();
+    for (int i = lane; i < cnt; i += 32) {
+      const int v = list[i];
+      const int xs = a.xadj[v], deg = a.xadj[v + 1] - xs;
+      constexpr int kHalf = 8;
       const int hb = hash_base(a, v);
-      TopK<H, kFirstKeepShort> tk;
+      const long long vw = a.vwgt[v], cap = weight_cap(a, v);
+      TopK<H, kTop> tk;
 #pragma unroll 1
-      for (int t0 = 0; t0 < deg; t0 += kHalf) {
-        int k[kHalf], w[kHalf];
+      for (int t0 = 0; t0 < deg; t0 += kHalf) {  // 8 entries in flight
+        int k[kHalf], w[kHalf], vk[kHalf];
 #pragma unroll
         for (int t = 0; t < kHalf; ++t) {
           k[t] = t0 + t < deg ? a.adjncy[xs + t0 + t] : -1;
           w[t] = t0 + t < deg ? a.adjwgt[xs + t0 + t] : 0;
         }
 #pragma unroll
+        for (int t = 0; t < kHalf; ++t) vk[t] = k[t] >= 0 ? a.vwgt[k[t]] : 0;
+#pragma unroll
         for (int t = 0; t < kHalf; ++t)
-          if (k[t] >= 0 && k[t] != v) tk.insert_edge(v, k[t], w[t], hb);
+          if (k[t] >= 0 && k[t] != v && pair_fits(cap, vw, vk[t])) tk.insert_edge(v, k[t], w[t], hb);
       }
       store_top(a, v, tk);
-      continue;
     }
-    const int sv = __ldcg(a.m2 + v);
-    if (sv >= 0) continue;
-    const long long vw = -1ll - sv;
-    int k[kSerialDeg], s[kSerialDeg];
-#pragma unroll
-    for (int t = 0; t < kSerialDeg; ++t) k[t] = t < deg ? a.adjncy[xs + t] : -1;
-#pragma unroll
-    for (int t = 0; t < kSerialDeg; ++t) s[t] = (k[t] >= 0 && !skip_gather) ? __ldcg(a.m2 + k[t]) : -1;
-    if (first) {
-      TopK<H, 1> tk;
-#pragma unroll
-      for (int t = 0; t < kSerialDeg; ++t)
-        if (k[t] >= 0 && (skip_gather ? k[t] != v : eligible<H>(a, vw, v, k[t], s[t])))
-          tk.insert_edge(v, k[t], a.adjwgt[xs + t], hash_base(a, v));
-      store_top(a, v, tk);
-    } else {
-      TopK<H, kTop> tk;
-#pragma unroll
-      for (int t = 0; t < kSerialDeg; ++t)
-        if (k[t] >= 0 && (skip_gather ? k[t] != v : eligible<H>(a, vw, v, k[t], s[t])))
-          tk.insert_edge(v, k[t], a.adjwgt[xs + t], hash_base(a, v));
-      store_top(a, v, tk);
-    }
-  }
-  // Chunk loop driver: chunks taken from a ticket when one is given (rows of
-  // very different lengths and the last chunk's merge make a fixed
-  // assignment uneven; the next ticket and its descriptor are fetched before
-  // the current chunk is scanned), else round robin over the warps.
-  auto drive = [&](auto &&scan) {
-    if (tick != nullptr) {
-      int q = 0;
-      if (lane == 0) q = atomicAdd(tick, 1);
-      q = __shfl_sync(0xffffffffu, q, 0);
-      int4 d = q < nchunks ? __ldcg(S.desc + q) : make_int4(0, 0, 0, 0);
-      while (q < nchunks) {
-        int qn = 0;
-        if (lane == 0) qn = atomicAdd(tick, 1);
-        qn = __shfl_sync(0xffffffffu, qn, 0);
-        const int4 dn = qn < nchunks ? __ldcg(S.desc + qn) : d;
-        scan(q, d);
-        q = qn;
-        d = dn;
-      }
-    } else {
-      int4 d = gwarp < nchunks ? __ldcg(S.desc + gwarp) : make_int4(0, 0, 0, 0);
-      for (int q = gwarp; q < nchunks; q += nwarps) {
-        const int4 dn = q + nwarps < nchunks ? __ldcg(S.desc + q + nwarps) : d;
-        scan(q, d);
-        d = dn;
-      }
-    }
-  };
-  if (skip_gather) {
-    // First round, every edge eligible: no neighbour state; multi-chunk rows
-    // merge one partial per chunk.
-    drive([&](int q, const int4 &d) {
-      const int v = d.x, i = d.w;
-      constexpr int KC = kFirstKeepChunk;
-      const TopK<H, KC> r1 = chunk_best<H, KC>(a, v, 0, d.y, d.z, true, wbuf);
-      if (i < 0) {
-        if (lane == 0) store_top(a, v, r1);
-        return;
-      }
-      const int nch = (a.xadj[v + 1] - a.xadj[v] + kChunk - 1) / kChunk;
-      int last = 0;
-      if (lane < KC) {
-        Cand<H> mine = r1.c[0];
-#pragma unroll
-        for (int t = 1; t < KC; ++t)
-          if (lane == t) mine = r1.c[t];
-        mine.store(a.part + ((size_t)q * kTop + lane) * kPartInts);
-      }
-      if (lane == 0) {
-        __threadfence();
-        last = atomicAdd(S.big_done + i, 1) == nch - 1;
-      }
-      last = __shfl_sync(0xffffffffu, last, 0);
-      if (last) {
-        __threadfence();
-        const int base = __ldcg(S.big_base + i);
-        const TopK<H, KC> rr =
-            merge_parts<H, KC>(a, nch * KC, [&](int t) { return (size_t)(base + t / KC) * kTop + t % KC; });
-        if (lane == 0) store_top(a, v, rr);
-      }
-    });
-    return;
-  }
-  // Scans with the neighbours' state.  A vertex of a scan list is unmatched
-  // (the lists are built after the previous round's commits), so its row's
-  // loads are issued together with its own state.
-  auto scan_chunk = [&](int q, const int4 &d) {
-    const int v = d.x, i = d.w;
-    const int sv = __ldcg(a.m2 + v);
-    const long long vw = -1ll - sv;
-    TopK<H, kTop> r;
-    if (first) {
-      const TopK<H, 1> r1 = chunk_best<H, 1>(a, v, vw, d.y, d.z, skip_gather, wbuf);
-      r.c[0] = r1.c[0];
-    } else {
-      r = chunk_best<H, kTop>(a, v, vw, d.y, d.z, false, wbuf);
-    }
-    if (sv >= 0) return;  // (not expected) uniform per warp, and alike for all chunks of the row
-    if (i < 0) {  // the row's only chunk
-      if (lane == 0) {
-        if (first) {
-          TopK<H, 1> r1;
-          r1.c[0] = r.c[0];
-          store_top(a, v, r1);
-        } else {
-          store_top(a, v, r);
-        }
-      }
-      return;
-    }
-    const int nch = (a.xadj[v + 1] - a.xadj[v] + kChunk - 1) / kChunk;
-    int last = 0;
-    if (lane < kTop) {
-      Cand<H> mine = r.c[0];
-#pragma unroll
-      for (int t = 1; t < kTop; ++t)
-        if (lane == t) mine = r.c[t];
-      mine.store(a.part + ((size_t)q * kTop + lane) * kPartInts);
-    }
-    if (lane == 0) {
-      __threadfence();
-      last = atomicAdd(S.big_done + i, 1) == nch - 1;
-    }
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (last) {  // merge the row's chunk lists
-      __threadfence();
-      const int base = __ldcg(S.big_base + i);
-      const TopK<H, kTop> rr = merge_parts<H, kTop>(a, nch * kTop, [&](int t) { return (size_t)base * kTop + t; });
-      if (lane == 0) {
-        if (first) {
-          TopK<H, 1> r1;
-          r1.c[0] = rr.c[0];
-          store_top(a, v, r1);
-        } else {
-          store_top(a, v, rr);
-        }
-      }
-    }
-  };
-  drive(scan_chunk);
-}
-
-// Before the rounds: initial state of every vertex (unmatched, no
-// candidate), the largest vertex weight, and the first round's chunk list of
-// rows longer than kSerialDeg.  The list counters are zeroed by the host.
-constexpr int kPrepThreads = 256;
-// Resident blocks per SM the first-round kernel is compiled for (register cap).
-#ifndef CM_FIRST_MINBLOCKS
-#define CM_FIRST_MINBLOCKS 8
-#endif
-constexpr int kFirstMinBlocks = CM_FIRST_MINBLOCKS;
-template <bool H>
-__global__ void __launch_bounds__(kPrepThreads) k_match_prep(MatchArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int gwarp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
-  const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-  const int n = a.n;
-  int wmax = 0;
-  for (long long b0 = (long long)gwarp * 32; b0 < n; b0 += (long long)nwarps * 32) {
-    const long long v = b0 + lane;
-    int xs = 0, deg = 0;
-    if (v < n) {
-      const int vw0 = a.vwgt[v];
-      wmax = max(wmax, vw0);
-      a.m2[v] = -1 - vw0;
-      a.ptr[v] = -1;
-      a.stamp[v] = 0;
-      a.top[v * kTop] = kNotScanned;
-      xs = a.xadj[v];
-      deg = a.xadj[v + 1] - xs;
-    }
-    append_scan(a, 0, deg > kSerialDeg, (int)v, xs, deg);
+    __syncwarp();  // the list is free for the next span
   }
   wmax = __reduce_max_sync(0xffffffffu, wmax);
   if (lane == 0 && wmax > 0) atomicMax(a.vmax, wmax);
 }
 
-// Phase A of the first round, as an ordinary launch with more warps per SM
-// than the persistent kernel can hold.  When even the two heaviest vertices
-// may pair and are light (2 vmax <= maxvwgt, 3 vmax < maxvwgt), every edge is
-// eligible while nothing is matched, and the scans skip the neighbour state.
-// Both forms are launched (the choice is made on the device, from vmax); the
-// one that does not apply returns at once.  Separate kernels keep each form's
-// register allocation to its own needs.
+// The lists of the rows longer than kSerialDeg, one warp a chunk, the warp of
+// a row's last chunk merging the chunks' lists.  Two forms: with every edge
+// eligible the scan reads no vertex weights and fits 32 registers.  Both are
+// launched (the choice is made on the device, from the largest vertex
+// weight); the one that does not apply returns at once.
 template <bool H, bool ALL>
-__global__ void __launch_bounds__(kPrepThreads, kFirstMinBlocks) k_match_first(MatchArgs a) {
-  const long long vmax = __ldcg(a.vmax);
-  const bool all_elig = 2 * vmax <= a.maxvwgt && 3 * vmax < a.maxvwgt;
-  if (all_elig != ALL) return;
+__global__ void __launch_bounds__(kPrepThreads, ALL ? kFirstMinBlocks : kFirstMinBlocks / 2) k_match_first(MatchArgs a) {
+  if (all_eligible(a) != ALL) return;
   const int lane = threadIdx.x & 31;
   const int gwarp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-  const int nchunks = (int)(__ldcg(a.big) & 0xffffffffu);
   __shared__ int2 sh_q[kPrepThreads / 32][32];
-  phase_a<H>(a, a.slot[0], true, ALL, a.n, nchunks, gwarp, nwarps, lane, sh_q[threadIdx.x >> 5], nullptr);
+  const Slot &S = a.slot[0];
+  const int nchunks = (int)(__ldcg(a.big) & 0xffffffffu);
+  constexpr int KC = kFirstKeepChunk;
+  int4 d = gwarp < nchunks ? __ldcg(S.desc + gwarp) : make_int4(0, 0, 0, 0);
+  for (int q = gwarp; q < nchunks; q += nwarps) {
+    const int4 dn = q + nwarps < nchunks ? __ldcg(S.desc + q + nwarps) : d;
+    const int v = d.x;
+    const TopK<H, KC> r = chunk_best<H, KC, kStatic>(a, v, d.y, d.z, ALL, sh_q[threadIdx.x >> 5]);
+    if (d.w < 0) {
+      if (lane == 0) store_top(a, v, r);
+    } else {
+      const int nch = (a.xadj[v + 1] - a.xadj[v] + kChunk - 1) / kChunk;
+      if (part_done<H, KC>(a, S, q, d, nch, r)) {
+        const int base = __ldcg(S.big_base + d.w);
+        const TopK<H, KC> rr =
+            merge_parts<H, KC>(a, nch * KC, [&](int t) { return (size_t)(base + t / KC) * kTop + t % KC; });
+        if (lane == 0) store_top(a, v, rr);
+      }
+    }
+    d = dn;
+  }
 }
 
+// Best candidate of a short row (deg <= kSerialDeg) that takes v now, by one
+// lane; *seen = the proposal it holds.  -1: none.
 template <bool H>
-__global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match(MatchArgs a) {
-  __shared__ int2 sh_q[kMatchThreads / 32][32];  // per warp: packed candidates of a chunk scan
-  __shared__ unsigned long long sh_cw[kMatchThreads / 32];  // phase C appends: per-warp packed counts
-  __shared__ int sh_cc[kMatchThreads / 32];                 // ... and chunk counts
-  __shared__ unsigned long long sh_cb[4];                   // ... and the lists' bases
-  __shared__ int sh_tk;                                     // phase C: the block's ticket
+__device__ __forceinline__ int rescan_short(const MatchArgs &a, int v, int xs, int deg, bool all, int hb, int *weight,
+                                            unsigned long long *seen) {
+  constexpr int kHalf = 8;
+  const long long vw = all ? 0 : a.vwgt[v], cap = all ? 0 : weight_cap(a, v);
+  TopK<H, 1> t1;
+  *seen = 0ull;
+#pragma unroll 1
+  for (int t0 = 0; t0 < deg; t0 += kHalf) {
+    int k[kHalf], w[kHalf];
+    unsigned long long b[kHalf];
+#pragma unroll
+    for (int t = 0; t < kHalf; ++t) {
+      k[t] = t0 + t < deg ? a.adjncy[xs + t0 + t] : -1;
+      w[t] = t0 + t < deg ? a.adjwgt[xs + t0 + t] : 0;
+    }
+#pragma unroll
+    for (int t = 0; t < kHalf; ++t) b[t] = k[t] >= 0 ? ld_best(a, k[t]) : 0ull;
+    if (!all) {
+      int vk[kHalf];
+#pragma unroll
+      for (int t = 0; t < kHalf; ++t) vk[t] = k[t] >= 0 ? a.vwgt[k[t]] : 0;
+#pragma unroll
+      for (int t = 0; t < kHalf; ++t)
+        if (!pair_fits(cap, vw, vk[t])) k[t] = -1;
+    }
+#pragma unroll
+    for (int t = 0; t < kHalf; ++t) {
+      if (k[t] < 0 || k[t] == v || (t1.c[0].valid() && w[t] < t1.c[0].weight())) continue;
+      const Cand<H> c = Cand<H>::make(v, k[t], w[t], hb);
+      if (c.better(t1.c[0]) && beats<H>(best_key(v, w[t]), b[t], v, k[t], hb)) {
+        t1.c[0] = c;
+        *seen = b[t];
+      }
+    }
+  }
+  *weight = t1.c[0].weight();
+  return t1.c[0].id();
+}
+
+// One lane a vertex: offers the vertex to its candidates in order and goes on
+// with whomever a taker gives up, until nobody is left without a proposal or
+// the free vertex needs a scan of a long row, which is queued (slot 1).  A lane
+// whose chain has ended takes the span's next vertex.
+template <bool H>
+__global__ void __launch_bounds__(kPrepThreads) k_match_propose(MatchArgs a) {
+  __shared__ int sh_v[kPrepThreads / 32][kSpan];
+  int *list = sh_v[threadIdx.x >> 5];
+  const bool all = all_eligible(a);
   const int lane = threadIdx.x & 31;
-  const long long gthread = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nthreads = (long long)gridDim.x * blockDim.x;
-  const int gwarp = (int)(gthread >> 5);
-  const int nwarps = (int)(nthreads >> 5);
+  const unsigned below = (1u << lane) - 1u;
+  const int gwarp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   const int n = a.n;
+  for (long long b0 = (long long)gwarp * a.span; b0 < n; b0 += (long long)nwarps * a.span) {
+    int cnt = 0, taken = 0;
+    for (int i = 0; i < a.span; i += 32) {
+      const int v = (int)(b0 + i + lane);
+      const bool has = v < n && a.xadj[v + 1] > a.xadj[v];
+      const unsigned m = __ballot_sync(0xffffffffu, has);
+      if (has) list[cnt + __popc(m & below)] = v;
+      cnt += __popc(m);
+    }
+    __syncwarp();
+    int cur = -1, hb = 0;
+    List L;
+    for (;;) {
+      const unsigned idle = __ballot_sync(0xffffffffu, cur < 0);
+      if (taken < cnt && idle) {
+        const int at = taken + __popc(idle & below);
+        if (cur < 0 && at < cnt) {
+          cur = list[at];
+          hb = hash_base(a, cur);  // a chain stays in its graph
+          L.load(a, cur);
+        }
+        taken += __popc(idle);
+      } else if (idle == 0xffffffffu) {
+        break;
+      }
+      int qv = -1, qx = 0, qdeg = 0;
+      if (cur >= 0) {
+        L.check<H>(a, cur, hb);
+        int c = L.id[0], w = L.w[0];
+        unsigned long long held = L.seen[0];
+        if (c == kUnknown) {
+          qx = a.xadj[cur];
+          qdeg = a.xadj[cur + 1] - qx;
+          if (qdeg > kSerialDeg) qv = cur;
+          else c = rescan_short<H>(a, cur, qx, qdeg, all, hb, &w, &held);
+        }
+        if (c < 0) {  // queued, or no candidate is left
+          cur = -1;
+        } else {
+          int out = -1;
+          if (offer<H>(a, cur, c, w, held, hb, &out)) {
+            cur = out;
+            if (cur >= 0) {
+              L.load(a, cur);
+              L.after(c);
+            }
+          }  // refused: c holds a better proposal now, which the next check sees
+        }
+      }
+      __syncwarp();
+      append_scan(a, 1, 1, qv >= 0, qv, qx, qdeg);
+    }
+    __syncwarp();  // the list is free for the next span
+  }
+}
+
+// A warp's chain, starting with v (free): its row is scanned, or `r` holds the
+// candidates of a scan already made (rows of several chunks).  With hashed ties
+// a scan first filters by weight alone -- the hash of every entry that ties
+// with its neighbour's proposal costs more than the scan -- and only when all
+// the candidates so found turn out to be refused is the row scanned again with
+// the full test.  A free vertex whose row has several chunks is queued for the
+// next round (slot par, counter ctr).  Convergent.
+template <bool H>
+__device__ __forceinline__ void warp_chain(const MatchArgs &a, int v, int xs, int xe, bool scanned,
+                                           const TopK<H, kTop> &r, bool all, int par, int ctr, int2 *wbuf) {
+  const int lane = threadIdx.x & 31;
+  const int hb = hash_base(a, v);
+  int cur = v;
+  List L;
+  auto take = [&](const TopK<H, kTop> &t) {  // the scan's candidates as a list
+#pragma unroll
+    for (int i = 0; i < kTop; ++i) {
+      L.id[i] = t.c[i].id();
+      L.w[i] = t.c[i].weight();
+    }
+    L.check<H>(a, cur, hb);
+  };
+  if (scanned) take(r);
+  else L.id[0] = kUnknown;
+  for (;;) {
+    if (L.id[0] == kUnknown) {
+      if (cur != v || scanned) {
+        xs = a.xadj[cur];
+        xe = a.xadj[cur + 1];
+      }
+      if (xe - xs > kChunk) {
+        append_scan(a, par, ctr, lane == 0, cur, xs, xe - xs);
+        return;
+      }
+      if constexpr (H) take(chunk_best<H, kTop, kWeak>(a, cur, xs, xe, all, wbuf));
+      if (!H || L.id[0] == kUnknown) take(chunk_best<H, kTop, kExact>(a, cur, xs, xe, all, wbuf));
+    }
+    const int c = L.id[0];
+    if (c == kNone) return;
+    if (c == kUnknown) continue;  // others took all of them meanwhile
+    int res = -2;  // -2: refused, else the vertex given up (-1: none)
+    if (lane == 0) {
+      int out = -1;
+      if (offer<H>(a, cur, c, L.w[0], L.seen[0], hb, &out)) res = out;
+    }
+    res = __shfl_sync(0xffffffffu, res, 0);
+    if (res == -2) {
+      L.drop();
+    } else {
+      if (res < 0) return;
+      cur = res;
+      L.load(a, cur);
+      L.after(c);
+      scanned = true;  // xs, xe are another row's
+    }
+    L.check<H>(a, cur, hb);
+  }
+}
+
+// Scans of the queued rows and the chains they start, in rounds; ONE_PASS: no
+// row has several chunks, so nothing is queued again and no barrier is needed
+// (an ordinary launch).
+template <bool H, bool ONE_PASS>
+__global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds(MatchArgs a) {
+  __shared__ int2 sh_q[kMatchThreads / 32][32];  // per warp: packed candidates of a chunk scan
+  const int lane = threadIdx.x & 31;
+  const bool all = all_eligible(a);
+  int2 *wbuf = sh_q[threadIdx.x >> 5];
   DevStatus *st = a.st;
-  const bool tracer = a.trace != nullptr && gthread == 0;
+  const bool first_thread = blockIdx.x == 0 && threadIdx.x == 0;
   auto trace = [&](int row, int col, unsigned long long v) {
-    if (tracer && row < a.trace_rows) a.trace[row * 8 + col] = v;
+    if (a.trace != nullptr && first_thread && row < a.trace_rows) a.trace[row * 8 + col] = v;
   };
   trace(0, 0, global_timer_ns());
-
-  // Tail mode: once a round's lists are small enough for one block, the
-  // other blocks return and block 0 runs the remaining rounds alone with
-  // block barriers instead of grid barriers (the rounds converge to the same
-  // matching whatever the schedule).  All blocks decide it alike: from the
-  // counters, read after a grid barrier.
+  trace(0, 1, global_timer_ns());
   bool tail = false;
-  int round = 0;
+  int round = 1;  // slot and counter 1 hold what k_match_propose queued
   for (;; ++round) {
-    const int par = round & 1;
+    const int par = round & 1, ctr = round % 3, next = (round + 1) % 3;
     const Slot &S = a.slot[par];
-    // round 0: the short-row scan list and the active list are the vertex range
-    const long long nsmall = round == 0 ? n : __ldcg(a.nsmall + par);
-    const int nupd = __ldcg(a.nupd + par);
-    const long long nact = round == 0 ? n : __ldcg(a.nact + par);
-    const unsigned long long bc = __ldcg(a.big + par);
-    const int nbig = (int)(bc >> 32), nchunks = (int)(bc & 0xffffffffu);
-    if (!tail && round > 0 && nsmall + nbig + nupd <= kTailItems && nchunks <= kTailChunks && nact <= kTailItems) {
+    const unsigned long long bc = __ldcg(a.big + ctr);
+    const int nchunks = (int)(bc & 0xffffffffu);
+    trace(round, 0, global_timer_ns());
+    trace(round, 5, bc >> 32);
+    trace(round, 6, (unsigned long long)nchunks);
+    if (nchunks == 0) break;
+    if (round > a.max_rounds) {
+      if (first_thread) record_error(st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
+      break;
+    }
+    // All blocks decide alike, from the counter read after a grid barrier.
+    if (!ONE_PASS && !tail && round > 1 && nchunks <= kTailChunks) {
       tail = true;
       if (blockIdx.x != 0) return;
     }
-    // this round's thread, warp and block indices (block 0 alone in tail mode)
-    const long long gth = tail ? (long long)threadIdx.x : gthread;
-    const long long nth = tail ? (long long)blockDim.x : nthreads;
-    const int gw = tail ? (int)(threadIdx.x >> 5) : gwarp;
-    const int nw = tail ? (int)(blockDim.x >> 5) : nwarps;
-    auto barrier = [&]() -> bool {
-      if (!tail) return grid_barrier(st, gridDim.x);
-      __syncthreads();
-      return ld_relaxed(&st->error) == 0;
-    };
-    if (round == 0) trace(0, 1, global_timer_ns());
-    trace(round + 1, 0, global_timer_ns());
-    trace(round + 1, 4, (unsigned long long)nsmall);
-    trace(round + 1, 5, (unsigned long long)nbig);
-    trace(round + 1, 6, (unsigned long long)nchunks);
-    trace(round + 1, 7, (unsigned long long)nupd);
-    if (nsmall == 0 && nbig == 0 && nupd == 0) break;
-    if (round >= a.max_rounds) {
-      if (gth == 0) record_error(st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
-      break;
+    if (!ONE_PASS && first_thread) {  // the counters of the round after the next
+      a.big[(round + 2) % 3] = 0;
+      a.tick[(round + 2) % 3] = 0;
     }
-    if (gth == 0) {  // the next round's lists and tickets start empty
-      a.nsmall[par ^ 1] = 0;
-      a.nupd[par ^ 1] = 0;
-      a.nact[par ^ 1] = 0;
-      a.big[par ^ 1] = 0;
-      a.tick[2 * (par ^ 1)] = 0;
-      a.tick[2 * (par ^ 1) + 1] = 0;
-    }
-    // A vertex's first scan keeps only its best candidate (most vertices never
-    // need more); a rescan fills the whole cache.
-    const bool first = round == 0;
-
-    // ---- phase A: full scans (the first round's ran in k_match_first) ---------
-    if (!first) phase_a<H>(a, S, false, false, nsmall, nchunks, gw, nw, lane, sh_q[threadIdx.x >> 5], a.tick + 2 * par);
-    if (!barrier()) return;
-    trace(round + 1, 1, global_timer_ns());
-
-    // ---- phase B: commit mutual pairs ----------------------------------------
-    // Candidates that changed this round: short scans, chunked scans, cache
-    // updates (in the first round every vertex, once).
-    const long long tot_b = first ? n : nsmall + nbig + nupd;
-    for (long long i = gth; i < tot_b; i += nth) {
-      int v;
-      if (i < nsmall) {
-        v = first ? (int)i : __ldcg(S.small + i);
-      } else if (i < nsmall + nbig) {
-        v = __ldcg(S.big_v + (i - nsmall));
-      } else {
-        v = __ldcg(S.upd + (i - nsmall - nbig));
-      }
-      const int p = __ldcg(a.ptr + v);
-      if (p < 0 || __ldcg(a.m2 + v) >= 0 || __ldcg(a.ptr + p) != v) continue;
-      // Both ends changed this round: the lower id commits.
-      if (p < v && __ldcg(a.stamp + p) == round) continue;
-      a.m2[v] = p;
-      a.m2[p] = v;
-    }
-    if (!barrier()) return;
-    trace(round + 1, 2, global_timer_ns());
-
-    // ---- phase C: filter the active list, refresh stale pointers -------------
-    // Blocks take kMatchThreads * kCU consecutive entries (block-wide appends).
-    // Blocks take kMatchThreads * kCU consecutive entries at a time from a
-    // ticket (a fixed assignment leaves most blocks idle once the list spans
-    // only one or two spans per block).
-    const long long span = (long long)kMatchThreads * kCU;
-    for (;;) {
-      if (threadIdx.x == 0) sh_tk = atomicAdd(a.tick + 2 * par + 1, 1);
-      __syncthreads();
-      const long long b0 = (long long)sh_tk * span;
-      __syncthreads();
-      if (b0 >= nact) break;
-      int x[kCU], p[kCU], sx[kCU], sp[kCU];
-#pragma unroll
-      for (int u = 0; u < kCU; ++u) {
-        const long long i = b0 + threadIdx.x + (long long)kMatchThreads * u;
-        x[u] = i < nact ? (first ? (int)i : __ldcg(S.act + i)) : -1;
-      }
-#pragma unroll
-      for (int u = 0; u < kCU; ++u) {
-        sx[u] = x[u] >= 0 ? __ldcg(a.m2 + x[u]) : 0;
-        p[u] = x[u] >= 0 ? __ldcg(a.ptr + x[u]) : -1;
-      }
-#pragma unroll
-      for (int u = 0; u < kCU; ++u)
-        if (sx[u] >= 0 || p[u] < 0) x[u] = -1;  // matched, or no candidate: out for good
-#pragma unroll
-      for (int u = 0; u < kCU; ++u) sp[u] = x[u] >= 0 ? __ldcg(a.m2 + p[u]) : -1;
-      bool keep[kCU], upd[kCU], scan[kCU];
-      int xs[kCU], deg[kCU];
-#pragma unroll
-      for (int u = 0; u < kCU; ++u) {
-        keep[u] = upd[u] = scan[u] = false;
-        xs[u] = deg[u] = 0;
-        const int xv = x[u];
-        if (xv < 0) continue;
-        if (sp[u] < 0) {
-          keep[u] = true;                    // waiting on an unmatched candidate
-          continue;
+    // Chunks are taken from a ticket: rows and chains differ in length.
+    int q = 0;
+    if (lane == 0) q = atomicAdd(a.tick + ctr, 1);
+    q = __shfl_sync(0xffffffffu, q, 0);
+    int4 d = q < nchunks ? __ldcg(S.desc + q) : make_int4(0, 0, 0, 0);
+    while (q < nchunks) {
+      int qn = 0;
+      if (lane == 0) qn = atomicAdd(a.tick + ctr, 1);
+      TopK<H, kTop> r;
+      bool mine = true;
+      if (d.w >= 0) {
+        r = chunk_best<H, kTop, kExact>(a, d.x, d.y, d.z, all, wbuf);
+        const int nch = (a.xadj[d.x + 1] - a.xadj[d.x] + kChunk - 1) / kChunk;
+        mine = part_done<H, kTop>(a, S, q, d, nch, r);
+        if (mine) {
+          const int base = __ldcg(S.big_base + d.w);
+          r = merge_parts<H, kTop>(a, nch * kTop, [&](int t) { return (size_t)base * kTop + t; });
         }
-        // from L2: phase A of this kernel rewrites the caches on other SMs
-        const int4 c = __ldcg(reinterpret_cast<const int4 *>(a.top) + xv);
-        const int cs[kTop] = {c.x, c.y, c.z, c.w};
-        int sm[kTop];
-#pragma unroll
-        for (int t = 0; t < kTop; ++t) sm[t] = cs[t] >= 0 ? __ldcg(a.m2 + cs[t]) : 0;
-        // first unmatched cached candidate; -1 = no candidate left, kUnknown or
-        // a full cache exhausted = rescan
-        int np = -2;
-#pragma unroll
-        for (int t = kTop - 1; t >= 0; --t) {
-          if (cs[t] >= 0 && sm[t] < 0) np = cs[t];
-          else if (cs[t] == -1) np = -1;
-          else if (cs[t] == kUnknown) np = -2;
-        }
-        if (np >= 0) {
-          a.ptr[xv] = np;
-          keep[u] = upd[u] = true;
-        } else if (np == -1) {
-          a.ptr[xv] = -1;                    // the cache held every candidate: none left
-        } else {
-          keep[u] = scan[u] = true;
-          xs[u] = a.xadj[xv];
-          deg[u] = a.xadj[xv + 1] - xs[u];
-        }
-        if (upd[u] || scan[u]) atomicMax(a.stamp + xv, round + 1);
       }
-      phase_c_append(a, par ^ 1, keep, upd, scan, x, xs, deg, sh_cw, sh_cc, sh_cb);
+      qn = __shfl_sync(0xffffffffu, qn, 0);
+      const int4 dn = qn < nchunks ? __ldcg(S.desc + qn) : d;
+      if (mine) warp_chain<H>(a, d.x, d.y, d.z, d.w >= 0, r, all, par ^ 1, next, wbuf);
+      q = qn;
+      d = dn;
     }
-    if (!barrier()) return;
-    trace(round + 1, 3, global_timer_ns());
+    trace(round, 3, global_timer_ns());
+    if (ONE_PASS) break;
+    if (!tail) {
+      if (!grid_barrier(st, gridDim.x)) return;
+    } else {
+      __threadfence();
+      __syncthreads();
+      if (ld_relaxed(&st->error) != 0) return;
+    }
   }
-  // (unmatched vertices become singletons in k_match_finish)
-  if (gthread == 0) st->rounds = round;
+  if (first_thread) st->rounds = round;
   trace(0, 3, global_timer_ns());
-  trace(0, 4, (unsigned long long)round);
+  trace(0, 4, (unsigned long long)(round - 1));
 }
 
-// After the rounds: every vertex still unmatched is a singleton.
-__global__ void k_match_finish(int n, int *__restrict__ m2) {
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x)
-    if (m2[v] < 0) m2[v] = (int)v;
+// The matching of an adjacency that is not symmetric: mutual proposals in
+// rounds until no pair forms.  Every unmatched vertex points at its most
+// preferred unmatched neighbour (ptr), and vertices that point at each other
+// are matched.  One warp a vertex, over the warps gw, gw + nw, ...; barrier()
+// separates the phases and returns false to give up.  Reads and writes of
+// other warps' vertices go to L2.
+template <bool H, typename B>
+__device__ void handshake_rounds(const MatchArgs &a, int *ptr, int *changed, int gw, int nw, B barrier) {
+  const int lane = threadIdx.x & 31;
+  const int n = a.n;
+  for (long long v = (long long)gw * 32 + lane; v < n; v += (long long)nw * 32) a.m2[v] = -1;
+  if (gw == 0 && lane == 0) changed[0] = changed[1] = changed[2] = 0;
+  if (!barrier()) return;
+  for (int round = 0;; ++round) {
+    if (gw == 0 && lane == 0) changed[(round + 1) % 3] = 0;
+    for (long long v = gw; v < n; v += nw) {
+      if (__ldcg(a.m2 + v) >= 0) continue;
+      const int hb = hash_base(a, (int)v);
+      const long long vw = a.vwgt[v], cap = weight_cap(a, (int)v);
+      Cand<H> c;
+      for (int j = a.xadj[v] + lane; j < a.xadj[v + 1]; j += 32) {
+        const int k = a.adjncy[j];
+        if (k == (int)v || __ldcg(a.m2 + k) >= 0 || !pair_fits(cap, vw, a.vwgt[k])) continue;
+        const Cand<H> x = Cand<H>::make((int)v, k, a.adjwgt[j], hb);
+        if (x.better(c)) c = x;
+      }
+      const int p = c.warp_best().id();
+      if (lane == 0) ptr[v] = p;
+    }
+    if (!barrier()) return;
+    bool any = false;
+    for (long long v = (long long)gw * 32 + lane; v < n; v += (long long)nw * 32) {
+      if (__ldcg(a.m2 + v) >= 0) continue;
+      const int p = __ldcg(ptr + v);
+      if (p > (int)v && __ldcg(ptr + p) == (int)v) {  // the lower end commits both
+        a.m2[v] = p;
+        a.m2[p] = (int)v;
+        any = true;
+      }
+    }
+    if (any) changed[round % 3] = 1;
+    if (!barrier()) return;
+    if (__ldcg(changed + round % 3) == 0) break;
+  }
+  for (long long v = (long long)gw * 32 + lane; v < n; v += (long long)nw * 32)
+    if (a.m2[v] < 0) a.m2[v] = (int)v;
+}
+
+// match[v] from best[]; a proposal that is not returned sets odd[0].  With
+// `alone` the last block then computes the matching by handshakes itself.
+template <bool H>
+__global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int alone) {
+  bool odd = false;
+  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < a.n;
+       v += (long long)gridDim.x * blockDim.x) {
+    const int h = best_holder(a.best[v]);
+    const bool mutual = h >= 0 && best_holder(a.best[h]) == (int)v;
+    a.m2[v] = mutual ? h : (int)v;
+    odd |= h >= 0 && !mutual;
+  }
+  if (odd) atomicOr(a.odd, 1);
+  if (!alone) return;
+  __threadfence();
+  __syncthreads();
+  __shared__ int s_last;
+  if (threadIdx.x == 0) s_last = atomicAdd(a.odd + 1, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!s_last || __ldcg(a.odd) == 0) return;
+  handshake_rounds<H>(a, a.top, a.odd + 2, threadIdx.x >> 5, blockDim.x >> 5, [&] {
+    __threadfence();
+    __syncthreads();
+    return true;
+  });
+}
+
+// The same for large graphs, with every resident block.
+template <bool H>
+__global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_handshake(MatchArgs a) {
+  if (__ldcg(a.odd) == 0) return;
+  handshake_rounds<H>(a, a.top, a.odd + 2, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5),
+                      (int)((gridDim.x * blockDim.x) >> 5), [&] { return grid_barrier(a.st, gridDim.x); });
 }
 
 // ---------------------------------------------------------------------------
@@ -1102,14 +1143,19 @@ int64_t max_chunks(int64_t n, int64_t m) { return m / kChunk + n + 64; }
 
 size_t match_ws_bytes(int64_t n, int64_t m) {
   const int64_t ch = max_chunks(n, m);
-  size_t b = (size_t)n * 4 * (3 + kTop);                      // ptr, stamp, top (+slack)
-  b += 2 * ((size_t)n * 4 * 6 + (size_t)ch * 16);             // two slots
+  size_t b = (size_t)n * (8 + 2 * 4 * kTop);                  // best, lists
+  b += 2 * ((size_t)n * 4 * 2 + (size_t)ch * 16);             // two slots
   b += (size_t)ch * 4 * kPartInts * kTop;                     // chunk partial lists
   return b + 64 * 256;
 }
 
+// Graphs above this many vertices + entries get the handshake kernel with
+// every block behind k_match_finish (a launch that returns at once costs a few
+// us, under 5% there); below it the last block of k_match_finish does the work.
+constexpr int64_t kAloneWork = 1 << 21;
+
 int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, int32_t *d_match, cudaStream_t s,
-                 const int32_t *vgid, const int32_t *gbase, const int32_t *gcap) {
+                 const int32_t *vgid, const int32_t *gbase, const int32_t *gcap, int64_t max_deg) {
   const int n = g->nvtxs;
   if (n == 0) return CM_OK;
   if (mode != CM_MATCH_HEM && mode != CM_MATCH_HEM_HASH && mode != CM_MATCH_RACY)
@@ -1153,68 +1199,88 @@ int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, 
     ok = ok && p != nullptr;
     return (int *)p;
   };
-  a.ptr = take((size_t)n * 4);
-  a.stamp = take((size_t)n * 4);
+  a.best = (unsigned long long *)take((size_t)n * 8);
   a.top = take((size_t)n * 4 * kTop);
+  a.topw = take((size_t)n * 4 * kTop);
   for (int p = 0; p < 2; ++p) {
     Slot &S = a.slot[p];
-    S.small = take((size_t)n * 4);
-    S.big_v = take((size_t)n * 4);
     S.big_base = take((size_t)n * 4);
     S.big_done = take((size_t)n * 4);
     S.desc = (int4 *)take((size_t)ch * 16);
-    S.upd = take((size_t)n * 4);
-    S.act = take((size_t)n * 4);
   }
   a.part = take((size_t)ch * 4 * kPartInts * kTop);
-  int *ctrs = take(320);  // list counters of both slots and the largest vertex weight
+  int *ctrs = take(256);  // counters of the slots, the largest vertex weight, flags
   if (!ok) return cm_fail(CM_ERR_NOMEM, "cm_match: workspace too small");
-  a.nsmall = ctrs;
-  a.nupd = ctrs + 16;
-  a.nact = ctrs + 32;
-  a.big = (unsigned long long *)(ctrs + 48);
-  a.vmax = ctrs + 64;
-  a.tick = ctrs + 72;
-  cudaMemsetAsync(ctrs, 0, 320, s);
-  a.max_rounds = n + 8;
+  a.big = (unsigned long long *)ctrs;
+  a.tick = ctrs + 8;
+  a.vmax = ctrs + 16;
+  a.odd = ctrs + 24;
+  cudaMemsetAsync(ctrs, 0, 256, s);
+  a.max_rounds = (long long)n + g->nedges + 8;
   a.st = ctx->d_status;
   a.trace = ctx->d_trace;
   a.trace_rows = ctx->trace_rows;
-  const int hm = mode == CM_MATCH_HEM_HASH ? 1 : 0;
-  const void *fn = hm ? (const void *)k_match<true> : (const void *)k_match<false>;
-  int &per_sm = ctx->match_blocks_per_sm[hm];  // queried once per context and tie order
-  if (per_sm == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMatchThreads, 0);
+  const bool hash = mode == CM_MATCH_HEM_HASH;
+  // No row longer than kChunk: the queued rows take one pass and no barrier.
+  const bool one_pass = max_deg <= kChunk;
+  const bool rounds = max_deg > kSerialDeg || a.trace != nullptr;
+  const bool alone = (int64_t)n + g->nedges <= kAloneWork;
+  const void *fn = hash ? (const void *)k_match_rounds<true, false> : (const void *)k_match_rounds<false, false>;
+  const void *hfn = hash ? (const void *)k_match_handshake<true> : (const void *)k_match_handshake<false>;
+  int &per_sm = ctx->match_blocks_per_sm[hash];  // queried once per context and tie order
+  if (per_sm == 0) {
+    int h_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMatchThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h_sm, hfn, kMatchThreads, 0);
+    per_sm = std::min(per_sm, h_sm);
+  }
   if (per_sm < 1) {
     per_sm = 0;
     return cm_fail(CM_ERR_CUDA, "cm_match: kernel cannot be resident");
   }
   // Small graphs take a few SMs, so that kernels of other contexts (other
-  // streams) can run beside this one; the kernel is grid-size agnostic.
+  // streams) can run beside this one; the kernels are grid-size agnostic.
   const int64_t want = (n + g->nedges) / kWorkPerBlock + 1;
   const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * per_sm, want);
   void *args[] = {(void *)&a};
   stage_begin(ctx, s);
   const unsigned pgrid = (unsigned)std::min<int64_t>((int64_t)ctx->num_sms * 8, n / kPrepThreads + 1);
-  const unsigned fgrid = (unsigned)std::min<int64_t>((int64_t)ctx->num_sms * 8, want * 4);
-  if (mode == CM_MATCH_HEM_HASH) {
-    k_match_prep<true><<<pgrid, kPrepThreads, 0, s>>>(a);
-    k_match_first<true, true><<<fgrid, kPrepThreads, 0, s>>>(a);
-    k_match_first<true, false><<<fgrid, kPrepThreads, 0, s>>>(a);
-  } else {
-    k_match_prep<false><<<pgrid, kPrepThreads, 0, s>>>(a);
-    k_match_first<false, true><<<fgrid, kPrepThreads, 0, s>>>(a);
-    k_match_first<false, false><<<fgrid, kPrepThreads, 0, s>>>(a);
+  a.span = (int)std::max<int64_t>(32, std::min<int64_t>(kSpan, n / ((int64_t)pgrid * kPrepThreads) * 32));
+  const unsigned fgrid = (unsigned)std::min<int64_t>((int64_t)ctx->num_sms * 8, std::max<int64_t>(want * 4, pgrid));
+  if (hash) k_match_prep<true><<<pgrid, kPrepThreads, 0, s>>>(a);
+  else k_match_prep<false><<<pgrid, kPrepThreads, 0, s>>>(a);
+  if (max_deg > kSerialDeg) {
+    if (hash) {
+      k_match_first<true, true><<<fgrid, kPrepThreads, 0, s>>>(a);
+      k_match_first<true, false><<<fgrid, kPrepThreads, 0, s>>>(a);
+    } else {
+      k_match_first<false, true><<<fgrid, kPrepThreads, 0, s>>>(a);
+      k_match_first<false, false><<<fgrid, kPrepThreads, 0, s>>>(a);
+    }
+    ctx->launches += 2;
   }
-  ctx->launches += 3;
-  cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kMatchThreads), args, 0, s);
-  if (e != cudaSuccess) {
-    stage_end(ctx, CM_STAGE_MATCH, s);
-    return cuda_status(e, "cm_match launch");
-  }
-  k_match_finish<<<(unsigned)std::min<int64_t>((int64_t)ctx->num_sms * 4, n / 256 + 1), 256, 0, s>>>(n, d_match);
-  stage_end(ctx, CM_STAGE_MATCH, s);
+  if (hash) k_match_propose<true><<<pgrid, kPrepThreads, 0, s>>>(a);
+  else k_match_propose<false><<<pgrid, kPrepThreads, 0, s>>>(a);
   ctx->launches += 2;
-  return CM_OK;
+  cudaError_t e = cudaSuccess;
+  if (rounds && one_pass) {
+    if (hash) k_match_rounds<true, true><<<grid, kMatchThreads, 0, s>>>(a);
+    else k_match_rounds<false, true><<<grid, kMatchThreads, 0, s>>>(a);
+    ctx->launches++;
+  } else if (rounds) {
+    e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kMatchThreads), args, 0, s);
+    ctx->launches++;
+  }
+  const unsigned vgrid = (unsigned)std::min<int64_t>((int64_t)ctx->num_sms * 8, n / kPrepThreads + 1);
+  if (hash) k_match_finish<true><<<vgrid, kPrepThreads, 0, s>>>(a, alone);
+  else k_match_finish<false><<<vgrid, kPrepThreads, 0, s>>>(a, alone);
+  ctx->launches++;
+  if (e == cudaSuccess && !alone) {
+    e = cudaLaunchCooperativeKernel(hfn, dim3(grid), dim3(kMatchThreads), args, 0, s);
+    ctx->launches++;
+  }
+  stage_end(ctx, CM_STAGE_MATCH, s);
+  return cuda_status(e != cudaSuccess ? e : cudaGetLastError(), "cm_match launch");
 }
 
 }  // namespace cm

@@ -51,13 +51,13 @@ enum {
 /* ---- matching modes ---------------------------------------------------- */
 enum {
   /* Heavy-edge matching, deterministic: every vertex prefers its heaviest
-   * eligible neighbour, ties to the lower vertex id; conflicts resolved by
-   * mutual-proposal handshakes iterated to a fixed point.  The result equals
-   * the sequential greedy matching over eligible edges sorted by
-   * (weight desc, min endpoint asc, max endpoint asc). */
+   * eligible neighbour, ties to the lower vertex id; a vertex keeps the best
+   * proposal it receives and the one it gives up goes on to its next
+   * candidate.  The result equals the sequential greedy matching over eligible
+   * edges sorted by (weight desc, min endpoint asc, max endpoint asc). */
   CM_MATCH_HEM = 0,
   /* Same, but equal weights are ordered by a fixed hash of the edge's
-   * endpoints (fewer handshake rounds on unit-weight meshes). */
+   * endpoints (shorter chains of displaced proposals on unit-weight meshes). */
   CM_MATCH_HEM_HASH = 1,
   /* One unsynchronised proposal pass plus cleanup, like cuMetis.cu:1563-1630
    * (cuda_shem2, cuda_cleanv, findc1): a light vertex that nobody claimed
@@ -156,11 +156,10 @@ int cm_ctx_set_stage_timing(cm_ctx *ctx, int enable);
  * GPU, and sleeping measured 8% slower there. */
 int cm_ctx_set_blocking_waits(cm_ctx *ctx, int enable);
 /* Matching trace: with max_rounds > 0 the next cm_match / cm_coarsen levels
- * record, per handshake round, device timestamps (ns) of the phase starts and
- * the round's work sizes.  cm_ctx_match_trace copies rows of 8 int64 of the
- * last matching: row 0 = {kernel start, init done, round-0 start, end,
- * rounds, 0, 0, 0}; row r+1 = {phase A, phase B, phase C, round end,
- * lane-sized rows, chunked rows, row chunks, wake chunks}.  0 disables. */
+ * record, per round of row rescans, device timestamps (ns) and the round's
+ * work sizes.  cm_ctx_match_trace copies rows of 8 int64 of the last matching:
+ * row 0 = {kernel start, init done, 0, end, rounds, 0, 0, 0}; row r+1 =
+ * {round start, 0, 0, round end, 0, rows, row chunks, 0}.  0 disables. */
 int cm_ctx_set_match_trace(cm_ctx *ctx, int32_t max_rounds);
 int cm_ctx_match_trace(cm_ctx *ctx, int64_t *out, int32_t cap_rows, int32_t *rows_out);
 int cm_ctx_stage_times(cm_ctx *ctx, double *ms, int32_t cap, int reset);
@@ -173,7 +172,10 @@ const char *cm_stage_name(int32_t stage);
  * 3*vwgt[v] < maxvwgt or 3*vwgt[k] < maxvwgt (cuMetis.cu:1570, 1583).
  * On return d_match[v] = partner, or v for a singleton (match is an
  * involution).  *rounds_out (optional host pointer) receives the number of
- * handshake rounds. The fine graph is not modified. */
+ * passes over the vertices that had to be scanned again.  The fine graph is
+ * not modified.  The adjacency should be symmetric with equal weights
+ * (cm_graph_validate); for one that is not, the matching is that of mutual
+ * proposals (each end the other's best unmatched neighbour, repeated). */
 int cm_match(cm_ctx *ctx, const cm_graph *g_dev, int32_t maxvwgt, int32_t mode,
              int32_t *d_match, int32_t *rounds_out, void *stream);
 

@@ -20,12 +20,12 @@
 //   3. boundary vertices grouped by target part -- here in vertex-id order
 //      within a part (a stable counting sort), where the reference's
 //      segmented sort leaves equal targets in an unspecified order;
-//   4. per target part one thread walks its group in order and moves a vertex
+//   4. per target part one block takes its group in order and moves a vertex
 //      when both parts stay inside their windows: first the moves towards a
 //      higher part id, then (second launch) towards a lower one.
-//      Part weights are updated with atomics while the part threads run, as
-//      in the reference, so concurrent groups see each other's moves in
-//      whatever order the hardware interleaves them.
+//      Part weights are updated with atomics while the other parts' blocks
+//      run, as by the reference's part threads, so concurrent groups see each
+//      other's moves in whatever order the hardware interleaves them.
 #include <algorithm>
 #include <chrono>
 #include <climits>
@@ -237,58 +237,188 @@ __global__ void k_part_starts(int nparts, const int *__restrict__ pcount, int *_
 
 // One warp per block of kSortBlock entries, in order: an entry's place is its
 // part's start + the block's offset for the part + its rank among the part's
-// earlier entries in the block.
-__global__ void k_sort_scatter(const int *__restrict__ d_nb, const int *__restrict__ bnd_v,
-                               const int *__restrict__ bnd_t, int nparts, int *__restrict__ bhist,
-                               const int *__restrict__ pstart, int *__restrict__ sorted_v) {
+// earlier entries in the block (running counts in shared memory up to
+// kSmemParts parts, so that the steps do not wait for global reads of each
+// other's counts).  The sorted record holds what the moves need -- vertex,
+// weight, part -- so that the walks read memory in order.
+__global__ void __launch_bounds__(32)
+k_sort_scatter(const int *__restrict__ d_nb, const int *__restrict__ bnd_v, const int *__restrict__ bnd_t, int nparts,
+               int *__restrict__ bhist, const int *__restrict__ pstart, const int *__restrict__ vwgt,
+               const int *__restrict__ where, int4 *__restrict__ sorted) {
+  extern __shared__ int s_cnt[];
   const int nb = *d_nb;
   const int lane = threadIdx.x & 31;
   const long long b = blockIdx.x;
   const long long lo = b * kSortBlock, hi = min((long long)nb, lo + kSortBlock);
+  if (lo >= hi) return;
   int *cnt = bhist + b * nparts;
-  for (long long i0 = lo; i0 < hi; i0 += 32) {
-    const long long i = i0 + lane;
-    const bool ok = i < hi;
-    const int t = ok ? bnd_t[i] : -1;
-    const unsigned m = __match_any_sync(0xffffffffu, t);
-    const int rank = __popc(m & ((1u << lane) - 1));
-    int base = 0;
-    if (ok) base = cnt[t];
+  if (nparts <= kSmemParts) {
+    for (int t = lane; t < nparts; t += 32) s_cnt[t] = cnt[t] + pstart[t];
     __syncwarp();
-    if (ok) {
-      sorted_v[pstart[t] + base + rank] = bnd_v[i];
-      if (rank == 0) cnt[t] = base + __popc(m);
+  }
+  constexpr int kAhead = 4;  // steps whose loads are in flight together
+  for (long long i0 = lo; i0 < hi; i0 += 32 * kAhead) {
+    int t[kAhead], v[kAhead], vw[kAhead], me[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const long long i = i0 + 32 * u + lane;
+      t[u] = i < hi ? bnd_t[i] : -1;
+      v[u] = i < hi ? bnd_v[i] : 0;
     }
-    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      vw[u] = t[u] >= 0 ? vwgt[v[u]] : 0;
+      me[u] = t[u] >= 0 ? where[v[u]] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const unsigned m = __match_any_sync(0xffffffffu, t[u]);
+      const int rank = __popc(m & ((1u << lane) - 1));
+      int base = 0;
+      if (t[u] >= 0) base = nparts <= kSmemParts ? s_cnt[t[u]] : pstart[t[u]] + cnt[t[u]];
+      __syncwarp();
+      if (t[u] >= 0) {
+        sorted[base + rank] = make_int4(v[u], vw[u], me[u], 0);
+        if (rank == 0) {
+          if (nparts <= kSmemParts) s_cnt[t[u]] = base + __popc(m);
+          else cnt[t[u]] += __popc(m);
+        }
+      }
+      __syncwarp();
+    }
   }
 }
 
-// One thread per target part walks its group in order (Exnode_part1 when
-// kUp, moves to a higher-or-equal part id; Exnode_part2 otherwise).
+// The group of target part `to` (blockIdx.x) in order (Exnode_part1 when kUp:
+// moves to a higher part id; Exnode_part2 otherwise): a vertex moves when part
+// to stays within [tomin, tomax] with it and its own part within its window
+// without it, given the moves before it.
+//
+// A walk vertex by vertex waits for several memory trips each (10.7 ms a phase
+// for an R-MAT 17 bisection, 0.49 ms for a 1000 x 1000 grid in 64 parts; a whole
+// pass went from 17.4 to 0.53 ms and from 0.86 to 0.26 ms), although most
+// stretches of a group are moved or refused as a whole.  So the block takes
+// kMoveThreads records at a time and settles them together when it can:
+//   - everyone moves: the weights leave their parts by atomics that return what
+//     was left; if every part stayed above its lower limit (and was not above
+//     its upper one before) and the sum fits part to, each vertex alone was
+//     allowed in order, for weights >= 0;
+//   - everyone is refused: nobody fits as the weights are now, and refusals
+//     change no weight.
+// Else the first warp settles the records in order, 32 at a time, by stretches:
+// the longest prefix that moves, then the longest that is refused.  Either way
+// the outcome for two parts is that of the walk; with more parts the blocks
+// race as the reference's threads do, but a lower limit is never crossed, since
+// a weight that would cross it is put back.
+constexpr int kMoveThreads = 512;
 template <bool kUp>
-__global__ void k_moves(int nparts, const int *__restrict__ pstart, const int *__restrict__ sorted_v,
-                        const int *__restrict__ vwgt, const int *__restrict__ maxw, const int *__restrict__ minw,
-                        int *pwgts, int *where, unsigned long long *moves) {
-  const int to = blockIdx.x * blockDim.x + threadIdx.x;
-  if (to >= nparts) return;
-  unsigned long long nm = 0;
+__global__ void __launch_bounds__(kMoveThreads)
+k_moves(const int *__restrict__ pstart, const int4 *__restrict__ sorted, const int *__restrict__ maxw,
+        const int *__restrict__ minw, int *pwgts, int *where, unsigned long long *moves) {
+  __shared__ int4 s_rec[kMoveThreads];
+  __shared__ int s_warp[kMoveThreads / 32], s_sum, s_pto;
+  const int to = blockIdx.x;
+  const bool racing = gridDim.x > 2;  // other blocks may take from the same parts
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tomax = maxw[to], tomin = minw[to];
-  for (int i = pstart[to]; i < pstart[to + 1]; ++i) {
-    const int v = sorted_v[i];
-    const int vw = vwgt[v];
-    const int me = where[v];
+  const int i0 = pstart[to], i1 = pstart[to + 1];
+  volatile int *pw = pwgts;
+  unsigned long long nm = 0;
+  const int4 none = make_int4(-1, 0, to, 0);
+  int4 next = i0 + (int)threadIdx.x < i1 ? sorted[i0 + threadIdx.x] : none;
+  for (int b = i0; b < i1; b += kMoveThreads) {
+    const int4 r = next;
+    next = b + kMoveThreads + (int)threadIdx.x < i1 ? sorted[b + kMoveThreads + threadIdx.x] : none;
+    const int me = r.z, vw = r.y;
     // me == to would add and remove the same weight: a no-op move, skipped
     // (the reference applies it, leaving a transient in pwgts[me]).
-    if (kUp ? (me >= to) : (me <= to)) continue;
-    const int pto = *(volatile int *)&pwgts[to], pme = *(volatile int *)&pwgts[me];
-    if (pto + vw >= tomin && pto + vw <= tomax && pme - vw >= minw[me] && pme - vw <= maxw[me]) {
-      atomicAdd(&pwgts[to], vw);
-      atomicSub(&pwgts[me], vw);
-      where[v] = to;
-      ++nm;
+    const bool cand = kUp ? me < to : me > to;
+    if (threadIdx.x == 0) s_pto = pw[to];  // one value for all: other blocks may change it
+    if (!__syncthreads_or(cand)) continue;
+    const int pto = s_pto, pme = cand ? pw[me] : 0;
+    const int lo = cand ? minw[me] : 0, hi = cand ? maxw[me] : 0;
+    const bool fits = cand && pto + vw >= tomin && pto + vw <= tomax && pme - vw >= lo && pme - vw <= hi;
+    if (!__syncthreads_or(fits)) continue;  // everyone is refused
+    const int total = __reduce_add_sync(0xffffffffu, cand ? vw : 0);
+    if (lane == 0) s_warp[warp] = total;
+    const bool plain = !cand || (vw >= 0 && vw < (1 << 20) && fits && pme <= hi);
+    if (__syncthreads_and(plain)) {
+      if (threadIdx.x == 0) {
+        int t = 0;
+        for (int w = 0; w < kMoveThreads / 32; ++w) t += s_warp[w];
+        s_sum = t;  // below 2^29
+      }
+      __syncthreads();
+      const int sum = s_sum;
+      if ((long long)pto + sum <= tomax) {
+        const bool ok = !cand || atomicSub(&pwgts[me], vw) - vw >= lo;
+        if (__syncthreads_and(ok)) {
+          if (cand) {
+            where[r.x] = to;
+            ++nm;
+          }
+          if (threadIdx.x == 0) {
+            atomicAdd(&pwgts[to], sum);
+            __threadfence();
+          }
+          __syncthreads();
+          continue;
+        }
+        if (cand) atomicAdd(&pwgts[me], vw);
+      }
     }
+    s_rec[threadIdx.x] = r;
+    __threadfence();
+    __syncthreads();
+    if (warp == 0) {
+      for (int c = 0; c < kMoveThreads && b + c < i1; c += 32) {
+        const int4 x = s_rec[c + lane];
+        unsigned left = __ballot_sync(0xffffffffu, kUp ? x.z < to : x.z > to);
+        while (left) {
+          const bool mine = left >> lane & 1u;
+          const int p = pw[to], q = mine ? pw[x.z] : 0;
+          const int qlo = mine ? minw[x.z] : 0, qhi = mine ? maxw[x.z] : 0;
+          // weights before each vertex if all of `left` move
+          int before = 0, gone = 0;
+          for (int j = 0; j < 32; ++j) {
+            const int wj = __shfl_sync(0xffffffffu, x.y, j), mj = __shfl_sync(0xffffffffu, x.z, j);
+            if ((left >> j & 1u) && j < lane) {
+              before += wj;
+              if (mj == x.z) gone += wj;
+            }
+          }
+          const int pt = p + before + x.y, pm = q - gone - x.y;
+          const bool ok = pt >= tomin && pt <= tomax && pm >= qlo && pm <= qhi;
+          const unsigned bad = __ballot_sync(0xffffffffu, mine && !ok);
+          const unsigned go = bad ? left & ((1u << (__ffs(bad) - 1)) - 1u) : left;
+          if (go) {
+            bool moved = go >> lane & 1u;
+            if (moved && atomicSub(&pwgts[x.z], x.y) - x.y < qlo && racing && x.y > 0) {  // another block came first
+              atomicAdd(&pwgts[x.z], x.y);
+              moved = false;
+            }
+            const int sum = __reduce_add_sync(0xffffffffu, moved ? x.y : 0);
+            if (lane == 0 && sum) atomicAdd(&pwgts[to], sum);
+            if (moved) {
+              where[x.x] = to;
+              ++nm;
+            }
+            left &= ~go;
+            __threadfence();
+            __syncwarp();
+          } else {
+            // the first is refused, and with it everyone up to the next that fits as things are
+            const bool fit = mine && p + x.y >= tomin && p + x.y <= tomax && q - x.y >= qlo && q - x.y <= qhi;
+            const unsigned yes = __ballot_sync(0xffffffffu, fit) & ~(left & (0u - left));
+            left = yes ? left & ~((1u << (__ffs(yes) - 1)) - 1u) : 0u;
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
-  if (nm) atomicAdd(moves, nm);
+  const int n32 = (int)__reduce_add_sync(0xffffffffu, (unsigned)nm);
+  if (lane == 0 && n32) atomicAdd(moves, (unsigned long long)n32);
 }
 
 __global__ void k_project(int n, const int *__restrict__ cmap, const int *__restrict__ cwhere,
@@ -315,7 +445,8 @@ __global__ void k_cut(int n, const int *__restrict__ xadj, const int *__restrict
 }
 
 struct RefineWs {
-  int *pwgts, *maxw, *minw, *flag, *target, *pos, *bnd_v, *bnd_t, *sorted_v, *bhist, *pcount, *pstart, *acc;
+  int *pwgts, *maxw, *minw, *flag, *target, *pos, *bnd_v, *bnd_t, *bhist, *pcount, *pstart, *acc;
+  int4 *sorted;  // boundary records (vertex, weight, part, 0) by target part
   unsigned long long *lb, *counters;  // counters[0] = moves, [1] = cut
   size_t bhist_ints, acc_ints, lb_words;
 };
@@ -326,7 +457,7 @@ size_t refine_ws_bytes(cm_ctx *ctx, int64_t n, int nparts) {
   const int64_t nblocks = (n + kSortBlock - 1) / kSortBlock + 1;
   size_t b = 0;
   b += (size_t)(3 * nparts + 2 * (nparts + 1)) * 4 + 5 * 256;
-  b += (size_t)(6 * n + 8) * 4 + 6 * 256;
+  b += (size_t)(9 * n + 8) * 4 + 6 * 256;
   b += (size_t)nblocks * nparts * 4 + 256;
   if (nparts > kSmemParts) b += (size_t)grid_warps(ctx) * nparts * 4 + 256;
   b += (size_t)(n / (kScanThreads * kScanItems) + 4) * 8 + 256 + 64;
@@ -345,7 +476,7 @@ int take_refine_ws(cm_ctx *ctx, int64_t n, int nparts, RefineWs &w) {
   w.pos = (int *)ws_take(ctx, (size_t)(n + 1) * 4);
   w.bnd_v = (int *)ws_take(ctx, (size_t)n * 4 + 4);
   w.bnd_t = (int *)ws_take(ctx, (size_t)n * 4 + 4);
-  w.sorted_v = (int *)ws_take(ctx, (size_t)n * 4 + 4);
+  w.sorted = (int4 *)ws_take(ctx, (size_t)n * 16 + 16);
   w.bhist_ints = (size_t)nblocks * nparts;
   w.bhist = (int *)ws_take(ctx, w.bhist_ints * 4);
   w.acc_ints = nparts > kSmemParts ? (size_t)grid_warps(ctx) * nparts : 0;
@@ -354,7 +485,7 @@ int take_refine_ws(cm_ctx *ctx, int64_t n, int nparts, RefineWs &w) {
   w.lb = (unsigned long long *)ws_take(ctx, w.lb_words * 8);
   w.counters = (unsigned long long *)ws_take(ctx, 64);
   if (!w.pwgts || !w.maxw || !w.minw || !w.pcount || !w.pstart || !w.flag || !w.target || !w.pos || !w.bnd_v ||
-      !w.bnd_t || !w.sorted_v || !w.bhist || (w.acc_ints && !w.acc) || !w.lb || !w.counters)
+      !w.bnd_t || !w.sorted || !w.bhist || (w.acc_ints && !w.acc) || !w.lb || !w.counters)
     return cm_fail(CM_ERR_NOMEM, "refine: workspace too small");
   return CM_OK;
 }
@@ -391,12 +522,10 @@ int refine_pass(cm_ctx *ctx, const cm_graph &g, int nparts, int32_t *where, Refi
   k_sort_counts<<<sort_blocks, 256, 0, s>>>(d_nb, w.bnd_t, nparts, w.bhist);
   k_sort_offsets<<<(nparts + 255) / 256, 256, 0, s>>>(d_nb, nparts, w.bhist, w.pcount);
   k_part_starts<<<1, 1024, 0, s>>>(nparts, w.pcount, w.pstart);
-  k_sort_scatter<<<sort_blocks, 32, 0, s>>>(d_nb, w.bnd_v, w.bnd_t, nparts, w.bhist, w.pstart, w.sorted_v);
-  const int mb = (nparts + 127) / 128;
-  k_moves<true><<<mb, 128, 0, s>>>(nparts, w.pstart, w.sorted_v, g.vwgt, w.maxw, w.minw, w.pwgts, where,
-                                   w.counters);
-  k_moves<false><<<mb, 128, 0, s>>>(nparts, w.pstart, w.sorted_v, g.vwgt, w.maxw, w.minw, w.pwgts, where,
-                                    w.counters);
+  k_sort_scatter<<<sort_blocks, 32, nparts <= kSmemParts ? nparts * 4 : 0, s>>>(
+      d_nb, w.bnd_v, w.bnd_t, nparts, w.bhist, w.pstart, g.vwgt, where, w.sorted);
+  k_moves<true><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, where, w.counters);
+  k_moves<false><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, where, w.counters);
   ctx->launches += 11;
   return check_launch(ctx, "refine");
 }

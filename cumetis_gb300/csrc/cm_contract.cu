@@ -12,19 +12,17 @@
 // loop cmap[x] == c, is sorted ascending by coarse id, and equal ids are merged
 // with their weights summed (int32, wrapping).
 //
-// Every sort is a shared-memory LSD radix sort with private per-thread digit
-// counters (cm_sort.cuh), sized to the row: no comparison network, no hash,
-// no atomics in the ranking.  Work split by expanded coarse-row length
-// L = deg(leader) + deg(follower):
+// Work split by expanded coarse-row length L = deg(leader) + deg(follower):
 //   L <= kTinyMax     : tiny units, one warp each.  Unit k owns the rows
 //                       whose diagonal (rows before + tiny entries before)
 //                       lies in [kD, (k+1)D) (D = kTinyDiag), so it holds
-//                       < D + kTinyMax entries of <= D/2 rows; their
-//                       (row, coarse id) keys are sorted together.
+//                       < D + kTinyMax entries of <= D/2 rows; every row is
+//                       bucket sorted in its share of the unit's buckets.
 //   kTinyMax < L <= kChunk : one block per row, sized to the row's class
 //                       (two classes per octave, capacities 1.5 and 2 times
 //                       a power of two, from 96 to kChunk entries; one warp
-//                       up to 512 entries), coarse-id keys only.
+//                       up to 512 entries): a shared-memory LSD radix sort of
+//                       the coarse ids (cm_sort.cuh).
 //   L > kChunk        : huge rows.  Chunks of kChunk entries are sorted,
 //                       merged pairwise (merge path, one launch per pass) and
 //                       deduplicated.
@@ -56,11 +54,10 @@ constexpr int kTinyMax = CM_TINY_MAX;
 #endif
 constexpr int kTinyDiag = CM_TINY_DIAG;
 constexpr int kTinyCap = (kTinyDiag + kTinyMax + 31) / 32 * 32;
-static_assert(kTinyDiag % 32 == 0 && kTinyDiag >= 2 * kTinyMax && kTinyCap <= 512, "CM_TINY_DIAG");
+static_assert(kTinyDiag % 32 == 0 && kTinyDiag >= 2 * kTinyMax && kTinyCap <= 256, "CM_TINY_DIAG");
 constexpr int kTinyItems = kTinyCap / 32;
 constexpr int kTinyRowsPerLane = kTinyDiag / 32;
 constexpr int kTinyMaxNz = kTinyDiag / 2;
-constexpr int kTinyRowBits = ilog2(kTinyMaxNz - 1) + 1;
 static_assert(kTinyMax == 16 || kTinyMax == 32 || kTinyMax == 64, "CM_TINY_MAX: 16, 32 or 64");
 // Rows longer than kChunk are sorted in kChunk-entry chunks and merged.
 #ifndef CM_CHUNK
@@ -348,25 +345,34 @@ k_unit_map(const int *d_cn, const int *__restrict__ eoff, int *__restrict__ firs
 // ---------------------------------------------------------------------------
 // Tiny units: one warp each
 // ---------------------------------------------------------------------------
-template <typename K>
 struct TinySmem {
-  SortPair<K> work[rslots(kTinyCap)];
-  SortScratch<32> sc;
-  int4 rmeta[kTinyMaxNz];  // per non-empty row: first entry in the unit, leader row start and length, follower row start
+  SortPair<unsigned> work[kTinyCap];        // (id, weight): gathered order, then bucket order, then sorted
+  __align__(16) int start[kTinyCap + 4];    // entries per bucket, then the buckets' first places
+  int4 rmeta[kTinyMaxNz];                   // per non-empty row: first entry in the unit, leader row start and length, follower row start
+  uint2 rmap[kTinyMaxNz];                   // ... its id -> bucket map: lowest id, scale
   int rcount[kTinyMaxNz], rfirst[kTinyMaxNz], rdst[kTinyMaxNz];
-  unsigned char rowid[kTinyCap];  // sorted row of every gathered entry
+  unsigned char rowid[kTinyCap];            // row of every gathered entry, then of every sorted one
   unsigned char nz_row[kTinyMaxNz];
-  int ctr;
 };
 static_assert(kTinyMaxNz <= 256 && kTinyDiag <= 256, "tiny unit row ids are 8-bit");
 
 // One warp per unit (grid-stride over the units).  Per unit: the rows'
 // metadata, every entry's row (a max-scan of the rows' first entries), the
-// gather of (row << idbits | coarse id, weight) pairs without self loops, a
-// radix sort of the keys, and every run of equal keys written once, weights
-// summed, to stage[eoff[c] ...) of its row; ucount[c] = the row's unique
-// entries (0 for empty rows; rows above kTinyMax are counted by their class).
-template <typename K>
+// gather of (coarse id, weight) pairs without self loops, the sort of every
+// row, and every run of equal ids written once, weights summed, to
+// stage[eoff[c] ...) of its row; ucount[c] = the row's unique entries (0 for
+// empty rows; rows above kTinyMax are counted by their class).
+//
+// The sort: a row of L entries has L buckets, its share of one array of
+// counters, and an id goes to the bucket at its place between the lowest and
+// the highest of four of the row's ids (the ends of its two fine rows; ids
+// beyond them go to the end buckets).  An atomic count per entry, one scan of
+// all counters and one scatter leave the entries in bucket order; an entry
+// then finds its place among the few of its bucket by comparing with them.
+// The work does not depend on the width of the ids; the radix sort of (row, id)
+// keys that this replaces took a pass per 4 bits, seven for 22-bit ids (R-MAT
+// 22: 472 -> 298 us, a weighted 101^3 grid's levels: 549 -> 380 us).  Bound by
+// issue and shared-memory latency at 32 resident warps per SM.
 __global__ void __launch_bounds__(32)
 k_tiny_units(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
              const int *d_sizes, const int *__restrict__ first_row, const int *unit_last,
@@ -374,13 +380,11 @@ k_tiny_units(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
              int *__restrict__ ucount, DevStatus *st) {
   constexpr int RPL = kTinyRowsPerLane;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  TinySmem<K> &S = *reinterpret_cast<TinySmem<K> *>(smem_raw);
+  TinySmem &S = *reinterpret_cast<TinySmem *>(smem_raw);
   const int lane = threadIdx.x;
   const unsigned below = lanemask_lt();
   const int nc = d_sizes[0];
   const int last = *unit_last;
-  const int idbits = id_bits(nc);
-  const unsigned idmask = idbits >= 32 ? 0xffffffffu : ((1u << idbits) - 1u);
   for (int u = blockIdx.x; u <= last; u += gridDim.x) {
     const int clo = first_row[u];
     const int chi = u < last ? first_row[u + 1] : nc;
@@ -425,8 +429,10 @@ k_tiny_units(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
         ex += (1 << 16) + len[i];
       }
     }
-    for (int e = lane; e < kTinyCap; e += 32) S.rowid[e] = 0;
-    if (lane == 0) S.ctr = 0;
+    for (int e = lane; e < kTinyCap; e += 32) {
+      S.rowid[e] = 0;
+      S.start[e] = 0;
+    }
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < RPL; ++i)
@@ -455,17 +461,18 @@ k_tiny_units(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
       }
     }
     __syncwarp();
-    // ---- gather (row << idbits | coarse id, weight), self loops dropped
+    // ---- gather (coarse id, weight); at[q] = the entry's row, -1 for none or a self loop
+    int x[kTinyItems], w[kTinyItems], at[kTinyItems];
     {
-      int src[kTinyItems], x[kTinyItems], w[kTinyItems], jj[kTinyItems];
+      int src[kTinyItems];
 #pragma unroll
       for (int q = 0; q < kTinyItems; ++q) {
         const int e = q * 32 + lane;
         src[q] = -1;
-        jj[q] = 0;
+        at[q] = -1;
         if (e < ntot) {
           const int j = S.rowid[e];
-          jj[q] = j;
+          at[q] = j;
           const int4 r = S.rmeta[j];
           src[q] = expanded_src(e - r.x, r.y, r.z, r.w);
         }
@@ -476,33 +483,93 @@ k_tiny_units(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
         w[q] = src[q] >= 0 ? __ldcs(adjwgt + src[q]) : 0;
       }
 #pragma unroll
-      for (int q = 0; q < kTinyItems; ++q) x[q] = src[q] >= 0 ? cmap[x[q]] : -1;
+      for (int q = 0; q < kTinyItems; ++q)
+        if (src[q] >= 0) x[q] = cmap[x[q]];
+    }
 #pragma unroll
-      for (int q = 0; q < kTinyItems; ++q) {
-        const bool keep = src[q] >= 0 && x[q] != clo + (int)S.nz_row[jj[q]];
-        append_pair<K>(S.work, &S.ctr, keep, ((K)jj[q] << idbits) | (K)(unsigned)x[q], w[q]);
+    for (int q = 0; q < kTinyItems; ++q)
+      if (at[q] >= 0) S.work[q * 32 + lane].k = (unsigned)x[q];
+    __syncwarp();
+    // ---- every row's id -> bucket map
+    for (int j = lane; j < nnz; j += 32) {
+      const int e0 = S.rmeta[j].x, dl = S.rmeta[j].z;
+      const int L = (j + 1 < nnz ? S.rmeta[j + 1].x : ntot) - e0;
+      const unsigned a0 = S.work[e0].k, a1 = S.work[e0 + max(dl, 1) - 1].k;
+      const unsigned b0 = S.work[e0 + min(dl, L - 1)].k, b1 = S.work[e0 + L - 1].k;
+      const unsigned lo = min(min(a0, a1), min(b0, b1)), hi = max(max(a0, a1), max(b0, b1));
+      S.rmap[j] = make_uint2(lo, bucket_scale(L, hi - lo));
+    }
+    __syncwarp();
+    // ---- count, scan, scatter in bucket order
+#pragma unroll
+    for (int q = 0; q < kTinyItems; ++q) {
+      const int j = at[q];
+      if (j < 0) continue;
+      const int c = clo + (int)S.nz_row[j];
+      at[q] = -1;
+      if (x[q] == c) continue;
+      const uint2 mp = S.rmap[j];
+      const int e0 = S.rmeta[j].x, L = (j + 1 < nnz ? S.rmeta[j + 1].x : ntot) - e0;
+      const int b = e0 + min(L - 1, bucket_of((unsigned)x[q], mp));
+      at[q] = j << 24 | b << 16 | atomicAdd(&S.start[b], 1);
+    }
+    __syncwarp();
+    int n;
+    {
+      int v[kTinyItems], sum = 0;
+#pragma unroll
+      for (int i = 0; i < kTinyItems; ++i) {
+        v[i] = sum;
+        sum += S.start[lane * kTinyItems + i];
+      }
+      const int inc = warp_inclusive_scan_i32(sum);
+      n = __shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll
+      for (int i = 0; i < kTinyItems; ++i) S.start[lane * kTinyItems + i] = inc - sum + v[i];
+      if (lane == 0) S.start[kTinyCap] = n;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < kTinyItems; ++q) {
+      if (at[q] == -1) continue;
+      const int p = S.start[at[q] >> 16 & 255] + (at[q] & 0xffff);
+      S.work[p] = make_pair_kv<unsigned>((unsigned)x[q], w[q]);
+      S.rowid[p] = (unsigned char)((unsigned)at[q] >> 24);
+    }
+    __syncwarp();
+    // ---- places within the buckets
+    unsigned crowded = 0;
+#pragma unroll
+    for (int q = 0; q < kTinyItems; ++q) {
+      if (at[q] == -1) continue;
+      const int b = at[q] >> 16 & 255, s0 = S.start[b], s1 = S.start[b + 1];
+      if (s1 - s0 > 1) {
+        at[q] = bucket_place(S.work, s0, s1, s0 + (at[q] & 0xffff), (unsigned)x[q]);
+        crowded |= 1u << q;
       }
     }
     __syncwarp();
-    const int n = S.ctr;
-    const int rowbits = nnz > 1 ? 32 - __clz(nnz - 1) : 0;
-    block_radix_sort<K, 32, kTinyItems>(S.work, S.sc, n, rowbits + idbits);
-    // ---- runs of equal keys: per sorted row, its first run's index and its
-    // number of runs; then every run to the row's stage
+#pragma unroll
+    for (int q = 0; q < kTinyItems; ++q)
+      if (crowded >> q & 1u) S.work[at[q]] = make_pair_kv<unsigned>((unsigned)x[q], w[q]);
+    __syncwarp();
+    // ---- runs of equal ids: per row, its first run's index and its number of
+    // runs; then every run to the row's stage
     unsigned hm[kTinyItems];
     int qbase = 0;
 #pragma unroll
     for (int r = 0; r < kTinyItems; ++r) {
       const int i = r * 32 + lane;
-      const K key = i < n ? S.work[i].k : (K)0;
-      const bool head = i < n && (i == 0 || S.work[i - 1].k != key);
-      hm[r] = __ballot_sync(0xffffffffu, head);
+      bool head = i < n, first = false;
+      int j = 0;
       if (head) {
-        const int j = (int)(key >> idbits);
-        const int q = qbase + __popc(hm[r] & below);
-        if (i == 0 || (int)(S.work[i - 1].k >> idbits) != j) S.rfirst[j] = q;
-        atomicAdd(&S.rcount[j], 1);
+        j = S.rowid[i];
+        first = i == 0 || S.rowid[i - 1] != j;
+        head = first || S.work[i - 1].k != S.work[i].k;
+        if (head) atomicAdd(&S.rcount[j], 1);
       }
+      hm[r] = __ballot_sync(0xffffffffu, head);
+      if (first) S.rfirst[j] = qbase + __popc(hm[r] & below);
       qbase += __popc(hm[r]);
     }
     __syncwarp();
@@ -517,12 +584,12 @@ k_tiny_units(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
     for (int r = 0; r < kTinyItems; ++r) {
       const int i = r * 32 + lane;
       if (hm[r] >> lane & 1u) {
-        const K key = S.work[i].k;
+        const unsigned key = S.work[i].k;
+        const int j = S.rowid[i];
         unsigned sum = (unsigned)S.work[i].v;
-        for (int j2 = i + 1; j2 < n && S.work[j2].k == key; ++j2) sum += (unsigned)S.work[j2].v;
-        const int j = (int)(key >> idbits);
+        for (int j2 = i + 1; j2 < n && S.work[j2].k == key && S.rowid[j2] == j; ++j2) sum += (unsigned)S.work[j2].v;
         const int q = qbase + __popc(hm[r] & below);
-        stage[S.rdst[j] + (q - S.rfirst[j])] = make_int2((int)((unsigned)key & idmask), (int)sum);
+        stage[S.rdst[j] + (q - S.rfirst[j])] = make_int2((int)key, (int)sum);
       }
       qbase += __popc(hm[r]);
     }
@@ -1019,20 +1086,14 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
     return cuda_status(cudaGetLastError(), "contract(empty)");
   }
   if (!ctx->contract_attrs_set) {  // once per context (the attributes last for the process)
-    cudaFuncSetAttribute(k_tiny_units<unsigned>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(TinySmem<unsigned>));
-    cudaFuncSetAttribute(k_tiny_units<unsigned long long>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(TinySmem<unsigned long long>));
+    cudaFuncSetAttribute(k_tiny_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TinySmem));
     cudaFuncSetAttribute(k_long_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(SegSmem<kChunkThreads, kChunkItems>));
     cudaFuncSetAttribute(k_long_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MergeSmem));
     class_attrs<0>(ctx);
-    int b32 = 0, b64 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b32, k_tiny_units<unsigned>, 32, sizeof(TinySmem<unsigned>));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b64, k_tiny_units<unsigned long long>, 32,
-                                                  sizeof(TinySmem<unsigned long long>));
-    ctx->unit_blocks_per_sm[0] = std::max(1, b32);
-    ctx->unit_blocks_per_sm[1] = std::max(1, b64);
+    int b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_tiny_units, 32, sizeof(TinySmem));
+    ctx->unit_blocks_per_sm = std::max(1, b);
     if (int rc2 = check_launch(ctx, "contract: kernel attributes")) return rc2;
     ctx->contract_attrs_set = true;
   }
@@ -1073,7 +1134,6 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
                        class_ctr, m, row_meta, s);
   if (rc) return rc;
   const int sms = ctx->num_sms;
-  const bool small_ids = n <= (1ll << (32 - kTinyRowBits));
 
   // Rows above kTinyMax on the auxiliary streams (one kernel per size class;
   // the chunked rows' sort, merge passes and dedup on the last stream), the
@@ -1116,13 +1176,9 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   k_unit_map<<<(unsigned)std::max<int64_t>(1, map_tiles), kMapThreads, 0, s>>>(d_sizes, eoff, first_row, unit_last,
                                                                                 map_lb, st);
   ctx->launches++;
-  const unsigned tiny_grid = grid_for((int64_t)sms * ctx->unit_blocks_per_sm[small_ids ? 0 : 1], nunits);
-  if (small_ids)
-    k_tiny_units<unsigned><<<tiny_grid, 32, sizeof(TinySmem<unsigned>), s>>>(
-        fine->adjncy, fine->adjwgt, cmap, d_sizes, first_row, unit_last, row_meta, eoff, stage1, ucount, st);
-  else
-    k_tiny_units<unsigned long long><<<tiny_grid, 32, sizeof(TinySmem<unsigned long long>), s>>>(
-        fine->adjncy, fine->adjwgt, cmap, d_sizes, first_row, unit_last, row_meta, eoff, stage1, ucount, st);
+  const unsigned tiny_grid = grid_for((int64_t)sms * ctx->unit_blocks_per_sm, nunits);
+  k_tiny_units<<<tiny_grid, 32, sizeof(TinySmem), s>>>(fine->adjncy, fine->adjwgt, cmap, d_sizes, first_row, unit_last,
+                                                       row_meta, eoff, stage1, ucount, st);
   ctx->launches++;
   if (any_big)
     for (int i = 0; i < cm_ctx::kAux; ++i) {

@@ -50,9 +50,9 @@ struct cm_ctx {
   // the matching kernel's resident blocks per SM (per tie order)
   bool contract_attrs_set = false;
   int match_blocks_per_sm[2] = {0, 0};
-  // resident blocks per SM of the contraction's tiny-unit kernel (32- and
-  // 64-bit keys) and of its row-class kernels
-  int unit_blocks_per_sm[2] = {1, 1};
+  // resident blocks per SM of the contraction's tiny-unit kernel and of its
+  // row-class kernels
+  int unit_blocks_per_sm = 1;
   int class_blocks_per_sm[16] = {1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1, 1};
 };
 

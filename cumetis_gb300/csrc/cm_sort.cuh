@@ -212,6 +212,31 @@ __device__ __forceinline__ void block_radix_sort(SortPair<K> *work, SortScratch<
   }
 }
 
+// Bucket sorts: an id goes to the bucket at its place between a row's lowest
+// and highest id; few ids share a bucket, and find their places in it by
+// comparing with one another.
+
+// Scale of the map from ids in [lo, lo + range] to `buckets` buckets.
+__device__ __forceinline__ unsigned bucket_scale(int buckets, unsigned range) {
+  const float f = (float)buckets * 4294967296.0f / ((float)range + 1.0f);
+  return f < 4294967040.0f ? (unsigned)f : 4294967040u;
+}
+// Bucket of id x under the map (lo, scale); not decreasing in x.  Ids above the
+// range may exceed the last bucket: the caller clamps.
+__device__ __forceinline__ int bucket_of(unsigned x, uint2 map) {
+  return (int)min(__umulhi(max(x, map.x) - map.x, map.y), 0x7fffffffu);
+}
+// Place of the pair at p (id x) among the pairs of its bucket [s0, s1): by id,
+// equal ids in their present order.
+__device__ __forceinline__ int bucket_place(const SortPair<unsigned> *work, int s0, int s1, int p, unsigned x) {
+  int place = s0;
+  for (int j = s0; j < s1; ++j) {
+    const unsigned y = work[j].k;
+    place += (y < x || (y == x && j < p)) ? 1 : 0;
+  }
+  return place;
+}
+
 // Visits the runs of equal keys of the sorted pairs s[0..n): for each run,
 // emit(key, sum of the run's values (wrapping like int atomicAdd), q) with q
 // the run's index in key order.  Returns the number of runs.  n <= NT * 32.

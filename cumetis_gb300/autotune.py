@@ -35,16 +35,8 @@ PARAMS = [
     ("CM_TINY_MAX", 64, [16, 32, 64], "cm_contract.cu"),    # rows sorted in one-warp batches; larger rows by size class
     ("CM_CHUNK", 16384, [8192, 16384], "cm_contract.cu"),    # huge-row segment (chunk) size
     ("CM_CHUNK_THREADS", 1024, [512, 1024], "cm_contract.cu"),  # threads sorting one chunk
-    ("CM_CLASS_ITEMS", 16, [8, 16], "cm_contract.cu"),        # entries per thread of the size-class blocks
+    ("CM_CLASS_ITEMS", 8, [4, 8], "cm_contract.cu"),          # entries per thread of the size-class blocks
     ("CM_MERGE_THREADS", 256, [256, 512], "cm_contract.cu"),
-    # resident blocks per SM asked of the compiler for a size-class shape (0: no launch bound)
-    ("CM_MB_32_12", 32, [0, 32], "cm_contract.cu"),
-    ("CM_MB_32_16", 22, [0, 22, 28], "cm_contract.cu"),
-    ("CM_MB_64_16", 13, [0, 13, 16], "cm_contract.cu"),
-    ("CM_MB_128_12", 9, [0, 9, 12], "cm_contract.cu"),
-    ("CM_MB_128_16", 6, [0, 6, 8], "cm_contract.cu"),
-    ("CM_MB_256_16", 3, [0, 3, 4], "cm_contract.cu"),
-    ("CM_MB_512_16", 2, [0, 2], "cm_contract.cu"),
 ]
 DEFAULTS = {name: d for name, d, _, _ in PARAMS}
 SOURCE = {name: src for name, _, _, src in PARAMS}
@@ -54,8 +46,7 @@ CHECK_TESTS = "test_long_rows or test_contract_bitexact or test_coarsen_hierarch
 def valid(cfg):
     """The sources' static constraints on combinations."""
     return (cfg["CM_CHUNK"] // cfg["CM_TINY_MAX"] <= 256  # at most sixteen size classes
-            and cfg["CM_CHUNK"] // cfg["CM_CHUNK_THREADS"] <= 16  # at most 16 pairs per thread of a chunk sort
-            and cfg["CM_CHUNK"] // cfg["CM_CLASS_ITEMS"] <= 1024)  # the largest class's block fits 1024 threads
+            and cfg["CM_CHUNK"] // cfg["CM_CHUNK_THREADS"] <= 16)  # at most 16 pairs per thread of a chunk sort
 
 
 def defines_by_source(cfg):

@@ -75,20 +75,22 @@ static_assert(kChunkItems >= 1 && kChunkItems <= 16 && kChunkItems * kChunkThrea
 // holds the rows of kTinyMax 2^j < L <= 1.5 kTinyMax 2^j entries, class 2j+1
 // those up to kTinyMax 2^(j+1).  A class's block has max(32, cap / items)
 // threads, items = kClassItems for the power-of-two capacities and 3/4 of it
-// for the others.
+// for the others; the classes that would need more than 1024 threads are
+// radix sorted by 1024 threads of 12 or 16 items.
 #ifndef CM_CLASS_ITEMS
-#define CM_CLASS_ITEMS 16
+#define CM_CLASS_ITEMS 8
 #endif
 constexpr int kClassItems = CM_CLASS_ITEMS;
-static_assert(kClassItems == 4 || kClassItems == 8 || kClassItems == 16, "CM_CLASS_ITEMS: 4, 8 or 16");
+static_assert(kClassItems == 4 || kClassItems == 8, "CM_CLASS_ITEMS: 4 or 8");
 constexpr int kClasses = 2 * ilog2(kChunk / kTinyMax);
 static_assert(kClasses <= kRowClasses, "row classes");
 constexpr int class_cap_entries(int k) {
   return (k & 1) ? (kTinyMax << ((k >> 1) + 1)) : (3 * (kTinyMax << (k >> 1))) / 2;
 }
 constexpr int class_item_target(int k) { return (k & 1) ? kClassItems : (3 * kClassItems) / 4; }
+constexpr bool class_radix(int k) { return class_cap_entries(k) / class_item_target(k) > 1024; }
 constexpr int class_threads(int k) {
-  return class_cap_entries(k) / class_item_target(k) < 32 ? 32 : class_cap_entries(k) / class_item_target(k);
+  return class_radix(k) ? 1024 : class_cap_entries(k) / class_item_target(k) < 32 ? 32 : class_cap_entries(k) / class_item_target(k);
 }
 // Rows above kCopySplit expanded entries are copied one warp per row, the
 // others 32 rows per warp.
@@ -162,63 +164,17 @@ __device__ __forceinline__ int segment_sorted_unique(SegSmem<NT, ITEMS> &S, int 
   __syncthreads();
   const int n = S.ctr;
   block_radix_sort<unsigned, NT, ITEMS>(S.work, S.sc, n, idbits);
-  return block_unique_emit<unsigned, NT, ITEMS>(S.work, n, S.sc, [&](unsigned key, int sum, int q) {
+  return block_unique_emit<unsigned, NT, ITEMS>(S.work, n, S.sc.tab, S.sc.scan, [&](unsigned key, int sum, int q) {
     dst[q] = make_int2((int)key, sum);
   });
 }
 
-// Rows of one size class: one block per row writes the row's unique entries
-// to stage[eoff[c] ...) and their number to ucount[c].
-// Resident blocks per SM asked of the compiler for a class shape (0: no
-// bound).  Left to itself the compiler gives these shapes 71-117 registers,
-// so that registers, not shared memory, cap their blocks per SM; the bounds
-// bring them to 56-72 registers without spills (nvcc 13.0, sm_103a), e.g.
-// <256,16> from 2 to 3 blocks and <64,16> from 10 to 14.  <512,16> at 2
-// blocks (64 registers, 28 bytes spilled) still gains a little; <64,12> and
-// <256,12> spill under any bound that would add a block and gain nothing.
-#ifndef CM_MB_32_12
-#define CM_MB_32_12 32
-#endif
-#ifndef CM_MB_32_16
-#define CM_MB_32_16 22
-#endif
-#ifndef CM_MB_64_16
-#define CM_MB_64_16 13
-#endif
-#ifndef CM_MB_128_12
-#define CM_MB_128_12 9
-#endif
-#ifndef CM_MB_128_16
-#define CM_MB_128_16 6
-#endif
-#ifndef CM_MB_256_16
-#define CM_MB_256_16 3
-#endif
-#ifndef CM_MB_64_12
-#define CM_MB_64_12 0
-#endif
-#ifndef CM_MB_256_12
-#define CM_MB_256_12 0
-#endif
-#ifndef CM_MB_512_16
-#define CM_MB_512_16 2
-#endif
+// Rows of one of the largest size classes, radix sorted: one block per row
+// writes the row's unique entries to stage[eoff[c] ...) and their number to
+// ucount[c].
 template <int NT, int ITEMS>
-constexpr int class_min_blocks() {
-  return (NT == 32 && ITEMS == 12)    ? CM_MB_32_12
-         : (NT == 32 && ITEMS == 16)  ? CM_MB_32_16
-         : (NT == 64 && ITEMS == 12)  ? CM_MB_64_12
-         : (NT == 64 && ITEMS == 16)  ? CM_MB_64_16
-         : (NT == 128 && ITEMS == 12) ? CM_MB_128_12
-         : (NT == 128 && ITEMS == 16) ? CM_MB_128_16
-         : (NT == 256 && ITEMS == 12) ? CM_MB_256_12
-         : (NT == 256 && ITEMS == 16) ? CM_MB_256_16
-         : (NT == 512 && ITEMS == 16) ? CM_MB_512_16
-                                      : 0;
-}
-template <int NT, int ITEMS>
-__global__ void __launch_bounds__(NT, class_min_blocks<NT, ITEMS>())
-k_class_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
+__global__ void __launch_bounds__(NT)
+k_radix_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
              const int *__restrict__ eoff, const int4 *__restrict__ row_meta, const int *__restrict__ list,
              const int *__restrict__ count, const int *d_cn, int2 *__restrict__ stage, int *__restrict__ ucount) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -230,6 +186,184 @@ k_class_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
     const int4 md = row_meta[c];
     const int U = segment_sorted_unique<NT, ITEMS>(S, c, md, 0, min(md.w, NT * ITEMS), idbits, adjncy, adjwgt, cmap,
                                                    stage + eoff[c]);
+    if (threadIdx.x == 0) ucount[c] = U;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Class rows: bucket sort
+// ---------------------------------------------------------------------------
+template <int NT, int ITEMS>
+struct RowSmem {
+  SortPair<unsigned> work[NT * ITEMS];
+  __align__(16) int start[NT * ITEMS + 4];  // entries per bucket, then the buckets' first places
+  int tab[NT], scan[NT / 32 + 1];
+  unsigned lo, hi;                          // range of the row's places
+  int load;                                 // sum over the entries of their bucket's size
+};
+// A row whose entries share their buckets with more than this many on average
+// is sorted by comparator passes instead (measured: see class_rows below).
+constexpr int kCrowded = 48;
+
+// Ascending sort of work[0..n) by id: Batcher's bitonic network in its form
+// with one comparator direction, in which places past n are never touched.
+template <int NT>
+__device__ __noinline__ void bitonic_sort(SortPair<unsigned> *work, int n) {
+  for (int k = 2; (k >> 1) < n; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      const int flip = j == (k >> 1) ? k - 1 : j;
+      for (int t = threadIdx.x; t < (n + j + 1) >> 1; t += NT) {
+        const int i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), p = i ^ flip;
+        if (p < n && work[i].k > work[p].k) {
+          const SortPair<unsigned> x = work[i];
+          work[i] = work[p];
+          work[p] = x;
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Writes the unique entries (coarse id, summed weight) of coarse row c's
+// expanded row (metadata md, md.w <= NT * ITEMS), ascending by id, self loops
+// dropped, to dst[0..U).  Returns U.  All NT threads call it; it ends with a
+// block barrier.
+//
+// Bucket sort: entry x's bucket is its place between the row's lowest and
+// highest, where places are the expanded offsets eoff[x].  Offsets grow with
+// the ids' degrees, and an edge leads to a vertex about in proportion to its
+// degree, so the buckets fill evenly also where most entries have low ids
+// (R-MAT: the top ten id bits are all zero for 6% of the entries).  As many
+// buckets as places: the entries of a bucket, one or two, find their order by
+// comparing with one another.
+template <int NT, int ITEMS>
+__device__ __forceinline__ int row_sorted_unique(RowSmem<NT, ITEMS> &S, int c, const int4 &md,
+                                                 const int *__restrict__ adjncy, const int *__restrict__ adjwgt,
+                                                 const int *__restrict__ cmap, const int *__restrict__ eoff,
+                                                 int2 *__restrict__ dst) {
+  constexpr int kCap = NT * ITEMS;
+  const int cnt = min(md.w, kCap);
+  const int tid = threadIdx.x, lane = tid & 31;
+  int x[ITEMS], w[ITEMS], at[ITEMS];  // at: -1 none or a self loop, then place, then bucket | rank << 16
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u) {
+    const int t = u * NT + tid;
+    at[u] = -1;
+    if (t < cnt) {
+      const int src = expanded_src(t, md.x, md.y, md.z);
+      x[u] = __ldcs(adjncy + src);
+      w[u] = __ldcs(adjwgt + src);
+      at[u] = 0;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u) S.start[u * NT + tid] = 0;
+  if (tid == 0) {
+    S.lo = 0xffffffffu;
+    S.hi = 0u;
+    S.load = 0;
+  }
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u)
+    if (at[u] == 0) {
+      x[u] = cmap[x[u]];
+      if (x[u] == c) at[u] = -1;
+    }
+  unsigned lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u)
+    if (at[u] == 0) {
+      at[u] = eoff[x[u]];
+      lo = min(lo, (unsigned)at[u]);
+      hi = max(hi, (unsigned)at[u]);
+    }
+  __syncthreads();
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0 && lo <= hi) {
+    atomicMin(&S.lo, lo);
+    atomicMax(&S.hi, hi);
+  }
+  __syncthreads();
+  if (S.lo > S.hi) {  // only self loops
+    __syncthreads();
+    return 0;
+  }
+  const uint2 map = make_uint2(S.lo, bucket_scale(kCap, S.hi - S.lo));
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u)
+    if (at[u] >= 0) {
+      const int b = min(bucket_of((unsigned)at[u], map), kCap - 1);
+      at[u] = b | atomicAdd(&S.start[b], 1) << 16;
+    }
+  __syncthreads();
+  int n;
+  {
+    int v[ITEMS], sum = 0;
+#pragma unroll
+    for (int u = 0; u < ITEMS; ++u) {
+      v[u] = S.start[tid * ITEMS + u];
+      sum += v[u];
+    }
+    int run = block_exclusive_scan<NT>(sum, S.scan, &n);
+#pragma unroll
+    for (int u = 0; u < ITEMS; ++u) {
+      S.start[tid * ITEMS + u] = run;
+      run += v[u];
+    }
+    if (tid == 0) S.start[kCap] = n;
+  }
+  __syncthreads();
+  int load = 0;
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u)
+    if (at[u] >= 0) {
+      const int b = at[u] & 0xffff;
+      load += S.start[b + 1] - S.start[b];
+      S.work[S.start[b] + (at[u] >> 16)] = make_pair_kv<unsigned>((unsigned)x[u], w[u]);
+    }
+  load = __reduce_add_sync(0xffffffffu, load);
+  if (lane == 0) atomicAdd(&S.load, load);
+  __syncthreads();
+  if (S.load <= kCrowded * n) {
+    unsigned crowded = 0;
+#pragma unroll
+    for (int u = 0; u < ITEMS; ++u)
+      if (at[u] >= 0) {
+        const int b = at[u] & 0xffff, s0 = S.start[b], s1 = S.start[b + 1];
+        if (s1 - s0 > 1) {
+          at[u] = bucket_place(S.work, s0, s1, s0 + (at[u] >> 16), (unsigned)x[u]);
+          crowded |= 1u << u;
+        }
+      }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < ITEMS; ++u)
+      if (crowded >> u & 1u) S.work[at[u]] = make_pair_kv<unsigned>((unsigned)x[u], w[u]);
+    __syncthreads();
+  } else {
+    bitonic_sort<NT>(S.work, n);
+  }
+  return block_unique_emit<unsigned, NT, ITEMS>(S.work, n, S.tab, S.scan, [&](unsigned key, int sum, int q) {
+    dst[q] = make_int2((int)key, sum);
+  });
+}
+
+// Rows of one size class: one block per row writes the row's unique entries
+// to stage[eoff[c] ...) and their number to ucount[c].
+template <int NT, int ITEMS>
+__global__ void __launch_bounds__(NT)
+k_class_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
+             const int *__restrict__ eoff, const int4 *__restrict__ row_meta, const int *__restrict__ list,
+             const int *__restrict__ count, int2 *__restrict__ stage, int *__restrict__ ucount) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RowSmem<NT, ITEMS> &S = *reinterpret_cast<RowSmem<NT, ITEMS> *>(smem_raw);
+  const int nrows = *count;
+  for (int i = blockIdx.x; i < nrows; i += gridDim.x) {
+    const int c = list[i];
+    const int4 md = row_meta[c];
+    const int U = row_sorted_unique<NT, ITEMS>(S, c, md, adjncy, adjwgt, cmap, eoff, stage + eoff[c]);
     if (threadIdx.x == 0) ucount[c] = U;
   }
 }
@@ -1032,9 +1166,16 @@ int64_t class_list_size(int64_t m) { return class_offset(m, kTinyMax, kRowClasse
 template <int K>
 void class_attrs(cm_ctx *ctx) {
   constexpr int NT = class_threads(K), IT = class_items(K);
-  cudaFuncSetAttribute(k_class_rows<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SegSmem<NT, IT>));
   int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_class_rows<NT, IT>, NT, sizeof(SegSmem<NT, IT>));
+  if constexpr (class_radix(K)) {
+    constexpr int bytes = (int)sizeof(SegSmem<NT, IT>);
+    cudaFuncSetAttribute(k_radix_rows<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_radix_rows<NT, IT>, NT, bytes);
+  } else {
+    constexpr int bytes = (int)sizeof(RowSmem<NT, IT>);
+    cudaFuncSetAttribute(k_class_rows<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_class_rows<NT, IT>, NT, bytes);
+  }
   ctx->class_blocks_per_sm[K] = std::max(1, b);
   if constexpr (K + 1 < kClasses) class_attrs<K + 1>(ctx);
 }
@@ -1049,9 +1190,14 @@ void launch_classes(cm_ctx *ctx, const cm_graph *fine, const int *cmap, const in
   const int64_t m = fine->nedges;
   if (row_bound > class_lo(kTinyMax, K)) {
     const unsigned grid = grid_for((int64_t)ctx->num_sms * ctx->class_blocks_per_sm[K], class_cap(m, kTinyMax, K));
-    k_class_rows<NT, IT><<<grid, NT, sizeof(SegSmem<NT, IT>), ctx->aux[K % cm_ctx::kAux]>>>(
-        fine->adjncy, fine->adjwgt, cmap, eoff, row_meta, class_list + class_offset(m, kTinyMax, K), class_ctr + K,
-        d_sizes, stage, ucount);
+    const int *list = class_list + class_offset(m, kTinyMax, K);
+    cudaStream_t s = ctx->aux[K % cm_ctx::kAux];
+    if constexpr (class_radix(K))
+      k_radix_rows<NT, IT><<<grid, NT, sizeof(SegSmem<NT, IT>), s>>>(fine->adjncy, fine->adjwgt, cmap, eoff, row_meta,
+                                                                     list, class_ctr + K, d_sizes, stage, ucount);
+    else
+      k_class_rows<NT, IT><<<grid, NT, sizeof(RowSmem<NT, IT>), s>>>(fine->adjncy, fine->adjwgt, cmap, eoff, row_meta,
+                                                                     list, class_ctr + K, stage, ucount);
     ctx->launches++;
   }
   if constexpr (K + 1 < kClasses)

@@ -239,10 +239,11 @@ __device__ __forceinline__ int bucket_place(const SortPair<unsigned> *work, int 
 
 // Visits the runs of equal keys of the sorted pairs s[0..n): for each run,
 // emit(key, sum of the run's values (wrapping like int atomicAdd), q) with q
-// the run's index in key order.  Returns the number of runs.  n <= NT * 32.
+// the run's index in key order.  Returns the number of runs.  n <= NT * 32;
+// scratch: tab of NT ints, scan of NT / 32 + 1.
 // All NT threads call it; it ends with a block barrier.
 template <typename K, int NT, int ITEMS, typename F>
-__device__ __forceinline__ int block_unique_emit(const SortPair<K> *s, int n, SortScratch<NT> &S, F emit) {
+__device__ __forceinline__ int block_unique_emit(const SortPair<K> *s, int n, int *tab, int *scan, F emit) {
   constexpr int NW = NT / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rounds = (n + NT - 1) / NT;  // <= ITEMS
@@ -255,14 +256,14 @@ __device__ __forceinline__ int block_unique_emit(const SortPair<K> *s, int n, So
       const int i = r * NT + threadIdx.x;
       const bool head = i < n && (i == 0 || s[i].k != s[i - 1].k);
       hm[r] = __ballot_sync(0xffffffffu, head);
-      if (lane == 0) S.tab[r * NW + warp] = __popc(hm[r]);
+      if (lane == 0) tab[r * NW + warp] = __popc(hm[r]);
     }
   }
   __syncthreads();
   const int ncell = rounds * NW;  // <= NT
   int total;
-  const int ex = block_exclusive_scan<NT>(threadIdx.x < ncell ? S.tab[threadIdx.x] : 0, S.scan, &total);
-  if (threadIdx.x < ncell) S.tab[threadIdx.x] = ex;
+  const int ex = block_exclusive_scan<NT>(threadIdx.x < ncell ? tab[threadIdx.x] : 0, scan, &total);
+  if (threadIdx.x < ncell) tab[threadIdx.x] = ex;
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < ITEMS; ++r) {
@@ -271,7 +272,7 @@ __device__ __forceinline__ int block_unique_emit(const SortPair<K> *s, int n, So
       const K key = s[i].k;
       unsigned sum = (unsigned)s[i].v;
       for (int j = i + 1; j < n && s[j].k == key; ++j) sum += (unsigned)s[j].v;
-      emit(key, (int)sum, S.tab[r * NW + warp] + __popc(hm[r] & below));
+      emit(key, (int)sum, tab[r * NW + warp] + __popc(hm[r] & below));
     }
   }
   __syncthreads();

@@ -27,7 +27,8 @@ k_cmap(int n, const int *__restrict__ xadj, const int *__restrict__ vwgt, const 
        int *__restrict__ cmap, int *__restrict__ leader, int *__restrict__ cvwgt, int *__restrict__ eoff,
        int *__restrict__ d_cnvtxs, int *__restrict__ long_list, int long_thr, unsigned long long *long_ctr,
        int long_chunk, int *__restrict__ chunk_row, int *__restrict__ class_list, int *__restrict__ class_ctr,
-       long long m_fine, int4 *__restrict__ row_meta, unsigned long long *__restrict__ lb, DevStatus *st) {
+       long long m_fine, int4 *__restrict__ row_meta, int2 *__restrict__ cplace, unsigned long long *__restrict__ lb,
+       DevStatus *st) {
   __shared__ int s_tile;
   __shared__ unsigned long long s_warp[kCmapThreads / 32];
   __shared__ unsigned long long s_excl;
@@ -87,6 +88,7 @@ k_cmap(int n, const int *__restrict__ xadj, const int *__restrict__ vwgt, const 
         const int xu = u != v ? xadj[u] : 0;
         const int L = dv + (u != v ? xadj[u + 1] - xu : 0);
         cmap[v] = c;
+        if (cplace) cplace[v] = make_int2(c, e);
         leader[c] = (int)v;
         // contraction row metadata: leader's row start and length, follower's row start
         if (row_meta) row_meta[c] = make_int4(xv, dv, xu, L);
@@ -137,12 +139,16 @@ k_cmap(int n, const int *__restrict__ xadj, const int *__restrict__ vwgt, const 
 }
 
 // Followers take their leader's id; also checks that match is an involution.
-__global__ void k_cmap_followers(int n, const int *__restrict__ match, int *__restrict__ cmap, DevStatus *st) {
+__global__ void k_cmap_followers(int n, const int *__restrict__ match, int *__restrict__ cmap,
+                                 int2 *__restrict__ cplace, DevStatus *st) {
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
     int u = match[v];
     if (u < 0 || u >= n) continue;  // already reported by k_cmap
     if (u != v && match[u] != v) record_error(st, CM_ERR_INVALID, ERR_SITE_MATCH_INVALID);
-    if (u < v) cmap[v] = cmap[u];
+    if (u < v) {
+      cmap[v] = cmap[u];
+      if (cplace) cplace[v] = cplace[u];
+    }
   }
 }
 
@@ -153,7 +159,7 @@ size_t cmap_ws_bytes(int64_t n) { return (size_t)((n + kCmapTile - 1) / kCmapTil
 int launch_cmap(cm_ctx *ctx, int32_t n, const int32_t *xadj, const int32_t *vwgt, const int32_t *match,
                 int32_t *cmap, int32_t *leader, int32_t *cvwgt, int32_t *eoff, int32_t *d_cnvtxs,
                 int32_t *long_list, int32_t long_threshold, int32_t long_chunk, unsigned long long *d_long_ctr,
-                int32_t *chunk_row, int32_t *class_list, int32_t *class_ctr, int64_t m, void *row_meta,
+                int32_t *chunk_row, int32_t *class_list, int32_t *class_ctr, int64_t m, void *row_meta, void *cplace,
                 cudaStream_t s) {
   if (n == 0) {
     cudaMemsetAsync(d_cnvtxs, 0, sizeof(int32_t), s);
@@ -168,10 +174,10 @@ int launch_cmap(cm_ctx *ctx, int32_t n, const int32_t *xadj, const int32_t *vwgt
   k_cmap<<<ntiles, kCmapThreads, 0, s>>>(n, xadj, vwgt, match, cmap, leader, cvwgt, eoff, d_cnvtxs, long_list,
                                           long_list ? long_threshold : INT32_MAX, d_long_ctr,
                                           long_chunk > 0 ? long_chunk : 1, chunk_row, class_list, class_ctr,
-                                          (long long)m, (int4 *)row_meta, lb, ctx->d_status);
+                                          (long long)m, (int4 *)row_meta, (int2 *)cplace, lb, ctx->d_status);
   ctx->launches++;
   int blocks = ctx->num_sms * 8;
-  k_cmap_followers<<<blocks, 256, 0, s>>>(n, match, cmap, ctx->d_status);
+  k_cmap_followers<<<blocks, 256, 0, s>>>(n, match, cmap, (int2 *)cplace, ctx->d_status);
   stage_end(ctx, CM_STAGE_CMAP, s);
   ctx->launches++;
   return check_launch(ctx, "cmap");
@@ -265,9 +271,9 @@ extern "C" int cm_build_cmap_noalloc(int32_t nvtxs, const int32_t *d_xadj, const
   // ticket and this call's tile words.
   cudaMemsetAsync(D.scratch, 0, (size_t)(kNoAllocStatusWords + ntiles + 1) * 8, s);
   k_cmap<<<ntiles, kCmapThreads, 0, s>>>(nvtxs, d_xadj, d_vwgt, d_match, d_cmap, d_leader, d_cvwgt, d_eoff, d_cnvtxs,
-                                          nullptr, INT32_MAX, nullptr, 1, nullptr, nullptr, nullptr, 0, nullptr, lb,
-                                          st);
-  k_cmap_followers<<<D.num_sms * 8, 256, 0, s>>>(nvtxs, d_match, d_cmap, st);
+                                          nullptr, INT32_MAX, nullptr, 1, nullptr, nullptr, nullptr, 0, nullptr, nullptr,
+                                          lb, st);
+  k_cmap_followers<<<D.num_sms * 8, 256, 0, s>>>(nvtxs, d_match, d_cmap, nullptr, st);
   k_noalloc_report<<<1, 1, 0, s>>>(st, d_cnvtxs);
   return cuda_status(cudaGetLastError(), "cm_build_cmap_noalloc launch");
 }

@@ -21,8 +21,7 @@
 //   kTinyMax < L <= kChunk : one block per row, sized to the row's class
 //                       (two classes per octave, capacities 1.5 and 2 times
 //                       a power of two, from 96 to kChunk entries; one warp
-//                       up to 512 entries): a shared-memory LSD radix sort of
-//                       the coarse ids (cm_sort.cuh).
+//                       up to 256 entries): a bucket sort in shared memory.
 //   L > kChunk        : huge rows.  Chunks of kChunk entries are sorted,
 //                       merged pairwise (merge path, one launch per pass) and
 //                       deduplicated.
@@ -75,8 +74,7 @@ static_assert(kChunkItems >= 1 && kChunkItems <= 16 && kChunkItems * kChunkThrea
 // holds the rows of kTinyMax 2^j < L <= 1.5 kTinyMax 2^j entries, class 2j+1
 // those up to kTinyMax 2^(j+1).  A class's block has max(32, cap / items)
 // threads, items = kClassItems for the power-of-two capacities and 3/4 of it
-// for the others; the classes that would need more than 1024 threads are
-// radix sorted by 1024 threads of 12 or 16 items.
+// for the others; the largest classes have 1024 threads of 12 or 16 items.
 #ifndef CM_CLASS_ITEMS
 #define CM_CLASS_ITEMS 8
 #endif
@@ -88,9 +86,9 @@ constexpr int class_cap_entries(int k) {
   return (k & 1) ? (kTinyMax << ((k >> 1) + 1)) : (3 * (kTinyMax << (k >> 1))) / 2;
 }
 constexpr int class_item_target(int k) { return (k & 1) ? kClassItems : (3 * kClassItems) / 4; }
-constexpr bool class_radix(int k) { return class_cap_entries(k) / class_item_target(k) > 1024; }
 constexpr int class_threads(int k) {
-  return class_radix(k) ? 1024 : class_cap_entries(k) / class_item_target(k) < 32 ? 32 : class_cap_entries(k) / class_item_target(k);
+  const int t = class_cap_entries(k) / class_item_target(k);
+  return t < 32 ? 32 : t > 1024 ? 1024 : t;
 }
 // Rows above kCopySplit expanded entries are copied one warp per row, the
 // others 32 rows per warp.
@@ -107,102 +105,21 @@ constexpr int kCopyBatch = 4;  // stage loads in flight per thread before their 
 // (as find_cnvtxsedge_original places them, cuMetis.cu:1014-1020).
 __device__ __forceinline__ int expanded_src(int o, int xl, int dl, int xf) { return o < dl ? xl + o : xf + (o - dl); }
 
-// Bits of a coarse id (ids < nc).
-__device__ __forceinline__ int id_bits(int nc) { return nc > 1 ? 32 - __clz(nc - 1) : 0; }
-
-// Appends (key, w) for the lanes with keep set to a padded sort buffer at a
-// shared counter (warp-aggregated; the order within the buffer is arbitrary).
-template <typename K>
-__device__ __forceinline__ void append_pair(SortPair<K> *buf, int *ctr, bool keep, K key, int w) {
-  const int lane = threadIdx.x & 31;
-  const unsigned m = __ballot_sync(0xffffffffu, keep);
-  int base = 0;
-  if (lane == 0 && m) base = atomicAdd(ctr, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (keep) buf[rslot(base + __popc(m & lanemask_lt()))] = make_pair_kv<K>(key, w);
-}
-
 // ---------------------------------------------------------------------------
-// One block sorts a segment of one row (class rows and chunks)
-// ---------------------------------------------------------------------------
-template <int NT, int ITEMS>
-struct SegSmem {
-  SortPair<unsigned> work[rslots(NT * ITEMS)];
-  SortScratch<NT> sc;
-  int ctr;
-};
-
-// Writes the unique entries (coarse id, summed weight) of entries
-// [cs, cs + cnt) of coarse row c's expanded row (metadata md), ascending by
-// id, self loops dropped, to dst[0..U).  Returns U.  cnt <= NT * ITEMS; all
-// NT threads call it; it ends with a block barrier.
-template <int NT, int ITEMS>
-__device__ __forceinline__ int segment_sorted_unique(SegSmem<NT, ITEMS> &S, int c, const int4 &md, int cs, int cnt,
-                                                     int idbits, const int *__restrict__ adjncy,
-                                                     const int *__restrict__ adjwgt, const int *__restrict__ cmap,
-                                                     int2 *__restrict__ dst) {
-  constexpr int kBatch = ITEMS < 4 ? ITEMS : 4;
-  if (threadIdx.x == 0) S.ctr = 0;
-  __syncthreads();
-  for (int b = 0; b < cnt; b += kBatch * NT) {
-    int src[kBatch], x[kBatch], w[kBatch];
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int t = b + u * NT + (int)threadIdx.x;
-      src[u] = t < cnt ? expanded_src(cs + t, md.x, md.y, md.z) : -1;
-    }
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      x[u] = src[u] >= 0 ? __ldcs(adjncy + src[u]) : 0;
-      w[u] = src[u] >= 0 ? __ldcs(adjwgt + src[u]) : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) x[u] = src[u] >= 0 ? cmap[x[u]] : c;
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) append_pair<unsigned>(S.work, &S.ctr, x[u] != c, (unsigned)x[u], w[u]);
-  }
-  __syncthreads();
-  const int n = S.ctr;
-  block_radix_sort<unsigned, NT, ITEMS>(S.work, S.sc, n, idbits);
-  return block_unique_emit<unsigned, NT, ITEMS>(S.work, n, S.sc.tab, S.sc.scan, [&](unsigned key, int sum, int q) {
-    dst[q] = make_int2((int)key, sum);
-  });
-}
-
-// Rows of one of the largest size classes, radix sorted: one block per row
-// writes the row's unique entries to stage[eoff[c] ...) and their number to
-// ucount[c].
-template <int NT, int ITEMS>
-__global__ void __launch_bounds__(NT)
-k_radix_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
-             const int *__restrict__ eoff, const int4 *__restrict__ row_meta, const int *__restrict__ list,
-             const int *__restrict__ count, const int *d_cn, int2 *__restrict__ stage, int *__restrict__ ucount) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SegSmem<NT, ITEMS> &S = *reinterpret_cast<SegSmem<NT, ITEMS> *>(smem_raw);
-  const int nrows = *count;
-  const int idbits = id_bits(*d_cn);
-  for (int i = blockIdx.x; i < nrows; i += gridDim.x) {
-    const int c = list[i];
-    const int4 md = row_meta[c];
-    const int U = segment_sorted_unique<NT, ITEMS>(S, c, md, 0, min(md.w, NT * ITEMS), idbits, adjncy, adjwgt, cmap,
-                                                   stage + eoff[c]);
-    if (threadIdx.x == 0) ucount[c] = U;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Class rows: bucket sort
+// One block sorts a segment of one row (class rows and chunks): bucket sort
 // ---------------------------------------------------------------------------
 template <int NT, int ITEMS>
 struct RowSmem {
   SortPair<unsigned> work[NT * ITEMS];
-  __align__(16) int start[NT * ITEMS + 4];  // entries per bucket, then the buckets' first places
+  int start[rslots(NT * ITEMS + 1)];        // at rslot(b): entries of bucket b, then its first place
   int tab[NT], scan[NT / 32 + 1];
   unsigned lo, hi;                          // range of the row's places
   int load;                                 // sum over the entries of their bucket's size
 };
 // A row whose entries share their buckets with more than this many on average
-// is sorted by comparator passes instead (measured: see class_rows below).
+// is sorted by comparator passes instead: a comparison within a bucket costs
+// about 5 instructions, a comparator pass of a row of L entries about 10 in each
+// of log2(L) (log2(L) + 1) / 2 steps, 360 to 1050 for L from 200 to 16384.
 constexpr int kCrowded = 48;
 
 // Ascending sort of work[0..n) by id: Batcher's bitonic network in its form
@@ -225,25 +142,30 @@ __device__ __noinline__ void bitonic_sort(SortPair<unsigned> *work, int n) {
   }
 }
 
-// Writes the unique entries (coarse id, summed weight) of coarse row c's
-// expanded row (metadata md, md.w <= NT * ITEMS), ascending by id, self loops
-// dropped, to dst[0..U).  Returns U.  All NT threads call it; it ends with a
-// block barrier.
+// Writes the unique entries (coarse id, summed weight) of entries
+// [cs, cs + cnt) of coarse row c's expanded row (metadata md), ascending by
+// id, self loops dropped, to dst[0..U).  Returns U.  cnt <= NT * ITEMS; all
+// NT threads call it; it ends with a block barrier.
 //
 // Bucket sort: entry x's bucket is its place between the row's lowest and
-// highest, where places are the expanded offsets eoff[x].  Offsets grow with
+// highest, where places are the expanded offsets (cplace: a fine vertex's
+// coarse id and offset in one 8-byte gather).  Offsets grow with
 // the ids' degrees, and an edge leads to a vertex about in proportion to its
 // degree, so the buckets fill evenly also where most entries have low ids
 // (R-MAT: the top ten id bits are all zero for 6% of the entries).  As many
 // buckets as places: the entries of a bucket, one or two, find their order by
-// comparing with one another.
+// comparing with one another.  One pass over the entries replaces the radix
+// sort's pass per 4 id bits: the row kernels of an R-MAT 22 level take 2.09 ms
+// of overlapped time against 2.92 ms (8193-12288 entries 367 -> 213 us, 257-384
+// 195 -> 115 us).  Bound by issue (46% busy) and by the L1 / shared-memory pipe
+// (72%): every gather of cplace takes a wavefront per entry.
 template <int NT, int ITEMS>
-__device__ __forceinline__ int row_sorted_unique(RowSmem<NT, ITEMS> &S, int c, const int4 &md,
-                                                 const int *__restrict__ adjncy, const int *__restrict__ adjwgt,
-                                                 const int *__restrict__ cmap, const int *__restrict__ eoff,
+__device__ __forceinline__ int row_sorted_unique(RowSmem<NT, ITEMS> &S, int c, const int4 &md, int cs,
+                                                 int cnt, const int *__restrict__ adjncy,
+                                                 const int *__restrict__ adjwgt, const int2 *__restrict__ cplace,
                                                  int2 *__restrict__ dst) {
   constexpr int kCap = NT * ITEMS;
-  const int cnt = min(md.w, kCap);
+  static_assert(kCap <= 1 << 14, "places are packed in 14 bits");
   const int tid = threadIdx.x, lane = tid & 31;
   int x[ITEMS], w[ITEMS], at[ITEMS];  // at: -1 none or a self loop, then place, then bucket | rank << 16
 #pragma unroll
@@ -251,33 +173,35 @@ __device__ __forceinline__ int row_sorted_unique(RowSmem<NT, ITEMS> &S, int c, c
     const int t = u * NT + tid;
     at[u] = -1;
     if (t < cnt) {
-      const int src = expanded_src(t, md.x, md.y, md.z);
+      const int src = expanded_src(cs + t, md.x, md.y, md.z);
       x[u] = __ldcs(adjncy + src);
       w[u] = __ldcs(adjwgt + src);
       at[u] = 0;
     }
   }
 #pragma unroll
-  for (int u = 0; u < ITEMS; ++u) S.start[u * NT + tid] = 0;
+  for (int u = 0; u < ITEMS; ++u) S.start[rslot(u * NT + tid)] = 0;
   if (tid == 0) {
     S.lo = 0xffffffffu;
     S.hi = 0u;
     S.load = 0;
   }
-#pragma unroll
-  for (int u = 0; u < ITEMS; ++u)
-    if (at[u] == 0) {
-      x[u] = cmap[x[u]];
-      if (x[u] == c) at[u] = -1;
-    }
   unsigned lo = 0xffffffffu, hi = 0u;
 #pragma unroll
   for (int u = 0; u < ITEMS; ++u)
     if (at[u] == 0) {
-      at[u] = eoff[x[u]];
+      const int2 y = cplace[x[u]];
+      x[u] = y.x;
+      at[u] = y.y;
+    }
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u) {
+    if (at[u] >= 0 && x[u] == c) at[u] = -1;
+    if (at[u] >= 0) {
       lo = min(lo, (unsigned)at[u]);
       hi = max(hi, (unsigned)at[u]);
     }
+  }
   __syncthreads();
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
@@ -295,52 +219,48 @@ __device__ __forceinline__ int row_sorted_unique(RowSmem<NT, ITEMS> &S, int c, c
   for (int u = 0; u < ITEMS; ++u)
     if (at[u] >= 0) {
       const int b = min(bucket_of((unsigned)at[u], map), kCap - 1);
-      at[u] = b | atomicAdd(&S.start[b], 1) << 16;
+      at[u] = b | atomicAdd(&S.start[rslot(b)], 1) << 16;
     }
   __syncthreads();
   int n;
   {
-    int v[ITEMS], sum = 0;
+    int sum = 0;
 #pragma unroll
-    for (int u = 0; u < ITEMS; ++u) {
-      v[u] = S.start[tid * ITEMS + u];
-      sum += v[u];
-    }
+    for (int u = 0; u < ITEMS; ++u) sum += S.start[rslot(tid * ITEMS + u)];
     int run = block_exclusive_scan<NT>(sum, S.scan, &n);
 #pragma unroll
     for (int u = 0; u < ITEMS; ++u) {
-      S.start[tid * ITEMS + u] = run;
-      run += v[u];
+      const int v = S.start[rslot(tid * ITEMS + u)];
+      S.start[rslot(tid * ITEMS + u)] = run;
+      run += v;
     }
-    if (tid == 0) S.start[kCap] = n;
+    if (tid == 0) S.start[rslot(kCap)] = n;
   }
   __syncthreads();
+  // at: -1 if alone in its bucket, else the bucket's first place | rank << 14 | (size - 1) << 22
   int load = 0;
 #pragma unroll
   for (int u = 0; u < ITEMS; ++u)
     if (at[u] >= 0) {
-      const int b = at[u] & 0xffff;
-      load += S.start[b + 1] - S.start[b];
-      S.work[S.start[b] + (at[u] >> 16)] = make_pair_kv<unsigned>((unsigned)x[u], w[u]);
+      const int b = at[u] & 0xffff, r = at[u] >> 16, s0 = S.start[rslot(b)], size = S.start[rslot(b + 1)] - s0;
+      S.work[s0 + r] = make_pair_kv<unsigned>((unsigned)x[u], w[u]);
+      load += size <= 256 ? size : kCap;  // too many for the packed form: as a crowded row
+      at[u] = size == 1 ? -1 : s0 | (r & 255) << 14 | (size - 1) << 22;
     }
   load = __reduce_add_sync(0xffffffffu, load);
   if (lane == 0) atomicAdd(&S.load, load);
   __syncthreads();
   if (S.load <= kCrowded * n) {
-    unsigned crowded = 0;
 #pragma unroll
     for (int u = 0; u < ITEMS; ++u)
       if (at[u] >= 0) {
-        const int b = at[u] & 0xffff, s0 = S.start[b], s1 = S.start[b + 1];
-        if (s1 - s0 > 1) {
-          at[u] = bucket_place(S.work, s0, s1, s0 + (at[u] >> 16), (unsigned)x[u]);
-          crowded |= 1u << u;
-        }
+        const int s0 = at[u] & 0x3fff;
+        at[u] = bucket_place(S.work, s0, s0 + (at[u] >> 22) + 1, s0 + (at[u] >> 14 & 255), (unsigned)x[u]);
       }
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < ITEMS; ++u)
-      if (crowded >> u & 1u) S.work[at[u]] = make_pair_kv<unsigned>((unsigned)x[u], w[u]);
+      if (at[u] >= 0) S.work[at[u]] = make_pair_kv<unsigned>((unsigned)x[u], w[u]);
     __syncthreads();
   } else {
     bitonic_sort<NT>(S.work, n);
@@ -354,7 +274,7 @@ __device__ __forceinline__ int row_sorted_unique(RowSmem<NT, ITEMS> &S, int c, c
 // to stage[eoff[c] ...) and their number to ucount[c].
 template <int NT, int ITEMS>
 __global__ void __launch_bounds__(NT)
-k_class_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
+k_class_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int2 *__restrict__ cplace,
              const int *__restrict__ eoff, const int4 *__restrict__ row_meta, const int *__restrict__ list,
              const int *__restrict__ count, int2 *__restrict__ stage, int *__restrict__ ucount) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -363,7 +283,8 @@ k_class_rows(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, con
   for (int i = blockIdx.x; i < nrows; i += gridDim.x) {
     const int c = list[i];
     const int4 md = row_meta[c];
-    const int U = row_sorted_unique<NT, ITEMS>(S, c, md, adjncy, adjwgt, cmap, eoff, stage + eoff[c]);
+    const int U = row_sorted_unique<NT, ITEMS>(S, c, md, 0, min(md.w, NT * ITEMS), adjncy, adjwgt, cplace,
+                                               stage + eoff[c]);
     if (threadIdx.x == 0) ucount[c] = U;
   }
 }
@@ -393,14 +314,13 @@ __device__ __forceinline__ int2 unpack_entry(unsigned long long v) {
 // chunk's length, which sort after every coarse id and are skipped by the
 // dedup.  chunk_np[q] = the merge passes the chunk's row needs.
 __global__ void __launch_bounds__(kChunkThreads, 1)
-k_long_sort(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ cmap,
+k_long_sort(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int2 *__restrict__ cplace,
             const int *__restrict__ eoff, const int4 *__restrict__ row_meta, const int *__restrict__ long_list,
-            const int *__restrict__ chunk_row, const unsigned long long *long_ctr, const int *d_cn,
-            int2 *__restrict__ stage, int *__restrict__ ucount, int *__restrict__ chunk_np) {
+            const int *__restrict__ chunk_row, const unsigned long long *long_ctr, int2 *__restrict__ stage,
+            int *__restrict__ ucount, int *__restrict__ chunk_np) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SegSmem<kChunkThreads, kChunkItems> &S = *reinterpret_cast<SegSmem<kChunkThreads, kChunkItems> *>(smem_raw);
+  RowSmem<kChunkThreads, kChunkItems> &S = *reinterpret_cast<RowSmem<kChunkThreads, kChunkItems> *>(smem_raw);
   const int nchunks = (int)(*long_ctr & 0xffffffffu);
-  const int idbits = id_bits(*d_cn);
   for (int q = blockIdx.x; q < nchunks; q += gridDim.x) {
     const int idx = chunk_row[q];
     const int c = long_list[2 * idx];
@@ -411,8 +331,7 @@ k_long_sort(const int *__restrict__ adjncy, const int *__restrict__ adjwgt, cons
     if (j == 0 && threadIdx.x == 0) ucount[c] = 0;  // the dedup adds the chunks' counts
     if (threadIdx.x == 0) chunk_np[q] = merge_passes(md.w);
     int2 *dst = stage + eoff[c] + cs;
-    const int U = segment_sorted_unique<kChunkThreads, kChunkItems>(S, c, md, cs, cnt, idbits, adjncy, adjwgt, cmap,
-                                                                    dst);
+    const int U = row_sorted_unique<kChunkThreads, kChunkItems>(S, c, md, cs, cnt, adjncy, adjwgt, cplace, dst);
     for (int t = U + threadIdx.x; t < cnt; t += kChunkThreads) dst[t] = make_int2((int)kPadId, 0);
   }
 }
@@ -1165,17 +1084,10 @@ int64_t class_list_size(int64_t m) { return class_offset(m, kTinyMax, kRowClasse
 
 template <int K>
 void class_attrs(cm_ctx *ctx) {
-  constexpr int NT = class_threads(K), IT = class_items(K);
+  constexpr int NT = class_threads(K), IT = class_items(K), bytes = (int)sizeof(RowSmem<NT, IT>);
+  cudaFuncSetAttribute(k_class_rows<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   int b = 0;
-  if constexpr (class_radix(K)) {
-    constexpr int bytes = (int)sizeof(SegSmem<NT, IT>);
-    cudaFuncSetAttribute(k_radix_rows<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_radix_rows<NT, IT>, NT, bytes);
-  } else {
-    constexpr int bytes = (int)sizeof(RowSmem<NT, IT>);
-    cudaFuncSetAttribute(k_class_rows<NT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_class_rows<NT, IT>, NT, bytes);
-  }
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_class_rows<NT, IT>, NT, bytes);
   ctx->class_blocks_per_sm[K] = std::max(1, b);
   if constexpr (K + 1 < kClasses) class_attrs<K + 1>(ctx);
 }
@@ -1183,25 +1095,19 @@ void class_attrs(cm_ctx *ctx) {
 // Launches the class kernels of the classes a row of at most row_bound
 // entries can fall in, round-robin on the auxiliary streams.
 template <int K>
-void launch_classes(cm_ctx *ctx, const cm_graph *fine, const int *cmap, const int *eoff, const int4 *row_meta,
-                    const int *class_list, const int *class_ctr, const int *d_sizes, int2 *stage, int *ucount,
-                    int64_t row_bound) {
+void launch_classes(cm_ctx *ctx, const cm_graph *fine, const int2 *cplace, const int *eoff, const int4 *row_meta,
+                    const int *class_list, const int *class_ctr, int2 *stage, int *ucount, int64_t row_bound) {
   constexpr int NT = class_threads(K), IT = class_items(K);
   const int64_t m = fine->nedges;
   if (row_bound > class_lo(kTinyMax, K)) {
     const unsigned grid = grid_for((int64_t)ctx->num_sms * ctx->class_blocks_per_sm[K], class_cap(m, kTinyMax, K));
-    const int *list = class_list + class_offset(m, kTinyMax, K);
-    cudaStream_t s = ctx->aux[K % cm_ctx::kAux];
-    if constexpr (class_radix(K))
-      k_radix_rows<NT, IT><<<grid, NT, sizeof(SegSmem<NT, IT>), s>>>(fine->adjncy, fine->adjwgt, cmap, eoff, row_meta,
-                                                                     list, class_ctr + K, d_sizes, stage, ucount);
-    else
-      k_class_rows<NT, IT><<<grid, NT, sizeof(RowSmem<NT, IT>), s>>>(fine->adjncy, fine->adjwgt, cmap, eoff, row_meta,
-                                                                     list, class_ctr + K, stage, ucount);
+    k_class_rows<NT, IT><<<grid, NT, sizeof(RowSmem<NT, IT>), ctx->aux[K % cm_ctx::kAux]>>>(
+        fine->adjncy, fine->adjwgt, cplace, eoff, row_meta, class_list + class_offset(m, kTinyMax, K), class_ctr + K,
+        stage, ucount);
     ctx->launches++;
   }
   if constexpr (K + 1 < kClasses)
-    launch_classes<K + 1>(ctx, fine, cmap, eoff, row_meta, class_list, class_ctr, d_sizes, stage, ucount, row_bound);
+    launch_classes<K + 1>(ctx, fine, cplace, eoff, row_meta, class_list, class_ctr, stage, ucount, row_bound);
 }
 }  // namespace
 
@@ -1217,7 +1123,7 @@ size_t contract_ws_bytes(int64_t n, int64_t m) {
   b += 256;                                            // counters
   b += (size_t)(n / kMapTile + 3) * 8 + 256;           // unit-map look-back
   b += (size_t)(n / (kScanThreads * kScanItems) + 3) * 8 + 256;  // count-scan look-back
-  b += (size_t)n * 16 + 256;                           // row metadata
+  b += (size_t)n * 24 + 512;                           // row metadata, coarse ids with places
   b += (size_t)m * 8 * 2 + 512;                        // stages
   b += cmap_ws_bytes(n);
   return b + 4096;
@@ -1234,7 +1140,7 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   if (!ctx->contract_attrs_set) {  // once per context (the attributes last for the process)
     cudaFuncSetAttribute(k_tiny_units, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TinySmem));
     cudaFuncSetAttribute(k_long_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(SegSmem<kChunkThreads, kChunkItems>));
+                         (int)sizeof(RowSmem<kChunkThreads, kChunkItems>));
     cudaFuncSetAttribute(k_long_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MergeSmem));
     class_attrs<0>(ctx);
     int b = 0;
@@ -1257,6 +1163,7 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   int *chunk_cnt = (int *)ws_take(ctx, (size_t)nchunks_max * 4);
   int *chunk_np = (int *)ws_take(ctx, (size_t)nchunks_max * 4);
   int4 *row_meta = (int4 *)ws_take(ctx, (size_t)n * 16);
+  int2 *cplace = (int2 *)ws_take(ctx, (size_t)n * 8);
   // [0] chunked rows (rows << 32 | chunks); ints 2 .. 2 + kRowClasses - 1 the
   // class counters; int 2 + kRowClasses the last tiny unit's index
   static_assert(2 + kRowClasses + 1 <= 32, "contraction counter block");
@@ -1266,7 +1173,7 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   int2 *stage0 = (int2 *)ws_take(ctx, (size_t)m * 8 + 8);
   int2 *stage1 = (int2 *)ws_take(ctx, (size_t)m * 8 + 8);
   if (!leader || !ucount || !eoff || !first_row || !long_list || !class_list || !chunk_row || !chunk_cnt ||
-      !chunk_np || !row_meta || !ctr || !map_lb || !scan_lb || !stage0 || !stage1)
+      !chunk_np || !row_meta || !cplace || !ctr || !map_lb || !scan_lb || !stage0 || !stage1)
     return cm_fail(CM_ERR_NOMEM, "contract: workspace too small");
   int *class_ctr = reinterpret_cast<int *>(ctr) + 2;
   int *unit_last = reinterpret_cast<int *>(ctr) + 2 + kRowClasses;
@@ -1277,7 +1184,7 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   cudaMemsetAsync(scan_lb, 0, (size_t)(scan_tiles + 3) * 8, s);
   int rc = launch_cmap(ctx, (int32_t)n, fine->xadj, fine->vwgt, match, cmap, leader, coarse->vwgt, eoff,
                        d_sizes /* n' lands in d_sizes[0] */, long_list, kTinyMax, kChunk, ctr, chunk_row, class_list,
-                       class_ctr, m, row_meta, s);
+                       class_ctr, m, row_meta, row_bound > kTinyMax ? cplace : nullptr, s);
   if (rc) return rc;
   const int sms = ctx->num_sms;
 
@@ -1294,15 +1201,14 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   if (any_big) {
     cudaEventRecord(ctx->fork_ev, s);
     for (int i = 0; i < cm_ctx::kAux; ++i) cudaStreamWaitEvent(ctx->aux[i], ctx->fork_ev, 0);
-    launch_classes<0>(ctx, fine, cmap, eoff, row_meta, class_list, class_ctr, d_sizes, stage1, ucount, row_bound);
+    launch_classes<0>(ctx, fine, cplace, eoff, row_meta, class_list, class_ctr, stage1, ucount, row_bound);
     if (chunked) {
       cudaStream_t cs = ctx->aux[cm_ctx::kAux - 1];
       // Grids of the chunked-row kernels scale with the most chunks the graph
       // can have (m / kChunk), so small graphs do not claim every SM.
       const int long_grid = (int)std::min<int64_t>(sms, m / kChunk / 4 + 1);
-      k_long_sort<<<long_grid, kChunkThreads, sizeof(SegSmem<kChunkThreads, kChunkItems>), cs>>>(
-          fine->adjncy, fine->adjwgt, cmap, eoff, row_meta, long_list, chunk_row, ctr, d_sizes, stage0, ucount,
-          chunk_np);
+      k_long_sort<<<long_grid, kChunkThreads, sizeof(RowSmem<kChunkThreads, kChunkItems>), cs>>>(
+          fine->adjncy, fine->adjwgt, cplace, eoff, row_meta, long_list, chunk_row, ctr, stage0, ucount, chunk_np);
       ctx->launches++;
       // Passes a row of at most min(m, row_bound) entries can need; each is a
       // plain launch.

@@ -121,7 +121,9 @@ namespace {
 
 size_t level_ws_bytes(int64_t n, int64_t m) {
   // matching and contraction run one after the other and share the workspace
-  return std::max(match_ws_bytes(n, m), contract_ws_bytes(n, m) + 1024);
+  size_t b = std::max(match_ws_bytes(n, m), contract_ws_bytes(n, m) + 1024);
+  const int64_t fm = std::min(m, kFusedWork), fn = std::min(n, kFusedWork);  // graphs that cm_levels.cu takes
+  return std::max(b, fused_ws_bytes(fn, fm) + 1024);
 }
 
 bool bad_graph(const cm_graph *g) {
@@ -184,6 +186,7 @@ extern "C" int cm_ctx_create(int device, cm_ctx **out) {
   if (!rc) rc = cuda_status(cudaMemset(ctx->d_status, 0, sizeof(DevStatus)), "status init");
   if (!rc) rc = cuda_status(cudaMallocHost(&ctx->h_status, sizeof(DevStatus)), "pinned status alloc");
   if (!rc) rc = cuda_status(cudaMallocHost(&ctx->h_small, 64), "pinned readback alloc");
+  if (!rc) rc = cuda_status(cudaMallocHost(&ctx->h_levels, cm_ctx::kReadbackBytes), "pinned readback alloc");
   if (!rc) rc = cuda_status(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "context stream");
   for (int i = 0; i < cm_ctx::kAux && !rc; ++i) {
     rc = cuda_status(cudaStreamCreateWithFlags(&ctx->aux[i], cudaStreamNonBlocking), "aux stream");
@@ -224,6 +227,7 @@ extern "C" void cm_ctx_destroy(cm_ctx *ctx) {
   if (ctx->d_status) cudaFree(ctx->d_status);
   if (ctx->h_status) cudaFreeHost(ctx->h_status);
   if (ctx->h_small) cudaFreeHost(ctx->h_small);
+  if (ctx->h_levels) cudaFreeHost(ctx->h_levels);
   if (ctx->d_trace) cudaFree(ctx->d_trace);
   for (int i = 0; i < cm_ctx::kAux; ++i) {
     if (ctx->aux[i]) cudaStreamDestroy(ctx->aux[i]);
@@ -487,9 +491,16 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
   int32_t *sizes = (int32_t *)ws_take(ctx, 64);
   const size_t level_ws_off = ctx->ws_used;
 
-  for (int level = 0;; ++level) {
+  for (;;) {
     cm_level &F = h->levels.back();
     const int64_t n = F.g.nvtxs, m = F.g.nedges;
+    if (fused_fits(ctx, n, m, row_bound / 2, params->match_mode)) {
+      int produced = 0, stopped = 0;
+      ctx->ws_used = level_ws_off;
+      if ((rc = launch_fused(ctx, h, params, s, &produced, &stopped, &row_bound))) return fail(rc);
+      if (stopped) break;
+      if (produced > 0) continue;
+    }
     cm_level C;
     if ((rc = alloc_level(C, n, m, ctx->pool, s))) return fail(rc);
     ctx->ws_used = level_ws_off;

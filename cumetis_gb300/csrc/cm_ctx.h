@@ -17,6 +17,8 @@ struct cm_ctx {
   cm::DevStatus *d_status = nullptr;   // device status block
   cm::DevStatus *h_status = nullptr;   // pinned host mirror for readbacks
   int32_t *h_small = nullptr;          // pinned 64-byte readback buffer
+  static constexpr size_t kReadbackBytes = 8192;
+  void *h_levels = nullptr;            // pinned readback of the levels of one launch (cm_levels.cu)
   char *ws = nullptr;           // device workspace (grown on demand)
   size_t ws_bytes = 0;
   size_t ws_used = 0;           // bump pointer of the current call
@@ -48,7 +50,7 @@ struct cm_ctx {
   cudaEvent_t wait_ev = nullptr;
   // launch set-up done once: the contraction kernels' shared-memory limits,
   // the matching kernel's resident blocks per SM (per tie order)
-  bool contract_attrs_set = false;
+  bool contract_attrs_set = false, levels_attrs_set = false;
   int match_blocks_per_sm[2] = {0, 0};
   // resident blocks per SM of the contraction's tiny-unit kernel and of its
   // row-class kernels
@@ -162,6 +164,23 @@ int launch_cmap(cm_ctx *ctx, int32_t n, const int32_t *xadj, const int32_t *vwgt
 // when unknown); kernels of row classes above it are not launched.
 int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int32_t *cmap, cm_graph *coarse,
                     int32_t *d_sizes, cudaStream_t s, int64_t row_bound);
+
+// Whole levels of a small graph in one kernel (cm_levels.cu).  Graphs of at
+// most kFusedWork vertices + entries take it (coarsening a 725 x 725 grid, whose
+// levels have 2.6 M, 1.6 M, 0.9 M, 0.5 M ... of them: 1350 us with 0.3 M, 1229
+// with 0.6 M, 1198 with 1.2 M, 1191 with 2 M; a 101^3 grid 2571, 2498, 2456, 2445;
+// larger graphs fill the chip in every kernel anyway).  launch_fused coarsens
+// h->levels.back() by the params' rules as far as the kernel can, appends the
+// levels (*produced; *stopped = 1 when the stop rule ended the coarsening) and
+// updates *row_bound; it waits for the stream.
+#ifndef CM_FUSED_WORK
+#define CM_FUSED_WORK 1200000
+#endif
+constexpr int64_t kFusedWork = CM_FUSED_WORK;
+size_t fused_ws_bytes(int64_t n, int64_t m);
+bool fused_fits(const cm_ctx *ctx, int64_t n, int64_t m, int64_t max_deg, int32_t mode);
+int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaStream_t s, int *produced, int *stopped,
+                 int64_t *row_bound);
 
 }  // namespace cm
 

@@ -194,13 +194,25 @@ __device__ __forceinline__ int warp_inclusive_scan_i32(int v) {
   return v;
 }
 
-// Block-wide exclusive scan of one int per thread (NT threads, multiple of
-// 32).  `sh` needs NT/32 + 1 ints.  Returns the exclusive prefix; *total gets
-// the block sum.
+// Barrier of the NT threads that work on something together: the block, or with
+// NT = 32 the calling warp (blocks may hold several).
+template <int NT>
+__device__ __forceinline__ void row_sync() {
+  if (NT == 32) __syncwarp();
+  else __syncthreads();
+}
+
+// Exclusive scan of one int per thread over the block, or with NT = 32 over the
+// calling warp (NT a multiple of 32).  `sh` needs NT/32 + 1 ints.  Returns the
+// exclusive prefix; *total gets the sum.
 template <int NT>
 __device__ __forceinline__ int block_exclusive_scan(int v, int *sh, int *total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = NT == 32 ? 0 : threadIdx.x >> 5;
   int inc = warp_inclusive_scan_i32(v);
+  if (NT == 32) {
+    *total = __shfl_sync(0xffffffffu, inc, 31);
+    return inc - v;
+  }
   if (lane == 31) sh[wid] = inc;
   __syncthreads();
   if (wid == 0) {

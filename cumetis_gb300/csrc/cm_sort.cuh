@@ -80,11 +80,12 @@ __device__ __forceinline__ int bucket_place(const SortPair<unsigned> *work, int 
 // emit(key, sum of the run's values (wrapping like int atomicAdd), q) with q
 // the run's index in key order.  Returns the number of runs.  n <= NT * 32;
 // scratch: tab of NT ints, scan of NT / 32 + 1.
-// All NT threads call it; it ends with a block barrier.
+// All threads of the block call it, or with NT = 32 those of a warp; it ends
+// with their barrier.
 template <typename K, int NT, int ITEMS, typename F>
 __device__ __forceinline__ int block_unique_emit(const SortPair<K> *s, int n, int *tab, int *scan, F emit) {
   constexpr int NW = NT / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = NT == 32 ? threadIdx.x & 31 : threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rounds = (n + NT - 1) / NT;  // <= ITEMS
   const unsigned below = lanemask_lt();
   unsigned hm[ITEMS];
@@ -92,29 +93,29 @@ __device__ __forceinline__ int block_unique_emit(const SortPair<K> *s, int n, in
   for (int r = 0; r < ITEMS; ++r) {
     hm[r] = 0u;
     if (r < rounds) {
-      const int i = r * NT + threadIdx.x;
+      const int i = r * NT + tid;
       const bool head = i < n && (i == 0 || s[i].k != s[i - 1].k);
       hm[r] = __ballot_sync(0xffffffffu, head);
       if (lane == 0) tab[r * NW + warp] = __popc(hm[r]);
     }
   }
-  __syncthreads();
+  row_sync<NT>();
   const int ncell = rounds * NW;  // <= NT
   int total;
-  const int ex = block_exclusive_scan<NT>(threadIdx.x < ncell ? tab[threadIdx.x] : 0, scan, &total);
-  if (threadIdx.x < ncell) tab[threadIdx.x] = ex;
-  __syncthreads();
+  const int ex = block_exclusive_scan<NT>(tid < ncell ? tab[tid] : 0, scan, &total);
+  if (tid < ncell) tab[tid] = ex;
+  row_sync<NT>();
 #pragma unroll
   for (int r = 0; r < ITEMS; ++r) {
     if (r < rounds && (hm[r] >> lane & 1u)) {
-      const int i = r * NT + threadIdx.x;
+      const int i = r * NT + tid;
       const K key = s[i].k;
       unsigned sum = (unsigned)s[i].v;
       for (int j = i + 1; j < n && s[j].k == key; ++j) sum += (unsigned)s[j].v;
       emit(key, (int)sum, tab[r * NW + warp] + __popc(hm[r] & below));
     }
   }
-  __syncthreads();
+  row_sync<NT>();
   return total;
 }
 

@@ -169,6 +169,8 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
   slab->ptr = p;
   slab->device = ctx_->device;
   slab->stream = s_;
+  std::vector<HostArray> in;
+  in.reserve(4 * count);
   for (int i = 0; i < count; ++i) {
     const cm_graph &g = graphs[i];
     const int64_t n = g.nvtxs, m = g.nedges;
@@ -182,10 +184,10 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
     cm_level L;
     carve_level(p, n, m, L);
     p += level_bytes(n, m);
-    cudaMemcpyAsync(L.g.xadj, g.xadj, (n + 1) * 4, cudaMemcpyHostToDevice, s_);
-    if (n) cudaMemcpyAsync(L.g.vwgt, g.vwgt, n * 4, cudaMemcpyHostToDevice, s_);
-    if (m) cudaMemcpyAsync(L.g.adjncy, g.adjncy, m * 4, cudaMemcpyHostToDevice, s_);
-    if (m) cudaMemcpyAsync(L.g.adjwgt, g.adjwgt, m * 4, cudaMemcpyHostToDevice, s_);
+    in.push_back({g.xadj, L.g.xadj, (size_t)(n + 1) * 4});
+    in.push_back({g.vwgt, L.g.vwgt, (size_t)n * 4});
+    in.push_back({g.adjncy, L.g.adjncy, (size_t)m * 4});
+    in.push_back({g.adjwgt, L.g.adjwgt, (size_t)m * 4});
     a.h->levels.push_back(L);
     int64_t tvwgt = 0, maxdeg = 0;
     for (int64_t v = 0; v < n; ++v) {
@@ -212,7 +214,7 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
     }
     active_.push_back(a);
   }
-  return cuda_status(cudaGetLastError(), "batch upload");
+  return upload_arrays(ctx_, in.data(), (int)in.size(), s_);
 }
 
 int BatchCoarsener::step(std::vector<std::pair<int64_t, cm_hierarchy *>> &finished) {

@@ -14,6 +14,7 @@ struct cm_ctx {
   int device = 0;
   int num_sms = 0;
   int max_smem_optin = 0;       // bytes of dynamic shared memory a block may opt into
+  bool reads_host = false;      // kernels may read any host memory (the host's page tables)
   cm::DevStatus *d_status = nullptr;   // device status block
   cm::DevStatus *h_status = nullptr;   // pinned host mirror for readbacks
   int32_t *h_small = nullptr;          // pinned 64-byte readback buffer
@@ -104,6 +105,15 @@ inline void ws_reset(cm_ctx *ctx) { ctx->ws_used = 0; }
 // Stage timing: events recorded on the launch stream around one kernel.
 void stage_begin(cm_ctx *ctx, cudaStream_t s);
 void stage_end(cm_ctx *ctx, int stage, cudaStream_t s);
+
+// Copies arrays from host memory (any: pageable, pinned) to the device on s.  The
+// host arrays must stay valid until the stream has run the copies.
+struct HostArray {
+  const void *src;
+  void *dst;
+  size_t bytes;
+};
+int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s);
 
 // Makes the context's device current.
 int set_device(cm_ctx *ctx);

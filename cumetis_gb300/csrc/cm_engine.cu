@@ -173,6 +173,8 @@ struct cm_engine {
       if (rc == CM_OK && !B->empty()) rc = B->step(fin);
       if (rc == CM_OK) rc = cm::cuda_status(cudaStreamSynchronize(sched_ctx->stream), "batch level");
       if (rc != CM_OK) {
+        // the jobs' host arrays may still be read by an upload in flight
+        cudaStreamSynchronize(sched_ctx->stream);
         for (auto &f : fin) cm_hierarchy_free(f.second);
         fail_all(rc);
         B = std::make_unique<cm::BatchCoarsener>(sched_ctx, sched_ctx->stream);  // frees what it held

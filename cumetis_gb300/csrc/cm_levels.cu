@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
     // ---- proposals
     for (int b0 = gw * 32; b0 < n; b0 += nw * 32) {
       int nq = 0;
-      propose_span<H, true>(a, b0, 32, false, S.prop.list, [&](int v, int, int) {
+      propose_span<H, true, 8>(a, b0, 32, false, S.prop.list, [&](int v, int, int) {
         const unsigned q = __ballot_sync(0xffffffffu, v >= 0);
         if (v >= 0) S.prop.queue[nq + __popc(q & below)] = v;
         nq += __popc(q);

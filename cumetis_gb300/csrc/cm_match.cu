@@ -174,9 +174,14 @@ __global__ void __launch_bounds__(kPrepThreads, ALL ? kFirstMinBlocks : kFirstMi
 }
 
 // The proposals (propose_span); free vertices that need a scan of a long row are
-// queued (slot 1).
+// queued (slot 1).  Bound by latency.  Hashed ties end chains early and leave the
+// chip to many short ones: 48 registers for 5 resident blocks per SM and 4
+// entries a rescan step (1400 x 1400 grid's matching 269 -> 241 us, R-MAT 22's
+// 2026 -> 1991).  Ties by id make few long chains, which want their reads in
+// flight together and no spills (a 700 x 700 triangulation: 3.51 ms with those
+// settings, 2.95 ms with 8 entries and lists read ahead).
 template <bool H>
-__global__ void __launch_bounds__(kPrepThreads) k_match_propose(MatchArgs a) {
+__global__ void __launch_bounds__(kPrepThreads, H ? 5 : 0) k_match_propose(MatchArgs a) {
   __shared__ int sh_v[kPrepThreads / 32][kSpan];
   int *list = sh_v[threadIdx.x >> 5];
   const bool all = all_eligible(a);
@@ -184,8 +189,9 @@ __global__ void __launch_bounds__(kPrepThreads) k_match_propose(MatchArgs a) {
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   const int n = a.n;
   for (long long b0 = (long long)gwarp * a.span; b0 < n; b0 += (long long)nwarps * a.span) {
-    propose_span<H, false>(a, b0, a.span, all, list,
-                           [&](int v, int xs, int deg) { append_scan(a, 1, 1, v >= 0, v, xs, deg); });
+    propose_span<H, !H, H ? 4 : 8>(a, b0, a.span, all, list, [&](int v, int xs, int deg) {
+      append_scan(a, 1, 1, v >= 0, v, xs, deg);
+    });
   }
 }
 

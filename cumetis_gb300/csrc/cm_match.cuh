@@ -584,11 +584,11 @@ __device__ __forceinline__ void short_list(const MatchArgs &a, int v, int xs, in
 }
 
 // Best candidate of a short row (deg <= kSerialDeg) that takes v now, by one
-// lane; *seen = the proposal it holds.  -1: none.
-template <bool H>
+// lane, AHEAD entries at a time; *seen = the proposal it holds.  -1: none.
+template <bool H, int AHEAD>
 __device__ __forceinline__ int rescan_short(const MatchArgs &a, int v, int xs, int deg, bool all, int hb, int *weight,
                                             unsigned long long *seen) {
-  constexpr int kHalf = 8;
+    constexpr int kHalf = AHEAD;
   const long long vw = all ? 0 : a.vwgt[v], cap = all ? 0 : weight_cap(a, v);
   TopK<H, 1> t1;
   *seen = 0ull;
@@ -632,10 +632,10 @@ __device__ __forceinline__ int rescan_short(const MatchArgs &a, int v, int xs, i
 // -1: nothing).  A lane whose chain has ended takes the span's next vertex.
 // list: span ints of the warp's shared memory.  AHEAD: a candidate most likely
 // gives up the vertex it was seen to hold, and that one's list is read while the
-// offer is under way: a third off a chain's step where steps are all that is
-// waited for (a 69 x 69 mesh); where the chip is full, the reads and registers
-// cost more than they give (R-MAT 22: +0.08 ms).
-template <bool H, bool AHEAD, typename Q>
+// offer is under way: it pays where chains are long (low-id ties on a 700 x 700
+// triangulation 3.21 -> 2.95 ms), and costs reads and registers where the chip is
+// full (hashed ties, R-MAT 22: +0.08 ms).  SCAN: entries of a rescan in flight.
+template <bool H, bool AHEAD, int SCAN, typename Q>
 __device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, int span, bool all, int *list, Q queue) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -673,7 +673,7 @@ __device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, i
         qx = a.xadj[cur];
         qdeg = a.xadj[cur + 1] - qx;
         if (qdeg > kSerialDeg) qv = cur;
-        else c = rescan_short<H>(a, cur, qx, qdeg, all, hb, &w, &held);
+        else c = rescan_short<H, SCAN>(a, cur, qx, qdeg, all, hb, &w, &held);
       }
       if (c < 0) {  // queued, or no candidate is left
         cur = -1;

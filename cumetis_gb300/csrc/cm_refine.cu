@@ -69,85 +69,179 @@ __global__ void k_part_weights(int n, int *__restrict__ where, const int *__rest
       if (h[i]) atomicAdd(&pwgts[i], h[i]);
 }
 
-// Balance window of each part from the total vertex weight (Sum_maxmin_pwgts).
-__global__ void k_part_bounds(int nparts, float tp, const int *__restrict__ pwgts, int *__restrict__ maxw,
-                              int *__restrict__ minw) {
-  __shared__ long long s_tot;
-  if (threadIdx.x == 0) s_tot = 0;
-  __syncthreads();
-  long long t = 0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) t += pwgts[i];
-  atomicAdd((unsigned long long *)&s_tot, (unsigned long long)t);
-  __syncthreads();
-  const int tvwgt = (int)s_tot;
-  const float ub = 1.03f;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-    maxw[i] = (int)(__fmul_rn(__fmul_rn(tp, (float)tvwgt), ub));
-    minw[i] = (int)(__fdiv_rn(__fmul_rn(tp, (float)tvwgt), ub));
+// Boundary test and target part of a vertex with at most N entries, by one lane.
+template <int N>
+__device__ __forceinline__ int lane_target(int xs, int deg, int me, const int *__restrict__ adjncy,
+                                           const int *__restrict__ adjwgt, const int *__restrict__ where, bool *bnd) {
+  int p[N], w[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    p[i] = i < deg ? adjncy[xs + i] : -1;
+    w[i] = i < deg ? adjwgt[xs + i] : 0;
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = p[i] >= 0 ? where[p[i]] : -1;
+  int mw = 0, ow = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    if (p[i] == me) mw += w[i];
+    else ow += w[i];
+  }
+  *bnd = ow > mw;
+  if (!*bnd) return me;
+  int bw = INT_MIN, bp = INT_MAX;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    if (p[i] < 0) continue;
+    int c = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (p[j] == p[i]) c += w[j];
+    if (c > bw || (c == bw && p[i] < bp)) {
+      bw = c;
+      bp = p[i];
+    }
+  }
+  return bw > mw ? bp : me;
+}
+
+// Boundary test and target part of the vertices with at most kLaneDeg entries,
+// one lane each (a warp each left 28 of 32 lanes idle on a 5-point mesh: 131 us for
+// 1000 x 1000 vertices, now 16); the others are listed, those above kWarpDeg from
+// the end of the list backwards.
+constexpr int kLaneDeg = 16, kWarpDeg = 1024;
+__global__ void __launch_bounds__(kRefThreads)
+k_boundary_short(int n, const int *__restrict__ xadj, const int *__restrict__ adjncy, const int *__restrict__ adjwgt,
+                 const int *__restrict__ where, int *__restrict__ flag, int *__restrict__ target,
+                 int *__restrict__ longer, int *nlonger) {
+  const int lane = threadIdx.x & 31;
+  const long long gw = (blockIdx.x * (long long)kRefThreads + threadIdx.x) >> 5;
+  const long long nw = (long long)gridDim.x * kRefWarps;
+  for (long long b0 = gw * 32; b0 < n; b0 += nw * 32) {
+    const long long v = b0 + lane;
+    int xs = 0, deg = 0, t = 0;
+    bool bnd = false;
+    if (v < n) {
+      xs = xadj[v];
+      deg = xadj[v + 1] - xs;
+    }
+    const bool listed = deg > kLaneDeg;
+    if (v < n && !listed) {
+      t = where[v];
+      if (deg > 0 && deg <= kLaneDeg / 2) t = lane_target<kLaneDeg / 2>(xs, deg, t, adjncy, adjwgt, where, &bnd);
+      else if (deg > 0) t = lane_target<kLaneDeg>(xs, deg, t, adjncy, adjwgt, where, &bnd);
+      flag[v] = bnd ? 1 : 0;
+      target[v] = t;
+    }
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned mid = __ballot_sync(0xffffffffu, listed && deg <= kWarpDeg);
+    const unsigned top = __ballot_sync(0xffffffffu, deg > kWarpDeg);
+    if (mid | top) {
+      int base = 0;
+      if (lane == 0 && mid) base = atomicAdd(nlonger, __popc(mid));
+      if (lane == 1 && top) base = atomicAdd(nlonger + 1, __popc(top));
+      const int bm = __shfl_sync(0xffffffffu, base, 0), bt = __shfl_sync(0xffffffffu, base, 1);
+      if (listed && deg <= kWarpDeg) longer[bm + __popc(mid & below)] = (int)v;
+      if (deg > kWarpDeg) longer[n - 1 - bt - __popc(top & below)] = (int)v;
+    }
   }
 }
 
-// Boundary test and target part, one warp per vertex.  acc holds one zeroed
-// int per part for this warp (shared memory when k <= kSmemParts, else a
-// global slice); it is zero again when the warp moves on.
+// Boundary test and target part of one vertex by NT threads (a warp, or the
+// block); acc: one zeroed int per part, zero again at the end; red: NT / 32 + 1
+// int2 of shared memory (unused by a warp).
+template <int NT>
+__device__ __forceinline__ void group_target(int v, const int *__restrict__ xadj, const int *__restrict__ adjncy,
+                                             const int *__restrict__ adjwgt, const int *__restrict__ where, int *acc,
+                                             int2 *red, int *__restrict__ flag, int *__restrict__ target) {
+  const int tid = NT == 32 ? threadIdx.x & 31 : threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int xs = xadj[v], xe = xadj[v + 1], me = where[v];
+  int mw = 0, ow = 0;
+  for (int j = xs + tid; j < xe; j += NT) {
+    const int w = adjwgt[j];
+    if (where[adjncy[j]] == me) mw += w;
+    else ow += w;
+  }
+  mw = __reduce_add_sync(0xffffffffu, mw);
+  ow = __reduce_add_sync(0xffffffffu, ow);
+  if (NT > 32) {
+    if (lane == 0) red[wid] = make_int2(mw, ow);
+    __syncthreads();
+    const int2 x = lane < NT / 32 ? red[lane] : make_int2(0, 0);
+    mw = __reduce_add_sync(0xffffffffu, x.x);
+    ow = __reduce_add_sync(0xffffffffu, x.y);
+    __syncthreads();
+  }
+  const bool bnd = ow > mw;
+  int t = me;
+  if (bnd) {
+    for (int j = xs + tid; j < xe; j += NT) atomicAdd(&acc[where[adjncy[j]]], adjwgt[j]);
+    row_sync<NT>();
+    int bw = INT_MIN, bp = INT_MAX;
+    for (int j = xs + tid; j < xe; j += NT) {
+      const int p = where[adjncy[j]];
+      const int w = acc[p];
+      if (w > bw || (w == bw && p < bp)) {
+        bw = w;
+        bp = p;
+      }
+    }
+    int wmax = __reduce_max_sync(0xffffffffu, bw);
+    int pmin = __reduce_min_sync(0xffffffffu, bw == wmax ? bp : INT_MAX);
+    if (NT > 32) {
+      if (lane == 0) red[wid] = make_int2(wmax, pmin);
+      __syncthreads();
+      const int2 x = lane < NT / 32 ? red[lane] : make_int2(INT_MIN, INT_MAX);
+      wmax = __reduce_max_sync(0xffffffffu, x.x);
+      pmin = __reduce_min_sync(0xffffffffu, x.x == wmax ? x.y : INT_MAX);
+    }
+    t = wmax > acc[me] ? pmin : me;
+    row_sync<NT>();
+    for (int j = xs + tid; j < xe; j += NT) acc[where[adjncy[j]]] = 0;
+    row_sync<NT>();
+  }
+  if (tid == 0) {
+    flag[v] = bnd ? 1 : 0;
+    target[v] = t;
+  }
+}
+
+// The listed vertices: the longest rows one block each (R-MAT 17: 204 us when one
+// warp made the hub's three passes, now 53), then
+// the others one warp each (round robin: an R-MAT graph's long rows have
+// neighbouring ids).  acc: one zeroed int per part for each warp (shared memory
+// when k <= kSmemParts, else a global slice).
 template <bool kShared>
 __global__ void __launch_bounds__(kRefThreads)
-k_boundary(int n, const int *__restrict__ xadj, const int *__restrict__ adjncy, const int *__restrict__ adjwgt,
-           const int *__restrict__ where, int nparts, int *__restrict__ acc_global, int *__restrict__ flag,
-           int *__restrict__ target) {
+k_boundary(int n, const int *__restrict__ longer, const int *__restrict__ nlonger, const int *__restrict__ xadj,
+           const int *__restrict__ adjncy, const int *__restrict__ adjwgt, const int *__restrict__ where, int nparts,
+           int *__restrict__ acc_global, int *__restrict__ flag, int *__restrict__ target) {
   extern __shared__ int acc_s[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long gw = (long long)blockIdx.x * kRefWarps + warp;
-  const long long nw = (long long)gridDim.x * kRefWarps;
-  int *acc = kShared ? acc_s + warp * nparts : acc_global + gw * nparts;
+  __shared__ int2 red[kRefWarps + 1];
+  const int warp = threadIdx.x >> 5;
+  const int gw = blockIdx.x * kRefWarps + warp, nw = gridDim.x * kRefWarps;
+  const int count = nlonger[0], top = nlonger[1];
+  if ((int)blockIdx.x * kRefWarps >= count && (int)blockIdx.x >= top) return;
+  int *acc_block = kShared ? acc_s : acc_global + (long long)blockIdx.x * kRefWarps * nparts;
   if (kShared) {
     for (int i = threadIdx.x; i < kRefWarps * nparts; i += kRefThreads) acc_s[i] = 0;
     __syncthreads();
   }
-  for (long long v = gw; v < n; v += nw) {
-    const int xs = xadj[v], xe = xadj[v + 1], me = where[v];
-    int mw = 0, ow = 0;
-    for (int j = xs + lane; j < xe; j += 32) {
-      const int w = adjwgt[j];
-      if (where[adjncy[j]] == me) mw += w;
-      else ow += w;
-    }
-    mw = __reduce_add_sync(0xffffffffu, mw);
-    ow = __reduce_add_sync(0xffffffffu, ow);
-    const bool bnd = ow > mw;
-    int t = me;
-    if (bnd) {
-      for (int j = xs + lane; j < xe; j += 32) atomicAdd(&acc[where[adjncy[j]]], adjwgt[j]);
-      __syncwarp();
-      int bw = INT_MIN, bp = INT_MAX;
-      for (int j = xs + lane; j < xe; j += 32) {
-        const int p = where[adjncy[j]];
-        const int w = acc[p];
-        if (w > bw || (w == bw && p < bp)) {
-          bw = w;
-          bp = p;
-        }
-      }
-      const int wmax = __reduce_max_sync(0xffffffffu, bw);
-      const int pmin = __reduce_min_sync(0xffffffffu, bw == wmax ? bp : INT_MAX);
-      const int mew = acc[me];
-      t = wmax > mew ? pmin : me;
-      __syncwarp();
-      for (int j = xs + lane; j < xe; j += 32) acc[where[adjncy[j]]] = 0;
-      __syncwarp();
-    }
-    if (lane == 0) {
-      flag[v] = bnd ? 1 : 0;
-      target[v] = t;
-    }
-  }
+  for (int i = blockIdx.x; i < top; i += gridDim.x)
+    group_target<kRefThreads>(longer[n - 1 - i], xadj, adjncy, adjwgt, where, acc_block, red, flag, target);
+  for (int i = gw; i < count; i += nw)
+    group_target<32>(longer[i], xadj, adjncy, adjwgt, where, acc_block + warp * nparts, red, flag, target);
 }
 
-// Exclusive scan of flags[0..n) into pos[0..n] (decoupled look-back over
-// 2048-entry tiles); pos[n] = total.
+// Boundary list in vertex order (decoupled look-back over 2048-vertex tiles), and
+// the entries of every target part in every kSortBlock entries of the list (the
+// first step of the stable counting sort by target: counts, prefix over blocks,
+// in-order scatter).  *d_nb = the list's length.
 constexpr int kScanThreads = 256, kScanItems = 8;
 __global__ void __launch_bounds__(kScanThreads)
-k_scan_flags(const int *__restrict__ flags, int n, int *__restrict__ pos, unsigned long long *lb, DevStatus *st) {
+k_boundary_list(const int *__restrict__ flags, const int *__restrict__ target, int n, int nparts,
+                int *__restrict__ bnd_v, int *__restrict__ bnd_t, int *__restrict__ bhist, int *__restrict__ d_nb,
+                unsigned long long *lb, DevStatus *st) {
   __shared__ int s_tile;
   __shared__ unsigned long long s_warp[kScanThreads / 32];
   __shared__ unsigned long long s_excl;
@@ -175,64 +269,76 @@ k_scan_flags(const int *__restrict__ flags, int n, int *__restrict__ pos, unsign
     if (lane == 0) s_excl = ex;
   }
   __syncthreads();
-  unsigned long long run = s_excl + s_warp[wid] + inc - sum;
+  long long run = (long long)(s_excl + s_warp[wid] + inc - sum);
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i >= n) break;
-    pos[base + i] = (int)run;
-    run += (unsigned)v[i];
-    if (base + i == n - 1) pos[n] = (int)run;
+    if (v[i]) {
+      const int t = target[base + i];
+      bnd_v[run] = (int)(base + i);
+      bnd_t[run] = t;
+      atomicAdd(&bhist[run / kSortBlock * nparts + t], 1);
+      ++run;
+    }
+    if (base + i == n - 1) *d_nb = (int)run;
   }
 }
 
-// Boundary list in vertex order: bnd_v[pos[v]] = v, bnd_t[...] = target[v].
-__global__ void k_compact(int n, const int *__restrict__ flag, const int *__restrict__ pos,
-                          const int *__restrict__ target, int *__restrict__ bnd_v, int *__restrict__ bnd_t) {
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x)
-    if (flag[v]) {
-      bnd_v[pos[v]] = (int)v;
-      bnd_t[pos[v]] = target[v];
-    }
-}
-
-// Stable counting sort of the boundary list by target part, three steps:
-// per-block counts, per-part prefix over blocks, in-order scatter.
-__global__ void k_sort_counts(const int *__restrict__ d_nb, const int *__restrict__ bnd_t, int nparts,
-                              int *__restrict__ bhist) {
-  const int nb = *d_nb;
-  const long long b = blockIdx.x;
-  for (long long i = b * kSortBlock + threadIdx.x; i < min((long long)nb, (b + 1) * kSortBlock); i += blockDim.x)
-    atomicAdd(&bhist[b * nparts + bnd_t[i]], 1);
-}
-
-__global__ void k_sort_offsets(const int *__restrict__ d_nb, int nparts, int *__restrict__ bhist,
-                               int *__restrict__ pcount) {
+// Prefix of every part's counts over the blocks (one warp a part), then by the
+// last block to finish: pstart[t], the exclusive prefix of the parts' totals, and
+// the parts' balance windows from the total vertex weight (Sum_maxmin_pwgts).
+constexpr int kOffsetThreads = 256;
+__global__ void __launch_bounds__(kOffsetThreads)
+k_sort_offsets(const int *__restrict__ d_nb, int nparts, float tp, const int *__restrict__ pwgts,
+               int *__restrict__ bhist, int *pcount, int *__restrict__ pstart, int *__restrict__ maxw,
+               int *__restrict__ minw, unsigned *done) {
+  __shared__ int scan[kOffsetThreads / 32 + 1];
+  __shared__ bool s_last;
+  __shared__ unsigned long long s_tot;
+  const int lane = threadIdx.x & 31;
   const int nb = *d_nb;
   const int nblocks = (nb + kSortBlock - 1) / kSortBlock;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nparts; t += gridDim.x * blockDim.x) {
+  const int warps = gridDim.x * (kOffsetThreads / 32);
+  for (int t = blockIdx.x * (kOffsetThreads / 32) + (threadIdx.x >> 5); t < nparts; t += warps) {
     int run = 0;
-    for (int b = 0; b < nblocks; ++b) {
-      const int c = bhist[(size_t)b * nparts + t];
-      bhist[(size_t)b * nparts + t] = run;
-      run += c;
+    for (int b0 = 0; b0 < nblocks; b0 += 32) {
+      const int b = b0 + lane;
+      const int c = b < nblocks ? bhist[(size_t)b * nparts + t] : 0;
+      const int inc = warp_inclusive_scan_i32(c);
+      if (b < nblocks) bhist[(size_t)b * nparts + t] = run + inc - c;
+      run += __shfl_sync(0xffffffffu, inc, 31);
     }
-    pcount[t] = run;
+    if (lane == 0) pcount[t] = run;
   }
-}
-
-// pstart[t] = exclusive prefix of pcount (one block).
-__global__ void k_part_starts(int nparts, const int *__restrict__ pcount, int *__restrict__ pstart) {
-  __shared__ int scan[1024 / 32 + 1];
+  __threadfence();
+  if (threadIdx.x == 0) s_tot = 0ull;
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
   int carry = 0;
-  for (int b = 0; b < nparts; b += 1024) {
+  long long wt = 0;
+  for (int b = 0; b < nparts; b += kOffsetThreads) {
     const int t = b + threadIdx.x;
-    const int c = t < nparts ? pcount[t] : 0;
+    const int c = t < nparts ? __ldcg(pcount + t) : 0;
     int tot;
-    const int ex = block_exclusive_scan<1024>(c, scan, &tot);
-    if (t < nparts) pstart[t] = carry + ex;
+    const int ex = block_exclusive_scan<kOffsetThreads>(c, scan, &tot);
+    if (t < nparts) {
+      pstart[t] = carry + ex;
+      wt += pwgts[t];
+    }
     carry += tot;
   }
   if (threadIdx.x == 0) pstart[nparts] = carry;
+  atomicAdd(&s_tot, (unsigned long long)wt);
+  __syncthreads();
+  const int tvwgt = (int)(long long)s_tot;
+  const float ub = 1.03f;
+  for (int i = threadIdx.x; i < nparts; i += kOffsetThreads) {
+    maxw[i] = (int)(__fmul_rn(__fmul_rn(tp, (float)tvwgt), ub));
+    minw[i] = (int)(__fdiv_rn(__fmul_rn(tp, (float)tvwgt), ub));
+  }
 }
 
 // One warp per block of kSortBlock entries, in order: an entry's place is its
@@ -445,47 +551,53 @@ __global__ void k_cut(int n, const int *__restrict__ xadj, const int *__restrict
 }
 
 struct RefineWs {
-  int *pwgts, *maxw, *minw, *flag, *target, *pos, *bnd_v, *bnd_t, *bhist, *pcount, *pstart, *acc;
+  int *pwgts, *maxw, *minw, *flag, *target, *bnd_v, *bnd_t, *bhist, *pcount, *pstart, *acc;
   int4 *sorted;  // boundary records (vertex, weight, part, 0) by target part
-  unsigned long long *lb, *counters;  // counters[0] = moves, [1] = cut
-  size_t bhist_ints, acc_ints, lb_words;
+  unsigned long long *counters;  // [0] = moves, [1] = cut
+  // cleared at the start of a pass, as one block: part weights, the list's
+  // length and the offsets kernel's block count, look-back words, counts
+  char *clear;
+  int *nb;
+  unsigned *done;
+  unsigned long long *lb;
+  size_t acc_ints;
 };
 
 int grid_warps(cm_ctx *ctx) { return ctx->num_sms * 8 * kRefWarps; }
 
-size_t refine_ws_bytes(cm_ctx *ctx, int64_t n, int nparts) {
+size_t pad256(size_t b) { return (b + 255) & ~(size_t)255; }
+// Bytes of the cleared block for a graph of n vertices, counts included.
+size_t clear_bytes(int64_t n, int nparts) {
   const int64_t nblocks = (n + kSortBlock - 1) / kSortBlock + 1;
+  return pad256((size_t)nparts * 4) + 256 + pad256((size_t)(n / (kScanThreads * kScanItems) + 4) * 8) +
+         pad256((size_t)nblocks * nparts * 4);
+}
+
+size_t refine_ws_bytes(cm_ctx *ctx, int64_t n, int nparts) {
   size_t b = 0;
-  b += (size_t)(3 * nparts + 2 * (nparts + 1)) * 4 + 5 * 256;
-  b += (size_t)(9 * n + 8) * 4 + 6 * 256;
-  b += (size_t)nblocks * nparts * 4 + 256;
+  b += (size_t)(2 * nparts + 2 * (nparts + 1)) * 4 + 5 * 256;
+  b += (size_t)(8 * n + 8) * 4 + 6 * 256;
+  b += clear_bytes(n, nparts) + 256;
   if (nparts > kSmemParts) b += (size_t)grid_warps(ctx) * nparts * 4 + 256;
-  b += (size_t)(n / (kScanThreads * kScanItems) + 4) * 8 + 256 + 64;
   return b + 4096;
 }
 
 int take_refine_ws(cm_ctx *ctx, int64_t n, int nparts, RefineWs &w) {
-  const int64_t nblocks = (n + kSortBlock - 1) / kSortBlock + 1;
-  w.pwgts = (int *)ws_take(ctx, (size_t)nparts * 4);
   w.maxw = (int *)ws_take(ctx, (size_t)nparts * 4);
   w.minw = (int *)ws_take(ctx, (size_t)nparts * 4);
   w.pcount = (int *)ws_take(ctx, (size_t)(nparts + 1) * 4);
   w.pstart = (int *)ws_take(ctx, (size_t)(nparts + 1) * 4);
   w.flag = (int *)ws_take(ctx, (size_t)n * 4 + 4);
   w.target = (int *)ws_take(ctx, (size_t)n * 4 + 4);
-  w.pos = (int *)ws_take(ctx, (size_t)(n + 1) * 4);
   w.bnd_v = (int *)ws_take(ctx, (size_t)n * 4 + 4);
   w.bnd_t = (int *)ws_take(ctx, (size_t)n * 4 + 4);
   w.sorted = (int4 *)ws_take(ctx, (size_t)n * 16 + 16);
-  w.bhist_ints = (size_t)nblocks * nparts;
-  w.bhist = (int *)ws_take(ctx, w.bhist_ints * 4);
+  w.clear = (char *)ws_take(ctx, clear_bytes(n, nparts));
   w.acc_ints = nparts > kSmemParts ? (size_t)grid_warps(ctx) * nparts : 0;
   w.acc = w.acc_ints ? (int *)ws_take(ctx, w.acc_ints * 4) : nullptr;
-  w.lb_words = (size_t)(n / (kScanThreads * kScanItems) + 4);
-  w.lb = (unsigned long long *)ws_take(ctx, w.lb_words * 8);
   w.counters = (unsigned long long *)ws_take(ctx, 64);
-  if (!w.pwgts || !w.maxw || !w.minw || !w.pcount || !w.pstart || !w.flag || !w.target || !w.pos || !w.bnd_v ||
-      !w.bnd_t || !w.sorted || !w.bhist || (w.acc_ints && !w.acc) || !w.lb || !w.counters)
+  if (!w.maxw || !w.minw || !w.pcount || !w.pstart || !w.flag || !w.target || !w.bnd_v || !w.bnd_t || !w.sorted ||
+      !w.clear || (w.acc_ints && !w.acc) || !w.counters)
     return cm_fail(CM_ERR_NOMEM, "refine: workspace too small");
   return CM_OK;
 }
@@ -496,37 +608,48 @@ int refine_pass(cm_ctx *ctx, const cm_graph &g, int nparts, int32_t *where, Refi
   const int n = g.nvtxs;
   if (n == 0) return CM_OK;
   const int sms = ctx->num_sms;
-  cudaMemsetAsync(w.pwgts, 0, (size_t)nparts * 4, s);
+  // the cleared block, laid out for this graph's size
+  char *c = w.clear;
+  w.pwgts = (int *)c;
+  c += pad256((size_t)nparts * 4);
+  w.nb = (int *)c;
+  w.done = (unsigned *)c + 1;
+  c += 256;
+  w.lb = (unsigned long long *)c;
+  c += pad256((size_t)(n / (kScanThreads * kScanItems) + 4) * 8);
+  w.bhist = (int *)c;
+  cudaMemsetAsync(w.clear, 0, clear_bytes(n, nparts), s);
   const size_t hsh = nparts <= 8192 ? (size_t)nparts * 4 : 0;
-  k_part_weights<<<sms * 4, 256, hsh, s>>>(n, where, g.vwgt, nparts, w.pwgts, proj_cmap, proj_cwhere);
-  // tpwgts = 1.0 / nparts rounded to float, as cuMetis_set_graph_admin stores it (cu:384)
-  k_part_bounds<<<1, 1024, 0, s>>>(nparts, (float)(1.0 / nparts), w.pwgts, w.maxw, w.minw);
+  const int vblocks = std::min(sms * 4, n / 256 + 1);
+  k_part_weights<<<vblocks, 256, hsh, s>>>(n, where, g.vwgt, nparts, w.pwgts, proj_cmap, proj_cwhere);
+  const int bblocks = std::min(sms * 8, n / kRefThreads + 1);
+  int *longer = w.bnd_v, *nlonger = w.nb + 2;  // listed until the boundary list is made
+  k_boundary_short<<<bblocks, kRefThreads, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, where, w.flag, w.target, longer,
+                                                   nlonger);
+  const int lblocks = (int)std::min<int64_t>(sms * 8, g.nedges / (kLaneDeg + 1) / kRefWarps + 1);
   if (nparts <= kSmemParts) {
     const size_t sm = (size_t)kRefWarps * nparts * 4;
     if (sm > 48 * 1024)
       cudaFuncSetAttribute(k_boundary<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_boundary<true><<<sms * 8, kRefThreads, sm, s>>>(n, g.xadj, g.adjncy, g.adjwgt, where, nparts, nullptr, w.flag,
-                                                     w.target);
+    k_boundary<true><<<lblocks, kRefThreads, sm, s>>>(n, longer, nlonger, g.xadj, g.adjncy, g.adjwgt, where, nparts,
+                                                     nullptr, w.flag, w.target);
   } else {
     cudaMemsetAsync(w.acc, 0, w.acc_ints * 4, s);
-    k_boundary<false><<<sms * 8, kRefThreads, 0, s>>>(n, g.xadj, g.adjncy, g.adjwgt, where, nparts, w.acc, w.flag,
-                                                     w.target);
+    k_boundary<false><<<lblocks, kRefThreads, 0, s>>>(n, longer, nlonger, g.xadj, g.adjncy, g.adjwgt, where, nparts,
+                                                     w.acc, w.flag, w.target);
   }
-  cudaMemsetAsync(w.lb, 0, w.lb_words * 8, s);
   const int scan_tiles = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
-  k_scan_flags<<<scan_tiles, kScanThreads, 0, s>>>(w.flag, n, w.pos, w.lb, ctx->d_status);
-  k_compact<<<sms * 4, 256, 0, s>>>(n, w.flag, w.pos, w.target, w.bnd_v, w.bnd_t);
-  const int *d_nb = w.pos + n;
+  k_boundary_list<<<scan_tiles, kScanThreads, 0, s>>>(w.flag, w.target, n, nparts, w.bnd_v, w.bnd_t, w.bhist, w.nb,
+                                                      w.lb, ctx->d_status);
   const int sort_blocks = (n + kSortBlock - 1) / kSortBlock;
-  cudaMemsetAsync(w.bhist, 0, (size_t)sort_blocks * nparts * 4, s);
-  k_sort_counts<<<sort_blocks, 256, 0, s>>>(d_nb, w.bnd_t, nparts, w.bhist);
-  k_sort_offsets<<<(nparts + 255) / 256, 256, 0, s>>>(d_nb, nparts, w.bhist, w.pcount);
-  k_part_starts<<<1, 1024, 0, s>>>(nparts, w.pcount, w.pstart);
+  // tpwgts = 1.0 / nparts rounded to float, as cuMetis_set_graph_admin stores it (cu:384)
+  k_sort_offsets<<<std::min(sms, (nparts + 7) / 8), kOffsetThreads, 0, s>>>(
+      w.nb, nparts, (float)(1.0 / nparts), w.pwgts, w.bhist, w.pcount, w.pstart, w.maxw, w.minw, w.done);
   k_sort_scatter<<<sort_blocks, 32, nparts <= kSmemParts ? nparts * 4 : 0, s>>>(
-      d_nb, w.bnd_v, w.bnd_t, nparts, w.bhist, w.pstart, g.vwgt, where, w.sorted);
+      w.nb, w.bnd_v, w.bnd_t, nparts, w.bhist, w.pstart, g.vwgt, where, w.sorted);
   k_moves<true><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, where, w.counters);
   k_moves<false><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, where, w.counters);
-  ctx->launches += 11;
+  ctx->launches += 8;
   return check_launch(ctx, "refine");
 }
 

@@ -306,33 +306,76 @@ __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, i
     if (k[u] == v) k[u] = -1;
 }
 
-// Inserts x into the descending list tw (the KK largest values seen, with
-// repeats).
-template <int KK>
-__device__ __forceinline__ void wlist_insert(int (&tw)[KK], int x) {
+// The warp's best KK candidates over entries [b, e), e - b <= 64, of v's row,
+// with FILTER among those that v beats the proposal of; every lane gets the list.
+template <bool H, int KK, bool FILTER>
+__device__ __forceinline__ TopK<H, KK> pair_best(const MatchArgs &a, int v, int b, int e, bool all, int hb) {
+  const int lane = threadIdx.x & 31, j0 = b + lane, j1 = j0 + 32;
+  int k0 = -1, k1 = -1, w0 = 0, w1 = 0;
+  if (j0 < e) {
+    k0 = a.adjncy[j0];
+    w0 = a.adjwgt[j0];
+  }
+  if (j1 < e) {
+    k1 = a.adjncy[j1];
+    w1 = a.adjwgt[j1];
+  }
+  if (k0 == v) k0 = -1;
+  if (k1 == v) k1 = -1;
+  if (!all) {
+    const long long vw = a.vwgt[v], cap = weight_cap(a, v);
+    const int x0 = k0 >= 0 ? a.vwgt[k0] : 0, x1 = k1 >= 0 ? a.vwgt[k1] : 0;
+    if (!pair_fits(cap, vw, x0)) k0 = -1;
+    if (!pair_fits(cap, vw, x1)) k1 = -1;
+  }
+  if (FILTER) {
+    const unsigned long long y0 = k0 >= 0 ? ld_best(a, k0) : 0ull, y1 = k1 >= 0 ? ld_best(a, k1) : 0ull;
+    if (k0 >= 0 && !beats<H>(best_key(v, w0), y0, v, k0, hb)) k0 = -1;
+    if (k1 >= 0 && !beats<H>(best_key(v, w1), y1, v, k1, hb)) k1 = -1;
+  }
+  Cand<H> c0, c1;
+  if (k0 >= 0) c0 = Cand<H>::make(v, k0, w0, hb);
+  if (k1 >= 0) c1 = Cand<H>::make(v, k1, w1, hb);
+  if (c1.better(c0)) {
+    const Cand<H> t = c0;
+    c0 = c1;
+    c1 = t;
+  }
+  TopK<H, KK> out;
 #pragma unroll
   for (int i = 0; i < KK; ++i) {
-    const int hi = max(tw[i], x);
-    x = min(tw[i], x);
-    tw[i] = hi;
+    const Cand<H> win = c0.warp_best();
+    out.c[i] = win;
+    if (!win.valid()) break;
+    if (c0.same(win)) {
+      c0 = c1;
+      c1 = Cand<H>();
+    }
+    if (c0.same(win)) c0 = Cand<H>();  // the lane's second entry is the same parallel edge
   }
+  return out;
 }
 
 // The warp's best KK candidates over entries [b, e) (e - b <= kMatchChunk) of v's
-// row; every lane gets the list.  Hash order: most entries are lighter than
-// the chunk's KK-th heaviest eligible entry and can never enter the list, so
-// a weight threshold W is found first and only entries of weight >= W get an
-// edge hash and a full comparison.  W is the KK-th largest weight of the
-// union of the lanes' own KK heaviest (a sub-multiset of the chunk), so at
-// least KK entries weigh >= W and the chunk's best KK are all among them.
-// The qualifying entries (usually KK plus the ties at W) are packed one per
-// lane through the warp's 32-entry buffer wbuf; more than 32 of them (many
+// row; every lane gets the list.  Hash order: most entries are lighter than the
+// chunk's KK-th heaviest eligible entry and can never enter the list, so a
+// weight threshold W is found first and only entries of weight >= W get an edge
+// hash and a full comparison.  W is the KK-th largest of the lanes' heaviest
+// eligible weights, so at least KK entries weigh >= W and the chunk's best KK
+// are all among them (a list of the KK heaviest weights per lane gives a slightly
+// higher W for eight times the instructions: R-MAT 22's matching 1937 against
+// 1891 us).  The
+// qualifying entries (usually KK, a few more and the ties at W) are packed one
+// per lane through the warp's 32-entry buffer wbuf; more than 32 of them (many
 // equal weights) take the per-lane lists instead.
 template <bool H, int KK, int FILTER>
 __device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, int b, int e, bool all, int2 *wbuf) {
   constexpr int U = kMatchChunk / 32;
   const int nu = (e - b + 31) >> 5;
   const int hb = hash_base(a, v);
+  // Rows and last chunks of up to 64 entries (most of a skewed graph's): two
+  // entries a lane, every one compared in full, against a proposal too.
+  if (nu <= 2) return pair_best<H, KK, FILTER != kStatic>(a, v, b, e, all, hb);
   int k[U], w[U];
   load_entries<H, FILTER>(a, v, b, e, all, hb, k, w);
   if constexpr (!H) {
@@ -345,36 +388,29 @@ __device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, int
   } else {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int tw[KK], rem = 0;
-#pragma unroll
-    for (int i = 0; i < KK; ++i) tw[i] = INT_MIN;
+    int top = INT_MIN;
+    bool has = false;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (u >= nu) break;
       if (k[u] >= 0) {
-        wlist_insert(tw, w[u]);
-        ++rem;
+        top = max(top, w[u]);
+        has = true;
       }
     }
-    rem = min(rem, KK);
-    // threshold: pop the lanes' list heads in descending order until KK
-    // entries are taken (or every list is empty: then all eligible entries
-    // qualify, W being the lightest of them)
+    // the lanes' heaviest in descending order until KK are taken; with fewer
+    // lanes than that every eligible entry qualifies
     int W = INT_MIN, taken = 0;
 #pragma unroll
     for (int r = 0; r < KK; ++r) {
-      const bool has = rem > 0;
-      if (!__ballot_sync(full, has)) break;
-      const int mine = has ? tw[0] : INT_MIN;
-      const int mx = __reduce_max_sync(full, mine);
-      const bool pop = has && mine == mx;
-      taken += __popc(__ballot_sync(full, pop));
-      W = mx;
-      if (pop) {
-#pragma unroll
-        for (int i = 0; i + 1 < KK; ++i) tw[i] = tw[i + 1];
-        --rem;
+      if (!__ballot_sync(full, has)) {
+        W = INT_MIN;
+        break;
       }
+      W = __reduce_max_sync(full, has ? top : INT_MIN);
+      const bool pop = has && top == W;
+      taken += __popc(__ballot_sync(full, pop));
+      has = has && !pop;
       if (taken >= KK) break;
     }
     int total = 0;
@@ -417,9 +453,9 @@ __device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, int
     }
     // Identical entries (parallel edges of equal weight) count once in the
     // list but each in `taken`: a list left short although lighter entries
-    // exist is recomputed over every eligible entry, so that a short list
+    // may exist is recomputed over every eligible entry, so that a short list
     // still means "no other candidate".
-    if (taken >= KK && !out.c[KK - 1].valid()) {
+    if (W != INT_MIN && !out.c[KK - 1].valid()) {
       TopK<H, KK> t;
 #pragma unroll
       for (int u = 0; u < U; ++u)

@@ -731,13 +731,15 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   int *class_ctr = reinterpret_cast<int *>(ctr) + 2;
   int *unit_last = reinterpret_cast<int *>(ctr) + 2 + kRowClasses;
   DevStatus *st = ctx->d_status;
+  const bool any_big = row_bound > kTinyMax;
   cudaMemsetAsync(ctr, 0, 128, s);
   cudaMemsetAsync(&st->max_row, 0, sizeof(int), s);
-  cudaMemsetAsync(map_lb, 0, (size_t)(map_tiles + 3) * 8, s);
+  if (any_big) cudaMemsetAsync(map_lb, 0, (size_t)(map_tiles + 3) * 8, s);
   cudaMemsetAsync(scan_lb, 0, (size_t)(scan_tiles + 3) * 8, s);
   int rc = launch_cmap(ctx, (int32_t)n, fine->xadj, fine->vwgt, match, cmap, leader, coarse->vwgt, eoff,
                        d_sizes /* n' lands in d_sizes[0] */, long_list, kTinyMax, kChunk, ctr, chunk_row, class_list,
-                       class_ctr, m, row_meta, row_bound > kTinyMax ? cplace : nullptr, s);
+                       class_ctr, m, row_meta, any_big ? cplace : nullptr, any_big ? nullptr : first_row, unit_last, kTinyDiag,
+                       (int32_t)(nunits + 2), s);
   if (rc) return rc;
   const int sms = ctx->num_sms;
 
@@ -748,7 +750,6 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
   // picks) and their number in ucount[c].  Classes above row_bound (an upper
   // bound of the expanded row length known to the caller) cannot have rows
   // and are not launched.
-  const bool any_big = row_bound > kTinyMax;
   const bool chunked = row_bound > kChunk;
   stage_begin(ctx, s);
   if (any_big) {
@@ -778,9 +779,11 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
       ctx->launches++;
     }
   }
-  k_unit_map<<<(unsigned)std::max<int64_t>(1, map_tiles), kMapThreads, 0, s>>>(d_sizes, eoff, first_row, unit_last,
-                                                                                map_lb, st);
-  ctx->launches++;
+  if (any_big) {  // else the coarse map has marked the units
+    k_unit_map<<<(unsigned)std::max<int64_t>(1, map_tiles), kMapThreads, 0, s>>>(d_sizes, eoff, first_row, unit_last,
+                                                                                  map_lb, st);
+    ctx->launches++;
+  }
   const unsigned tiny_grid = grid_for((int64_t)sms * ctx->unit_blocks_per_sm, (nunits + kTinyWarps - 1) / kTinyWarps);
   k_tiny_units<<<tiny_grid, 32 * kTinyWarps, kTinyWarps * sizeof(TinySmem), s>>>(fine->adjncy, fine->adjwgt, cmap, d_sizes, first_row, unit_last,
                                                        row_meta, eoff, stage1, ucount, st);

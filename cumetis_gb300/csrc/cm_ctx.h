@@ -164,12 +164,15 @@ int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, 
 // long_chunk entries by size class (class_offset(m, long_threshold, k) of
 // class_list, counts in class_ctr[k]), longer ones as chunked rows.  cplace
 // (int2 per vertex, optional): the vertex's coarse id and that row's expanded
-// offset together.
+// offset together.  first_row (max_units entries, optional, when no row is longer
+// than long_threshold): first row of every unit of unit_diag diagonals, the last
+// unit in *unit_last.
 int launch_cmap(cm_ctx *ctx, int32_t n, const int32_t *xadj, const int32_t *vwgt, const int32_t *match,
                 int32_t *cmap, int32_t *leader, int32_t *cvwgt, int32_t *eoff, int32_t *d_cnvtxs,
                 int32_t *long_list, int32_t long_threshold, int32_t long_chunk, unsigned long long *d_long_ctr,
                 int32_t *chunk_row, int32_t *class_list, int32_t *class_ctr, int64_t m, void *row_meta,
-                void *cplace, cudaStream_t s);
+                void *cplace, int32_t *first_row, int32_t *unit_last, int32_t unit_diag, int32_t max_units,
+                cudaStream_t s);
 // row_bound: an upper bound of the longest expanded coarse row (INT64_MAX
 // when unknown); kernels of row classes above it are not launched.
 int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int32_t *cmap, cm_graph *coarse,

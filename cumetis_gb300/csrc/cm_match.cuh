@@ -306,6 +306,18 @@ __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, i
     if (k[u] == v) k[u] = -1;
 }
 
+// Chains end by themselves (every step improves some best[]); a limit all the
+// same: true, with CM_ERR_LIMIT recorded, once a warp's loop has run past the
+// wait limit (looked at every 65536 turns).
+__device__ __forceinline__ bool chain_overrun(const MatchArgs &a, unsigned turn, uint64_t &since) {
+  if ((turn & 0xffffu) != 0xffffu) return false;
+  const uint64_t now = global_timer_ns();
+  if (since == 0) since = now;
+  if (now - since <= kWaitLimitNs) return false;
+  if ((threadIdx.x & 31) == 0) record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
+  return true;
+}
+
 // The warp's best KK candidates over entries [b, e), e - b <= 64, of v's row,
 // with FILTER among those that v beats the proposal of; every lane gets the list.
 template <bool H, int KK, bool FILTER>
@@ -687,7 +699,9 @@ __device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, i
   __syncwarp();
   int cur = -1, hb = 0;
   List L;
-  for (;;) {
+  uint64_t since = 0;
+  for (unsigned turn = 0;; ++turn) {
+    if (chain_overrun(a, turn, since)) break;
     const unsigned idle = __ballot_sync(0xffffffffu, cur < 0);
     if (taken < cnt && idle) {
       const int at = taken + __popc(idle & below);
@@ -758,7 +772,9 @@ __device__ __forceinline__ void warp_chain(const MatchArgs &a, int v, int xs, in
   };
   if (scanned) take(r);
   else L.id[0] = kUnknown;
-  for (;;) {
+  uint64_t since = 0;
+  for (unsigned turn = 0;; ++turn) {
+    if (chain_overrun(a, turn, since)) return;
     if (L.id[0] == kUnknown) {
       if (cur != v || scanned) {
         xs = a.xadj[cur];

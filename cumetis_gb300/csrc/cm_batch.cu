@@ -180,6 +180,7 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
     a.h = new cm_hierarchy();
     a.h->device = ctx_->device;
     a.h->stream = s_;
+    a.h->host_direct = ctx_->reads_host;
     a.h->slabs.push_back(slab);
     cm_level L;
     carve_level(p, n, m, L);

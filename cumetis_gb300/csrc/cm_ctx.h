@@ -14,7 +14,7 @@ struct cm_ctx {
   int device = 0;
   int num_sms = 0;
   int max_smem_optin = 0;       // bytes of dynamic shared memory a block may opt into
-  bool reads_host = false;      // kernels may read any host memory (the host's page tables)
+  bool reads_host = false;      // kernels may access any host memory (the host's page tables)
   cm::DevStatus *d_status = nullptr;   // device status block
   cm::DevStatus *h_status = nullptr;   // pinned host mirror for readbacks
   int32_t *h_small = nullptr;          // pinned 64-byte readback buffer
@@ -86,6 +86,7 @@ struct cm_slab {
 struct cm_hierarchy {
   int device = 0;
   cudaStream_t stream = nullptr;
+  bool host_direct = false;  // its context's reads_host
   std::vector<cm_level> levels;
   int32_t maxvwgt = 0;
   std::vector<int32_t> rounds;
@@ -108,6 +109,7 @@ void stage_end(cm_ctx *ctx, int stage, cudaStream_t s);
 
 // Copies arrays from host memory (any: pageable, pinned) to the device on s.  The
 // host arrays must stay valid until the stream has run the copies.
+// (download_arrays in cm_ctx.cu takes the other direction.)
 struct HostArray {
   const void *src;
   void *dst;

@@ -311,7 +311,7 @@ __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, i
 // wait limit (looked at every 65536 turns).
 __device__ __forceinline__ bool chain_overrun(const MatchArgs &a, unsigned turn, uint64_t &since) {
   if ((turn & 0xffffu) != 0xffffu) return false;
-  const uint64_t now = global_timer_ns();
+  const uint64_t now = __shfl_sync(0xffffffffu, global_timer_ns(), 0);  // one answer for the warp
   if (since == 0) since = now;
   if (now - since <= kWaitLimitNs) return false;
   if ((threadIdx.x & 31) == 0) record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);

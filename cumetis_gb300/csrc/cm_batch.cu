@@ -148,9 +148,18 @@ void carve_level(char *p, int64_t n, int64_t m, cm_level &L) {
 
 }  // namespace
 
-BatchCoarsener::BatchCoarsener(cm_ctx *ctx, cudaStream_t s) : ctx_(ctx), s_(s) {}
+// The join's tables are rewritten by the next level, after this level's readback
+// has waited for the stream; the split's only after the next level's has.
+struct BatchCoarsener::Tables {
+  std::vector<Item> join, split;
+  std::vector<Desc> D, D2;
+  std::vector<int> vbase, gcap;
+};
+
+BatchCoarsener::BatchCoarsener(cm_ctx *ctx, cudaStream_t s) : ctx_(ctx), s_(s), tab_(new Tables) {}
 
 BatchCoarsener::~BatchCoarsener() {
+  cudaStreamSynchronize(s_);  // uploads in flight read the tables and the callers' arrays
   for (auto &it : active_) cm_hierarchy_free(it.h);
 }
 
@@ -171,6 +180,8 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
   slab->stream = s_;
   std::vector<HostArray> in;
   in.reserve(4 * count);
+  std::vector<Active> fresh;
+  fresh.reserve(count);
   for (int i = 0; i < count; ++i) {
     const cm_graph &g = graphs[i];
     const int64_t n = g.nvtxs, m = g.nedges;
@@ -190,6 +201,14 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
     in.push_back({g.adjncy, L.g.adjncy, (size_t)m * 4});
     in.push_back({g.adjwgt, L.g.adjwgt, (size_t)m * 4});
     a.h->levels.push_back(L);
+    fresh.push_back(a);
+  }
+  rc = upload_arrays(ctx_, in.data(), (int)in.size(), s_);
+  // while the arrays move: the weight limits and the longest rows
+  for (int i = 0; i < count; ++i) {
+    const cm_graph &g = graphs[i];
+    const int64_t n = g.nvtxs;
+    Active &a = fresh[i];
     int64_t tvwgt = 0, maxdeg = 0;
     for (int64_t v = 0; v < n; ++v) {
       tvwgt += g.vwgt[v];
@@ -200,9 +219,12 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
     a.row_bound = 2 * maxdeg;
     if (n == 0) {  // nothing to coarsen: an empty coarse level, as cm_coarsen makes
       char *q = nullptr;
-      if ((rc = cuda_status(cudaMallocFromPoolAsync((void **)&q, level_bytes(0, 0), ctx_->pool, s_), "batch alloc"))) {
-        cm_hierarchy_free(a.h);
-        return rc;
+      const int rc2 =
+          cuda_status(cudaMallocFromPoolAsync((void **)&q, level_bytes(0, 0), ctx_->pool, s_), "batch alloc");
+      if (rc2) {
+        if (!rc) rc = rc2;
+        active_.push_back(a);  // freed with the rest
+        continue;
       }
       cm_level C;
       carve_level(q, 0, 0, C);
@@ -215,7 +237,7 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
     }
     active_.push_back(a);
   }
-  return upload_arrays(ctx_, in.data(), (int)in.size(), s_);
+  return rc;
 }
 
 int BatchCoarsener::step(std::vector<std::pair<int64_t, cm_hierarchy *>> &finished) {
@@ -258,9 +280,13 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
   cudaStream_t s = s_;
   int64_t N = 0, M = 0, row_bound = 0;
   int32_t min_cap = INT32_MAX;
-  std::vector<int> vbase(ng + 1), ebase(ng + 1), gcap(ng);
-  std::vector<Desc> D(ng);
-  std::vector<Item> items;
+  std::vector<int> ebase(ng + 1), &vbase = tab_->vbase, &gcap = tab_->gcap;
+  std::vector<Desc> &D = tab_->D, &D2 = tab_->D2;
+  std::vector<Item> &items = tab_->join, &items2 = tab_->split;
+  vbase.resize(ng + 1);
+  gcap.resize(ng);
+  D.resize(ng);
+  items.clear();
   for (int k = 0; k < ng; ++k) {
     const Active &a = active_[grp[k]];
     const cm_graph &g = a.h->levels.back().g;
@@ -310,12 +336,14 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
   (void)take(bN);  // spare
   auto release = [&](int code) {
     cudaFreeAsync(base, s);
+    if (code) cudaStreamSynchronize(s);
     return code;
   };
-  cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(d_D, D.data(), ng * sizeof(Desc), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(d_vbase, vbase.data(), (ng + 1) * 4, cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(d_gcap, gcap.data(), ng * 4, cudaMemcpyHostToDevice, s);
+  const HostArray up[] = {{items.data(), d_items, items.size() * sizeof(Item)},
+                          {D.data(), d_D, ng * sizeof(Desc)},
+                          {vbase.data(), d_vbase, (size_t)(ng + 1) * 4},
+                          {gcap.data(), d_gcap, (size_t)ng * 4}};
+  if ((rc = upload_arrays(ctx_, up, 4, s))) return release(rc);
   const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx_->num_sms * 8, items.size()));
   k_join<<<grid, kItemThreads, 0, s>>>(d_items, (int)items.size(), d_D, U.xadj, U.adjncy, U.adjwgt, U.vwgt, vgid,
                                        (int)N, (int)M);
@@ -336,13 +364,15 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
   k_batch_sizes<<<(unsigned)((ng + 255) / 256), 256, 0, s>>>(d_vbase, ng, cmap, C.xadj, sizes, d_sz);
   ctx_->launches++;
   std::vector<int4> sz(ng);
+  const bool pinned = ng * sizeof(int4) <= cm_ctx::kReadbackBytes;
   cudaMemcpyAsync(ctx_->h_status, ctx_->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
-  cudaMemcpyAsync(sz.data(), d_sz, ng * sizeof(int4), cudaMemcpyDeviceToHost, s);
+  cudaMemcpyAsync(pinned ? ctx_->h_levels : sz.data(), d_sz, ng * sizeof(int4), cudaMemcpyDeviceToHost, s);
   if ((rc = stream_wait(ctx_, s, "batch level sync"))) return release(rc);
   if (ctx_->h_status->error) {
     rc = take_device_error(ctx_, s);
     return release(rc ? rc : CM_ERR_CUDA);
   }
+  if (pinned) std::memcpy(sz.data(), ctx_->h_levels, ng * sizeof(int4));
   const int32_t rounds = ctx_->h_status->rounds;
   const int64_t next_bound = 2 * (int64_t)ctx_->h_status->max_row;
 
@@ -357,14 +387,15 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
   slab->ptr = sp;
   slab->device = ctx_->device;
   slab->stream = s;
-  items.clear();
+  D2 = D;
+  items2.clear();
   for (int k = 0; k < ng; ++k) {
     Active &a = active_[grp[k]];
     cm_level &F = a.h->levels.back();
     cm_level L;
     carve_level(sp, sz[k].y, sz[k].w, L);
     sp += level_bytes(sz[k].y, sz[k].w);
-    Desc &d = D[k];
+    Desc &d = D2[k];
     d.oxadj = L.g.xadj;
     d.oadjncy = L.g.adjncy;
     d.oadjwgt = L.g.adjwgt;
@@ -376,9 +407,9 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
     d.cbase = sz[k].x;
     d.cebase = sz[k].z;
     d.nfine = F.g.nvtxs;
-    add_items(items, k, kItemVertices, sz[k].y, kItemVertexChunk);
-    add_items(items, k, kItemEntries, sz[k].w, kItemEntryChunk);
-    add_items(items, k, kItemFine, F.g.nvtxs, kItemVertexChunk);
+    add_items(items2, k, kItemVertices, sz[k].y, kItemVertexChunk);
+    add_items(items2, k, kItemEntries, sz[k].w, kItemEntryChunk);
+    add_items(items2, k, kItemFine, F.g.nvtxs, kItemVertexChunk);
     const int64_t n = F.g.nvtxs, cn = sz[k].y, cm_ = sz[k].w;
     a.h->levels.push_back(L);  // F is not used past this point
     a.h->slabs.push_back(slab);
@@ -390,20 +421,21 @@ int BatchCoarsener::level(const std::vector<int> &grp, std::vector<char> &stop) 
     stop[grp[k]] = go_on ? 0 : 1;
   }
   Item *d_items2 = nullptr;
-  if ((rc = cuda_status(cudaMallocFromPoolAsync((void **)&d_items2, std::max<size_t>(items.size(), 1) * sizeof(Item),
+  if ((rc = cuda_status(cudaMallocFromPoolAsync((void **)&d_items2, std::max<size_t>(items2.size(), 1) * sizeof(Item),
                                                 ctx_->pool, s),
                         "batch split items")))
     return release(rc);
-  cudaMemcpyAsync(d_items2, items.data(), items.size() * sizeof(Item), cudaMemcpyHostToDevice, s);
-  cudaMemcpyAsync(d_D, D.data(), ng * sizeof(Desc), cudaMemcpyHostToDevice, s);
-  const unsigned grid2 = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx_->num_sms * 8, items.size()));
-  k_split<<<grid2, kItemThreads, 0, s>>>(d_items2, (int)items.size(), d_D, C.xadj, C.adjncy, C.adjwgt, C.vwgt, match,
+  const HostArray up2[] = {{items2.data(), d_items2, items2.size() * sizeof(Item)}, {D2.data(), d_D, ng * sizeof(Desc)}};
+  if ((rc = upload_arrays(ctx_, up2, 2, s))) {
+    cudaFreeAsync(d_items2, s);
+    return release(rc);
+  }
+  const unsigned grid2 = (unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx_->num_sms * 8, items2.size()));
+  k_split<<<grid2, kItemThreads, 0, s>>>(d_items2, (int)items2.size(), d_D, C.xadj, C.adjncy, C.adjwgt, C.vwgt, match,
                                          cmap);
   ctx_->launches++;
   rc = check_launch(ctx_, "batch split");
   cudaFreeAsync(d_items2, s);
-  // host tables above are pageable: the copies have been staged before the
-  // calls returned, so the vectors may go
   return release(rc);
 }
 
@@ -431,6 +463,7 @@ extern "C" int cm_coarsen_batch(cm_ctx *ctx, int32_t ngraphs, const cm_graph *gr
   while (rc == CM_OK && !B.empty()) rc = B.step(fin);
   for (auto &f : fin) out[f.first] = f.second;
   if (rc != CM_OK) {
+    cudaStreamSynchronize(s);  // an upload in flight may still read the graphs
     for (int i = 0; i < ngraphs; ++i) {
       cm_hierarchy_free(out[i]);
       out[i] = nullptr;

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <utility>
+#include <memory>
 #include <vector>
 
 #include "cm_ctx.h"
@@ -38,10 +39,12 @@ class BatchCoarsener {
     cm_hierarchy *h = nullptr;
     int64_t row_bound = 0;  // bound of the next expanded row
   };
+  struct Tables;
   int level(const std::vector<int> &grp, std::vector<char> &stop);
   cm_ctx *ctx_;
   cudaStream_t s_;
   std::vector<Active> active_;
+  std::unique_ptr<Tables> tab_;  // a level's host tables, which the device may still be reading
 };
 
 }  // namespace cm

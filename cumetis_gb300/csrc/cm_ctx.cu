@@ -586,6 +586,10 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
   // largest degree): the contraction skips the kernels of row classes that
   // cannot occur.
   int64_t row_bound = 0;
+  // A small device graph's weights and rows are measured by the kernel that coarsens
+  // it; a kernel and a readback of their own cost 20 to 27 us (69x69 triangulated grid
+  // 461-474 -> 441-447 us).
+  bool measure = input_on_device && fused_fits(ctx, n0, m0, 0, params->match_mode);
   if (input_on_device) {
     L0.g = *g;
     L0.owns_graph = false;
@@ -596,16 +600,18 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
     L0.block = p;
     L0.match = (int32_t *)p;
     L0.cmap = (int32_t *)(p + bv);
-    unsigned long long *d_stats = (unsigned long long *)ws_take(ctx, 16);
-    cudaMemsetAsync(d_stats, 0, 16, s);
-    k_input_stats<<<std::max(1, ctx->num_sms * 4), 256, 0, s>>>(g->vwgt, g->xadj, n0, d_stats);
-    ctx->launches++;
-    unsigned long long *hs = reinterpret_cast<unsigned long long *>(ctx->h_small);
-    if ((rc = cuda_status(cudaMemcpyAsync(hs, d_stats, 16, cudaMemcpyDeviceToHost, s), "input stats readback")) ||
-        (rc = stream_wait(ctx, s, "input stats sync")))
-      return fail(rc);
-    tvwgt = (int64_t)hs[0];
-    row_bound = 2 * (int64_t)hs[1];
+    if (!measure) {
+      unsigned long long *d_stats = (unsigned long long *)ws_take(ctx, 16);
+      cudaMemsetAsync(d_stats, 0, 16, s);
+      k_input_stats<<<std::max(1, ctx->num_sms * 4), 256, 0, s>>>(g->vwgt, g->xadj, n0, d_stats);
+      ctx->launches++;
+      unsigned long long *hs = reinterpret_cast<unsigned long long *>(ctx->h_small);
+      if ((rc = cuda_status(cudaMemcpyAsync(hs, d_stats, 16, cudaMemcpyDeviceToHost, s), "input stats readback")) ||
+          (rc = stream_wait(ctx, s, "input stats sync")))
+        return fail(rc);
+      tvwgt = (int64_t)hs[0];
+      row_bound = 2 * (int64_t)hs[1];
+    }
   } else {
     if ((rc = alloc_level(L0, n0, m0, ctx->pool, s))) return fail(rc);
     L0.g.nvtxs = (int32_t)n0;
@@ -631,10 +637,11 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
   for (;;) {
     cm_level &F = h->levels.back();
     const int64_t n = F.g.nvtxs, m = F.g.nedges;
-    if (fused_fits(ctx, n, m, row_bound / 2, params->match_mode)) {
+    if (measure || fused_fits(ctx, n, m, row_bound / 2, params->match_mode)) {
       int produced = 0, stopped = 0;
       ctx->ws_used = level_ws_off;
-      if ((rc = launch_fused(ctx, h, params, s, &produced, &stopped, &row_bound))) return fail(rc);
+      if ((rc = launch_fused(ctx, h, params, s, &produced, &stopped, &row_bound, measure))) return fail(rc);
+      measure = false;
       if (stopped) break;
       if (produced > 0) continue;
     }

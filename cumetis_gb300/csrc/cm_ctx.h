@@ -193,9 +193,12 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
 #endif
 constexpr int64_t kFusedWork = CM_FUSED_WORK;
 size_t fused_ws_bytes(int64_t n, int64_t m);
+// With measure, the graph's longest row and weights are not known yet: the kernel
+// finds them, and produces nothing where a row is too long for it; *row_bound and
+// (where the parameters leave it open) the hierarchy's maxvwgt are set.
 bool fused_fits(const cm_ctx *ctx, int64_t n, int64_t m, int64_t max_deg, int32_t mode);
 int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaStream_t s, int *produced, int *stopped,
-                 int64_t *row_bound);
+                 int64_t *row_bound, bool measure);
 
 }  // namespace cm
 

@@ -71,6 +71,9 @@ struct LevelArgs {
   unsigned *bar;             // barrier arrivals
   FusedLevel *out;           // [kMaxFused]
   int *result;               // [0] levels produced, [1] 1 if the stop rule ended the coarsening
+  // First level not measured yet: take the sum of its weights and its longest row
+  // into result[2..5] and, with derive_cap, the weight limit from them.
+  int measure, derive_cap;
   int coarsen_to, max_levels;
   double shrink;
 };
@@ -181,6 +184,25 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
     used += (ints + 63) & ~63ll;
     return at;
   };
+  if (A.measure) {
+    unsigned long long *stats = reinterpret_cast<unsigned long long *>(A.result + 2), sum = 0ull, longest = 0ull;
+    for (int v = blockIdx.x * kLvThreads + threadIdx.x; v < n; v += gridDim.x * kLvThreads) {
+      sum += (unsigned long long)(long long)vwgt[v];
+      longest = max(longest, (unsigned long long)(unsigned)(xadj[v + 1] - xadj[v]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    }
+    if (lane == 0) {
+      atomicAdd(stats, sum);
+      atomicMax(stats + 1, longest);
+    }
+    if (!level_barrier(A.bar, target, gridDim.x, st)) return;
+    if (__ldcg(stats + 1) > kMatchChunk) return;  // the separate kernels' graph
+    if (A.derive_cap) a.maxvwgt = (int)(1.5 * (double)(long long)__ldcg(stats) / A.coarsen_to);
+  }
   for (int level = 0;; ++level) {
     const int nb = min((int)gridDim.x, 1 + (n + m) / kLvWork);
     if ((int)blockIdx.x >= nb) return;
@@ -388,7 +410,7 @@ bool fused_fits(const cm_ctx *ctx, int64_t n, int64_t m, int64_t max_deg, int32_
 }
 
 int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaStream_t s, int *produced, int *stopped,
-                 int64_t *row_bound) {
+                 int64_t *row_bound, bool measure) {
   static_assert(kFusedWork <= 1 << kCountBits, "packed scan");
   *produced = 0;
   *stopped = 0;
@@ -457,6 +479,8 @@ int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaS
   A.cmap0 = F.cmap;
   A.arena = (int *)slab->ptr;
   A.arena_ints = arena_ints;
+  A.measure = measure;
+  A.derive_cap = measure && p->maxvwgt <= 0;
   A.coarsen_to = p->coarsen_to;
   A.max_levels = p->max_levels - ((int)h->levels.size() - 1);
   A.shrink = p->shrink;
@@ -479,6 +503,12 @@ int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaS
   }
   *produced = r->result[0];
   *stopped = r->result[1];
+  if (measure) {
+    long long stats[2];
+    memcpy(stats, r->result + 2, sizeof stats);
+    if (p->maxvwgt <= 0) h->maxvwgt = (int32_t)(1.5 * (double)stats[0] / p->coarsen_to);
+    *row_bound = 2 * stats[1];
+  }
   if (*produced > 0) h->slabs.push_back(slab);
   for (int i = 0; i < *produced; ++i) {
     const FusedLevel &o = r->level[i];

@@ -402,7 +402,8 @@ k_sort_scatter(const int *__restrict__ d_nb, const int *__restrict__ bnd_v, cons
 //
 // A walk vertex by vertex waits for several memory trips each (10.7 ms a phase
 // for an R-MAT 17 bisection, 0.49 ms for a 1000 x 1000 grid in 64 parts; a whole
-// pass went from 17.4 to 0.53 ms and from 0.86 to 0.26 ms), although most
+// pass went from 17.4 to 0.53 ms and from 0.86 to 0.26 ms; with the boundary test
+// by row length it takes 0.28 and 0.13), although most
 // stretches of a group are moved or refused as a whole.  So the block takes
 // kMoveThreads records at a time and settles them together when it can:
 //   - everyone moves: the weights leave their parts by atomics that return what

@@ -141,6 +141,10 @@ __global__ void __launch_bounds__(256) k_copy_arrays(const __grid_constant__ Cop
 // One kernel for the arrays of many graphs: a copy call from pageable memory
 // costs 9 to 12 us however small, and the four arrays of each of 64 graphs took
 // 3.85 ms.  Large arrays move as fast either way (190 to 200 GB/s).
+// Large pinned arrays stay with the copy engines, which leave the SMs to other
+// contexts: four contexts that coarsen R-MAT 22 from pinned memory in turn take 6.7
+// to 8.2 ms a step, with the kernel 10.6 to 11.4 (one context alone 15.1 either way).
+constexpr size_t kPinnedCopyBytes = 1 << 20;
 int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s) {
   for (int i = 0; i < count; ++i)
     if (a[i].bytes && !a[i].src) return cm_fail(CM_ERR_CUDA, "upload: null host array");
@@ -161,6 +165,16 @@ int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s) {
   };
   for (int i = 0; i < count; ++i) {
     if (a[i].bytes == 0) continue;
+    bool copy = ((size_t)a[i].src & 3) != 0;  // the kernel moves whole words
+    if (!copy && a[i].bytes >= kPinnedCopyBytes) {
+      cudaPointerAttributes at{};
+      if (cudaPointerGetAttributes(&at, a[i].src) != cudaSuccess) cudaGetLastError();
+      else copy = at.type == cudaMemoryTypeHost;
+    }
+    if (copy) {
+      cudaMemcpyAsync(a[i].dst, a[i].src, a[i].bytes, cudaMemcpyHostToDevice, s);
+      continue;
+    }
     const volatile char *c = (const volatile char *)a[i].src;
     (void)c[0];  // a bad address fails here, on the host
     (void)c[a[i].bytes - 1];
@@ -180,7 +194,8 @@ int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s) {
 // never touched before: 17 to 1007 instead of 41 to 1864), the coarsest graphs of a
 // batch of 64 in 1.2 ms instead of 2.65.  The host writes a word of every page
 // first: a bad address fails there, and the kernel meets mapped pages only.  Larger
-// levels, not measured, and memory that is not the host's stay with the copy calls.
+// levels (not measured), large pinned arrays (kPinnedCopyBytes) and memory that is
+// not the host's or not on a word boundary stay with the copy calls.
 constexpr size_t kDirectBytes = 32 << 20;
 int download_arrays(const cm_hierarchy *h, const HostArray *a, int count, const char *what) {
   cudaStream_t s = h->stream;
@@ -190,13 +205,13 @@ int download_arrays(const cm_hierarchy *h, const HostArray *a, int count, const 
   for (int i = 0; i < count && direct; ++i) {  // host memory, at its own address (a copy call refuses the rest)
     cudaPointerAttributes at{};
     if (a[i].bytes == 0) continue;
-    if (!a[i].dst || cudaPointerGetAttributes(&at, a[i].dst) != cudaSuccess) {
+    if (!a[i].dst || ((size_t)a[i].dst & 3) || cudaPointerGetAttributes(&at, a[i].dst) != cudaSuccess) {
       cudaGetLastError();
       direct = false;
       break;
     }
     direct = (at.type == cudaMemoryTypeUnregistered ||
-              (at.type == cudaMemoryTypeHost && at.devicePointer == a[i].dst));
+              (at.type == cudaMemoryTypeHost && at.devicePointer == a[i].dst && a[i].bytes < kPinnedCopyBytes));
   }
   if (!direct) {
     for (int i = 0; i < count; ++i)

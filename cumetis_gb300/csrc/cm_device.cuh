@@ -49,6 +49,20 @@ __device__ __forceinline__ int ld_relaxed(const int *p) {
   asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+// Reads of words that other warps change while this kernel runs.  Volatile: each
+// one is made where it stands, and again on every turn of a loop (the __ldcg
+// intrinsics promise neither).
+__device__ __forceinline__ unsigned ld_fresh(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int ld_fresh(const int *p) { return (int)ld_fresh(reinterpret_cast<const unsigned *>(p)); }
+__device__ __forceinline__ unsigned long long ld_fresh(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -64,6 +78,11 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
 }
 __device__ __forceinline__ void st_release64(unsigned long long *p, unsigned long long v) {
   asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Whether a kernel has recorded an error, one answer for the calling warp.
+__device__ __forceinline__ bool warp_sees_error(const DevStatus *st) {
+  return __shfl_sync(0xffffffffu, ld_relaxed(&st->error), 0) != 0;
 }
 
 // Grid-wide barrier for kernels launched cooperatively (all blocks resident).

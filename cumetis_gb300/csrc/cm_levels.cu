@@ -241,17 +241,18 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
     // ---- proposals
     for (int b0 = gw * 32; b0 < n; b0 += nw * 32) {
       int nq = 0;
-      propose_span<H, true, 8>(a, b0, 32, false, S.prop.list, [&](int v, int, int) {
+      bool ok = propose_span<H, true, 8>(a, b0, 32, false, S.prop.list, [&](int v, int, int) {
         const unsigned q = __ballot_sync(0xffffffffu, v >= 0);
         if (v >= 0) S.prop.queue[nq + __popc(q & below)] = v;
         nq += __popc(q);
       });
       __syncwarp();
-      for (int i = 0; i < nq; ++i) {
+      for (int i = 0; i < nq && ok; ++i) {
         const int v = S.prop.queue[i];
-        warp_chain<H>(a, v, xadj[v], xadj[v + 1], false, TopK<H, kTop>(), false, 0, 0, S.prop.wbuf);
+        ok = warp_chain<H>(a, v, xadj[v], xadj[v + 1], false, TopK<H, kTop>(), false, 0, 0, S.prop.wbuf);
       }
       __syncwarp();
+      if (!ok || (b0 + nw * 32 < n && warp_sees_error(st))) break;  // the barrier sees the error
     }
     if (!level_barrier(A.bar, target, nb, st)) return;
 

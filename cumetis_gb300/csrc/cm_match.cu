@@ -188,10 +188,12 @@ __global__ void __launch_bounds__(kPrepThreads, H ? 5 : 0) k_match_propose(Match
   const int gwarp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
   const int nwarps = (int)(((long long)gridDim.x * blockDim.x) >> 5);
   const int n = a.n;
-  for (long long b0 = (long long)gwarp * a.span; b0 < n; b0 += (long long)nwarps * a.span) {
-    propose_span<H, !H, H ? 4 : 8>(a, b0, a.span, all, list, [&](int v, int xs, int deg) {
+  const long long step = (long long)nwarps * a.span;
+  for (long long b0 = (long long)gwarp * a.span; b0 < n; b0 += step) {
+    const bool ok = propose_span<H, !H, H ? 4 : 8>(a, b0, a.span, all, list, [&](int v, int xs, int deg) {
       append_scan(a, 1, 1, v >= 0, v, xs, deg);
     });
+    if (!ok || (b0 + step < n && warp_sees_error(a.st))) return;
   }
 }
 
@@ -235,14 +237,18 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
       a.big[(round + 2) % 3] = 0;
       a.tick[(round + 2) % 3] = 0;
     }
-    // Chunks are taken from a ticket: rows and chains differ in length.
+    // Chunks are taken from a ticket: rows and chains differ in length.  No more
+    // once a kernel has failed.
     int q = 0;
     if (lane == 0) q = atomicAdd(a.tick + ctr, 1);
     q = __shfl_sync(0xffffffffu, q, 0);
     int4 d = q < nchunks ? __ldcg(S.desc + q) : make_int4(0, 0, 0, 0);
     while (q < nchunks) {
       int qn = 0;
-      if (lane == 0) qn = atomicAdd(a.tick + ctr, 1);
+      if (lane == 0) {
+        qn = atomicAdd(a.tick + ctr, 1);
+        if (ld_relaxed(&st->error) != 0) qn = INT_MAX;
+      }
       TopK<H, kTop> r;
       bool mine = true;
       if (d.w >= 0) {
@@ -256,7 +262,7 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
       }
       qn = __shfl_sync(0xffffffffu, qn, 0);
       const int4 dn = qn < nchunks ? __ldcg(S.desc + qn) : d;
-      if (mine) warp_chain<H>(a, d.x, d.y, d.z, d.w >= 0, r, all, par ^ 1, next, wbuf);
+      if (mine && !warp_chain<H>(a, d.x, d.y, d.z, d.w >= 0, r, all, par ^ 1, next, wbuf)) break;
       q = qn;
       d = dn;
     }

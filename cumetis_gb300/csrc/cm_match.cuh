@@ -176,7 +176,7 @@ __device__ __forceinline__ unsigned long long best_key(int v, int w) {
   return ((unsigned long long)((unsigned)w ^ 0x80000000u) << 32) | (unsigned)~(unsigned)v;
 }
 __device__ __forceinline__ int best_holder(unsigned long long b) { return b == 0ull ? -1 : (int)~(unsigned)b; }
-__device__ __forceinline__ unsigned long long ld_best(const MatchArgs &a, int k) { return __ldcg(a.best + k); }
+__device__ __forceinline__ unsigned long long ld_best(const MatchArgs &a, int k) { return ld_fresh(a.best + k); }
 
 // v's proposal (key) to c beats the proposal b that c holds.
 template <bool H>
@@ -288,7 +288,7 @@ __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, i
     unsigned bw[U];  // the weight half of best[]; 0 for none
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      bw[u] = (u < nu && k[u] >= 0) ? __ldcg(reinterpret_cast<const unsigned *>(a.best + k[u]) + 1) : 0u;
+      bw[u] = (u < nu && k[u] >= 0) ? ld_fresh(reinterpret_cast<const unsigned *>(a.best + k[u]) + 1) : 0u;
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (((unsigned)w[u] ^ 0x80000000u) < bw[u]) k[u] = -1;
@@ -636,7 +636,7 @@ __device__ __forceinline__ void short_list(const MatchArgs &a, int v, int xs, in
 template <bool H, int AHEAD>
 __device__ __forceinline__ int rescan_short(const MatchArgs &a, int v, int xs, int deg, bool all, int hb, int *weight,
                                             unsigned long long *seen) {
-    constexpr int kHalf = AHEAD;
+  constexpr int kHalf = AHEAD;
   const long long vw = all ? 0 : a.vwgt[v], cap = all ? 0 : weight_cap(a, v);
   TopK<H, 1> t1;
   *seen = 0ull;
@@ -683,8 +683,9 @@ __device__ __forceinline__ int rescan_short(const MatchArgs &a, int v, int xs, i
 // offer is under way: it pays where chains are long (low-id ties on a 700 x 700
 // triangulation 3.21 -> 2.95 ms), and costs reads and registers where the chip is
 // full (hashed ties, R-MAT 22: +0.08 ms).  SCAN: entries of a rescan in flight.
+// False after an overrun.
 template <bool H, bool AHEAD, int SCAN, typename Q>
-__device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, int span, bool all, int *list, Q queue) {
+__device__ __forceinline__ bool propose_span(const MatchArgs &a, long long b0, int span, bool all, int *list, Q queue) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int n = a.n;
@@ -701,7 +702,7 @@ __device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, i
   List L;
   uint64_t since = 0;
   for (unsigned turn = 0;; ++turn) {
-    if (chain_overrun(a, turn, since)) break;
+    if (chain_overrun(a, turn, since)) return false;
     const unsigned idle = __ballot_sync(0xffffffffu, cur < 0);
     if (taken < cnt && idle) {
       const int at = taken + __popc(idle & below);
@@ -746,6 +747,7 @@ __device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, i
     queue(qv, qx, qdeg);
   }
   __syncwarp();  // the list is free for the next span
+  return true;
 }
 
 // A warp's chain, starting with v (free): its row is scanned, or `r` holds the
@@ -754,58 +756,91 @@ __device__ __forceinline__ void propose_span(const MatchArgs &a, long long b0, i
 // with its neighbour's proposal costs more than the scan -- and only when all
 // the candidates so found turn out to be refused is the row scanned again with
 // the full test.  A free vertex whose row has several chunks is queued for the
-// next round (slot par, counter ctr).  Convergent.
+// next round (slot par, counter ctr).  Convergent; false after an overrun.
+//
+// The candidates lie in the lanes: lane t < kTop holds the t-th, reads the proposal
+// that this neighbour holds and compares.  best[] changes while the warp looks at
+// it, so every decision comes from a ballot or a shuffle: lanes that each read
+// best[] for themselves can see different proposals, take different branches and
+// wait for one another in the scans' collectives for good.
 template <bool H>
-__device__ __forceinline__ void warp_chain(const MatchArgs &a, int v, int xs, int xe, bool scanned,
+__device__ __forceinline__ bool warp_chain(const MatchArgs &a, int v, int xs, int xe, bool scanned,
                                            const TopK<H, kTop> &r, bool all, int par, int ctr, int2 *wbuf) {
+  constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int hb = hash_base(a, v);
   int cur = v;
-  List L;
-  auto take = [&](const TopK<H, kTop> &t) {  // the scan's candidates as a list
+  int id = kUnknown, w = 0, from = kTop;  // this lane's candidate; lanes before `from` are done with
+  unsigned long long seen = 0ull;         // the proposal it holds
+  auto take = [&](const TopK<H, kTop> &t) {  // a scan's candidates
 #pragma unroll
-    for (int i = 0; i < kTop; ++i) {
-      L.id[i] = t.c[i].id();
-      L.w[i] = t.c[i].weight();
-    }
-    L.check<H>(a, cur, hb);
+    for (int i = 0; i < kTop; ++i)
+      if (lane == i) {
+        id = t.c[i].id();
+        w = t.c[i].weight();
+      }
+    from = 0;
+  };
+  // The lane of the first candidate that would take cur; kNone: there is none,
+  // kUnknown: the list is used up.
+  auto next = [&]() -> int {
+    const bool live = lane >= from && lane < kTop, cand = live && id >= 0;
+    seen = cand ? ld_best(a, id) : 0ull;
+    const unsigned yes = __ballot_sync(full, cand && beats<H>(best_key(cur, w), seen, cur, id, hb));
+    const unsigned end = __ballot_sync(full, live && id < 0);  // nothing behind the first of these
+    const int y = yes ? __ffs(yes) - 1 : kTop, e = end ? __ffs(end) - 1 : kTop;
+    if (y < e) return y;
+    return e < kTop && __shfl_sync(full, id, e) == kNone ? kNone : kUnknown;
   };
   if (scanned) take(r);
-  else L.id[0] = kUnknown;
   uint64_t since = 0;
   for (unsigned turn = 0;; ++turn) {
-    if (chain_overrun(a, turn, since)) return;
-    if (L.id[0] == kUnknown) {
+    if (chain_overrun(a, turn, since)) return false;
+    int at = next();
+    if (at == kUnknown) {
       if (cur != v || scanned) {
         xs = a.xadj[cur];
         xe = a.xadj[cur + 1];
       }
       if (xe - xs > kMatchChunk) {
         append_scan(a, par, ctr, lane == 0, cur, xs, xe - xs);
-        return;
+        return true;
       }
-      if constexpr (H) take(chunk_best<H, kTop, kWeak>(a, cur, xs, xe, all, wbuf));
-      if (!H || L.id[0] == kUnknown) take(chunk_best<H, kTop, kExact>(a, cur, xs, xe, all, wbuf));
+      if constexpr (H) {
+        take(chunk_best<H, kTop, kWeak>(a, cur, xs, xe, all, wbuf));
+        at = next();
+      }
+      if (!H || at == kUnknown) {
+        take(chunk_best<H, kTop, kExact>(a, cur, xs, xe, all, wbuf));
+        at = next();
+      }
+      if (at == kUnknown) {  // others took all of them meanwhile
+        from = kTop;
+        continue;
+      }
     }
-    const int c = L.id[0];
-    if (c == kNone) return;
-    if (c == kUnknown) continue;  // others took all of them meanwhile
+    if (at == kNone) return true;
+    const int c = __shfl_sync(full, id, at);
     int res = -2;  // -2: refused, else the vertex given up (-1: none)
-    if (lane == 0) {
+    if (lane == at) {
       int out = -1;
-      if (offer<H>(a, cur, c, L.w[0], L.seen[0], hb, &out)) res = out;
+      if (offer<H>(a, cur, id, w, seen, hb, &out)) res = out;
     }
-    res = __shfl_sync(0xffffffffu, res, 0);
+    res = __shfl_sync(full, res, at);
     if (res == -2) {
-      L.drop();
-    } else {
-      if (res < 0) return;
-      cur = res;
-      L.load(a, cur);
-      L.after(c);
-      scanned = true;  // xs, xe are another row's
+      from = at + 1;
+      continue;
     }
-    L.check<H>(a, cur, hb);
+    if (res < 0) return true;
+    cur = res;
+    scanned = true;  // xs, xe are another row's
+    if (lane < kTop) {
+      id = a.top[(size_t)cur * kTop + lane];
+      w = a.topw[(size_t)cur * kTop + lane];
+    }
+    // go on behind c; when c is not listed it came from a rescan, and the list is used up
+    const unsigned listed = __ballot_sync(full, lane < kTop && id == c);
+    from = listed ? __ffs(listed) : kTop;
   }
 }
 

@@ -166,7 +166,7 @@ __device__ __forceinline__ unsigned long long lookback_resolve(unsigned long lon
     const unsigned inc_mask = __ballot_sync(0xffffffffu, flag == 2);
     const int last = inc_mask ? (__ffs(inc_mask) - 1) : 31;
     if (__any_sync(0xffffffffu, lane <= last && flag == 0)) {
-      if (global_timer_ns() - t0 > kWaitLimitNs) {
+      if (__shfl_sync(0xffffffffu, global_timer_ns() - t0 > kWaitLimitNs, 0)) {  // one answer for the warp
         if (lane == 0) record_error(st, CM_ERR_LIMIT, ERR_SITE_LOOKBACK);
         excl = 0;
         break;

@@ -24,8 +24,8 @@
 //
 // What the kernel does not handle ends it before that level -- rows of more
 // than kMaxRow expanded or kMatchChunk fine entries, an adjacency that is not
-// symmetric, an allocation that turns out too small -- and the caller does the
-// level with the separate kernels.
+// symmetric, a very long chain, an allocation that turns out too small -- and the
+// caller does the level with the separate kernels.
 #include <algorithm>
 
 #include "cm_ctx.h"
@@ -45,6 +45,10 @@ constexpr int kLvThreads = 512, kLvWarps = kLvThreads / 32;
 #endif
 constexpr int kLvWork = CM_LEVEL_WORK;
 constexpr int kLvItems = 8, kMaxRow = 32 * kLvItems;  // longest expanded row: one warp sorts it
+// Turns of a warp's chains in one level: about 0.3 s, while the other blocks wait at
+// a barrier.  A level with a longer chain is left to the separate kernels, where
+// nobody waits for it.
+constexpr unsigned kFusedSteps = 1u << 18;
 constexpr int kMaxFused = 64;                         // levels of one launch
 constexpr int kCountBits = 21;                        // vertices and entries stay below 2^21 (packed scan)
 static_assert(kTinyMax < kMaxRow, "row lengths");
@@ -239,20 +243,23 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
     if (__ldcg(flags) != 0) return;
 
     // ---- proposals
+    unsigned steps = kFusedSteps;
     for (int b0 = gw * 32; b0 < n; b0 += nw * 32) {
       int nq = 0;
-      bool ok = propose_span<H, true, 8>(a, b0, 32, false, S.prop.list, [&](int v, int, int) {
+      ChainEnd end = propose_span<H, true, 8, true>(a, b0, 32, false, S.prop.list, &steps, [&](int v, int, int) {
         const unsigned q = __ballot_sync(0xffffffffu, v >= 0);
         if (v >= 0) S.prop.queue[nq + __popc(q & below)] = v;
         nq += __popc(q);
       });
       __syncwarp();
-      for (int i = 0; i < nq && ok; ++i) {
+      for (int i = 0; i < nq && end == kChainDone; ++i) {
         const int v = S.prop.queue[i];
-        ok = warp_chain<H>(a, v, xadj[v], xadj[v + 1], false, TopK<H, kTop>(), false, 0, 0, S.prop.wbuf);
+        end = warp_chain<H, kGiveUp>(a, v, xadj[v], xadj[v + 1], false, TopK<H, kTop>(), false, 0, 0, &steps,
+                                     S.prop.wbuf);
       }
       __syncwarp();
-      if (!ok || (b0 + nw * 32 < n && warp_sees_error(st))) break;  // the barrier sees the error
+      if (end == kChainLong) unfit = true;  // the level is given up behind the partners
+      if (end != kChainDone || (b0 + nw * 32 < n && warp_sees_error(st))) break;  // (a barrier sees errors)
     }
     if (!level_barrier(A.bar, target, nb, st)) return;
 

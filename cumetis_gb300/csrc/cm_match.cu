@@ -35,7 +35,7 @@
 //                    warp following the chain; rows of several chunks are merged
 //                    by the last chunk's warp, and a displaced one is queued for
 //                    the next round (grid barrier; a round with few chunks runs
-//                    on one block).
+//                    on one block), as is the free vertex of a long chain.
 //   k_match_finish   match[v] = the partner, or v.
 //
 // Only an adjacency that is not symmetric can end with an offer that is not
@@ -190,10 +190,11 @@ __global__ void __launch_bounds__(kPrepThreads, H ? 5 : 0) k_match_propose(Match
   const int n = a.n;
   const long long step = (long long)nwarps * a.span;
   for (long long b0 = (long long)gwarp * a.span; b0 < n; b0 += step) {
-    const bool ok = propose_span<H, !H, H ? 4 : 8>(a, b0, a.span, all, list, [&](int v, int xs, int deg) {
-      append_scan(a, 1, 1, v >= 0, v, xs, deg);
-    });
-    if (!ok || (b0 + step < n && warp_sees_error(a.st))) return;
+    const ChainEnd end =
+        propose_span<H, !H, H ? 4 : 8, false>(a, b0, a.span, all, list, nullptr, [&](int v, int xs, int deg) {
+          append_scan(a, 1, 1, v >= 0, v, xs, deg);
+        });
+    if (end != kChainDone || (b0 + step < n && warp_sees_error(a.st))) return;
   }
 }
 
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
     if (lane == 0) q = atomicAdd(a.tick + ctr, 1);
     q = __shfl_sync(0xffffffffu, q, 0);
     int4 d = q < nchunks ? __ldcg(S.desc + q) : make_int4(0, 0, 0, 0);
+    unsigned steps = kChainSteps;  // of this warp in this round
     while (q < nchunks) {
       int qn = 0;
       if (lane == 0) {
@@ -262,7 +264,9 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
       }
       qn = __shfl_sync(0xffffffffu, qn, 0);
       const int4 dn = qn < nchunks ? __ldcg(S.desc + qn) : d;
-      if (mine && !warp_chain<H>(a, d.x, d.y, d.z, d.w >= 0, r, all, par ^ 1, next, wbuf)) break;
+      if (mine && warp_chain<H, ONE_PASS ? kEndless : kQueue>(a, d.x, d.y, d.z, d.w >= 0, r, all, par ^ 1, next,
+                                                              &steps, wbuf) != kChainDone)
+        break;
       q = qn;
       d = dn;
     }

@@ -306,17 +306,28 @@ __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, i
     if (k[u] == v) k[u] = -1;
 }
 
-// Chains end by themselves (every step improves some best[]); a limit all the
-// same: true, with CM_ERR_LIMIT recorded, once a warp's loop has run past the
-// wait limit (looked at every 65536 turns).
-__device__ __forceinline__ bool chain_overrun(const MatchArgs &a, unsigned turn, uint64_t &since) {
-  if ((turn & 0xffffu) != 0xffffu) return false;
-  const uint64_t now = __shfl_sync(0xffffffffu, global_timer_ns(), 0);  // one answer for the warp
-  if (since == 0) since = now;
-  if (now - since <= kWaitLimitNs) return false;
-  if ((threadIdx.x & 31) == 0) record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
-  return true;
-}
+// How a chain, or a span's chains, ended.
+enum ChainEnd : int {
+  kChainDone = 0,
+  kChainFailed = 1,  // CM_ERR_LIMIT recorded
+  kChainLong = 2,    // the steps allowed are used up (k_levels)
+};
+
+// Chains end by themselves: every accepted offer improves some best[], at most once
+// for every entry of the graph.  A path whose weights grow from one end to the other
+// makes one chain of n / 2 dependent steps (8 M vertices: 3 s), so a chain has no
+// limit on its length.  What could only be a fault has one: a refusal means that
+// the neighbour holds a better proposal for good, so a vertex is refused at most
+// once per entry of its row before it is taken or has no candidate left.
+constexpr int kLaneRefusals = kSerialDeg + kTop, kWarpRefusals = kMatchChunk + kTop;
+
+// Where other warps wait for a chain at a grid barrier, whose wait has a limit, a
+// warp takes at most kChainSteps accepted offers a round (about 0.1 s) and queues
+// the vertex that is free then for the next round.
+#ifndef CM_CHAIN_STEPS
+#define CM_CHAIN_STEPS 65536
+#endif
+constexpr unsigned kChainSteps = CM_CHAIN_STEPS;
 
 // The warp's best KK candidates over entries [b, e), e - b <= 64, of v's row,
 // with FILTER among those that v beats the proposal of; every lane gets the list.
@@ -563,8 +574,8 @@ __device__ __forceinline__ void write_descs(int4 *desc, bool take, int x, int xs
   }
 }
 
-// Queues x (row of deg > kSerialDeg entries starting at xs) for a scan: slot
-// `par`, counter `ctr`; convergent.
+// Queues x (row of deg > 0 entries starting at xs) for a scan: slot `par`,
+// counter `ctr`; convergent.
 __device__ __forceinline__ void append_scan(const MatchArgs &a, int par, int ctr, bool take, int x, int xs, int deg) {
   if (!__any_sync(0xffffffffu, take)) return;
   const Slot &S = a.slot[par];
@@ -683,9 +694,11 @@ __device__ __forceinline__ int rescan_short(const MatchArgs &a, int v, int xs, i
 // offer is under way: it pays where chains are long (low-id ties on a 700 x 700
 // triangulation 3.21 -> 2.95 ms), and costs reads and registers where the chip is
 // full (hashed ties, R-MAT 22: +0.08 ms).  SCAN: entries of a rescan in flight.
-// False after an overrun.
-template <bool H, bool AHEAD, int SCAN, typename Q>
-__device__ __forceinline__ bool propose_span(const MatchArgs &a, long long b0, int span, bool all, int *list, Q queue) {
+// BOUNDED: every turn takes one of *steps, and without any left the warp gives up
+// (kChainLong).
+template <bool H, bool AHEAD, int SCAN, bool BOUNDED, typename Q>
+__device__ __forceinline__ ChainEnd propose_span(const MatchArgs &a, long long b0, int span, bool all, int *list,
+                                                 unsigned *steps, Q queue) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int n = a.n;
@@ -700,9 +713,13 @@ __device__ __forceinline__ bool propose_span(const MatchArgs &a, long long b0, i
   __syncwarp();
   int cur = -1, hb = 0;
   List L;
-  uint64_t since = 0;
-  for (unsigned turn = 0;; ++turn) {
-    if (chain_overrun(a, turn, since)) return false;
+  int refused = 0;  // offers of cur in a row
+  bool failed = false;
+  for (;;) {
+    if (BOUNDED) {
+      if (*steps == 0) return kChainLong;
+      --*steps;
+    }
     const unsigned idle = __ballot_sync(0xffffffffu, cur < 0);
     if (taken < cnt && idle) {
       const int at = taken + __popc(idle & below);
@@ -728,6 +745,7 @@ __device__ __forceinline__ bool propose_span(const MatchArgs &a, long long b0, i
       }
       if (c < 0) {  // queued, or no candidate is left
         cur = -1;
+        refused = 0;
       } else {
         int out = -1;
         const int guess = AHEAD ? best_holder(held) : -1;
@@ -735,19 +753,24 @@ __device__ __forceinline__ bool propose_span(const MatchArgs &a, long long b0, i
         if (AHEAD && guess >= 0) N.load(a, guess);
         if (offer<H>(a, cur, c, w, held, hb, &out)) {
           cur = out;
+          refused = 0;
           if (cur >= 0) {
             if (AHEAD && cur == guess) L = N;
             else L.load(a, cur);
             L.after(c);
           }
-        }  // refused: c holds a better proposal now, which the next check sees
+        } else if (++refused > kLaneRefusals) {  // c holds a better proposal now, which the next check sees
+          record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
+          failed = true;
+          cur = -1;
+        }
       }
     }
     __syncwarp();
     queue(qv, qx, qdeg);
   }
-  __syncwarp();  // the list is free for the next span
-  return true;
+  // (the list is free for the next span)
+  return __any_sync(0xffffffffu, failed) ? kChainFailed : kChainDone;
 }
 
 // A warp's chain, starting with v (free): its row is scanned, or `r` holds the
@@ -756,16 +779,20 @@ __device__ __forceinline__ bool propose_span(const MatchArgs &a, long long b0, i
 // with its neighbour's proposal costs more than the scan -- and only when all
 // the candidates so found turn out to be refused is the row scanned again with
 // the full test.  A free vertex whose row has several chunks is queued for the
-// next round (slot par, counter ctr).  Convergent; false after an overrun.
+// next round (slot par, counter ctr).  Every accepted offer takes one of *steps;
+// without any left the free vertex is queued too (kQueue) or the warp gives up
+// (kGiveUp: kChainLong).  Convergent.
 //
 // The candidates lie in the lanes: lane t < kTop holds the t-th, reads the proposal
 // that this neighbour holds and compares.  best[] changes while the warp looks at
 // it, so every decision comes from a ballot or a shuffle: lanes that each read
 // best[] for themselves can see different proposals, take different branches and
 // wait for one another in the scans' collectives for good.
-template <bool H>
-__device__ __forceinline__ bool warp_chain(const MatchArgs &a, int v, int xs, int xe, bool scanned,
-                                           const TopK<H, kTop> &r, bool all, int par, int ctr, int2 *wbuf) {
+enum : int { kEndless = 0, kQueue = 1, kGiveUp = 2 };
+template <bool H, int LIMIT>
+__device__ __forceinline__ ChainEnd warp_chain(const MatchArgs &a, int v, int xs, int xe, bool scanned,
+                                               const TopK<H, kTop> &r, bool all, int par, int ctr, unsigned *steps,
+                                               int2 *wbuf) {
   constexpr unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int hb = hash_base(a, v);
@@ -793,9 +820,11 @@ __device__ __forceinline__ bool warp_chain(const MatchArgs &a, int v, int xs, in
     return e < kTop && __shfl_sync(full, id, e) == kNone ? kNone : kUnknown;
   };
   if (scanned) take(r);
-  uint64_t since = 0;
-  for (unsigned turn = 0;; ++turn) {
-    if (chain_overrun(a, turn, since)) return false;
+  for (int refused = 0;;) {  // offers and scans of cur in a row that came to nothing
+    if (refused > kWarpRefusals) {
+      if (lane == 0) record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
+      return kChainFailed;
+    }
     int at = next();
     if (at == kUnknown) {
       if (cur != v || scanned) {
@@ -804,7 +833,7 @@ __device__ __forceinline__ bool warp_chain(const MatchArgs &a, int v, int xs, in
       }
       if (xe - xs > kMatchChunk) {
         append_scan(a, par, ctr, lane == 0, cur, xs, xe - xs);
-        return true;
+        return kChainDone;
       }
       if constexpr (H) {
         take(chunk_best<H, kTop, kWeak>(a, cur, xs, xe, all, wbuf));
@@ -816,10 +845,11 @@ __device__ __forceinline__ bool warp_chain(const MatchArgs &a, int v, int xs, in
       }
       if (at == kUnknown) {  // others took all of them meanwhile
         from = kTop;
+        ++refused;
         continue;
       }
     }
-    if (at == kNone) return true;
+    if (at == kNone) return kChainDone;
     const int c = __shfl_sync(full, id, at);
     int res = -2;  // -2: refused, else the vertex given up (-1: none)
     if (lane == at) {
@@ -829,11 +859,20 @@ __device__ __forceinline__ bool warp_chain(const MatchArgs &a, int v, int xs, in
     res = __shfl_sync(full, res, at);
     if (res == -2) {
       from = at + 1;
+      ++refused;
       continue;
     }
-    if (res < 0) return true;
+    if (res < 0) return kChainDone;
     cur = res;
+    refused = 0;
     scanned = true;  // xs, xe are another row's
+    if (LIMIT != kEndless && *steps > 0) --*steps;
+    if (LIMIT != kEndless && *steps == 0) {
+      if (LIMIT == kGiveUp) return kChainLong;
+      xs = a.xadj[cur];
+      append_scan(a, par, ctr, lane == 0, cur, xs, a.xadj[cur + 1] - xs);
+      return kChainDone;
+    }
     if (lane < kTop) {
       id = a.top[(size_t)cur * kTop + lane];
       w = a.topw[(size_t)cur * kTop + lane];

@@ -285,52 +285,147 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
   trace(0, 4, (unsigned long long)(round - 1));
 }
 
-// The matching of an adjacency that is not symmetric: mutual proposals in
-// rounds until no pair forms.  Every unmatched vertex points at its most
-// preferred unmatched neighbour (ptr), and vertices that point at each other
-// are matched.  One warp a vertex, over the warps gw, gw + nw, ...; barrier()
-// separates the phases and returns false to give up.  Reads and writes of
-// other warps' vertices go to L2.
+// The matching of an adjacency that is not symmetric: mutual proposals until no
+// pair forms.  Every unmatched vertex points at its most preferred unmatched
+// neighbour, and vertices that point at each other are matched; whichever pairs
+// are matched first, the outcome is the same.  Rounds over a list of the vertices
+// that have to point anew (at first all), in three phases:
+//   point   the first unmatched of the vertex's listed candidates, or of its row;
+//   commit  the pairs;
+//   wake    neighbours that point at a vertex matched now go on the next list.
+// A vertex is woken through the matched one's row, so it can be missed where its own
+// entry has no counterpart: when the list is empty, one pass over all vertices
+// finds those.  The work is that of the rows looked at, not rounds times vertices:
+// a path in order takes n / 2 rounds of a few vertices each.  At most 2 n + 4
+// rounds: all but every second match a pair.
+// Over the warps gw, gw + nw, ...; barrier() separates the phases and returns false
+// to give up.  What other warps write is read fresh.
 template <bool H, typename B>
-__device__ void handshake_rounds(const MatchArgs &a, int *ptr, int *changed, int gw, int nw, B barrier) {
-  const int lane = threadIdx.x & 31;
-  const int n = a.n;
-  for (long long v = (long long)gw * 32 + lane; v < n; v += (long long)nw * 32) a.m2[v] = -1;
-  if (gw == 0 && lane == 0) changed[0] = changed[1] = changed[2] = 0;
-  if (!barrier()) return;
-  for (int round = 0;; ++round) {
-    if (gw == 0 && lane == 0) changed[(round + 1) % 3] = 0;
-    for (long long v = gw; v < n; v += nw) {
-      if (__ldcg(a.m2 + v) >= 0) continue;
-      const int hb = hash_base(a, (int)v);
-      const long long vw = a.vwgt[v], cap = weight_cap(a, (int)v);
-      Cand<H> c;
-      for (int j = a.xadj[v] + lane; j < a.xadj[v + 1]; j += 32) {
-        const int k = a.adjncy[j];
-        if (k == (int)v || __ldcg(a.m2 + k) >= 0 || !pair_fits(cap, vw, a.vwgt[k])) continue;
-        const Cand<H> x = Cand<H>::make((int)v, k, a.adjwgt[j], hb);
-        if (x.better(c)) c = x;
-      }
-      const int p = c.warp_best().id();
-      if (lane == 0) ptr[v] = p;
-    }
-    if (!barrier()) return;
-    bool any = false;
-    for (long long v = (long long)gw * 32 + lane; v < n; v += (long long)nw * 32) {
-      if (__ldcg(a.m2 + v) >= 0) continue;
-      const int p = __ldcg(ptr + v);
-      if (p > (int)v && __ldcg(ptr + p) == (int)v) {  // the lower end commits both
-        a.m2[v] = p;
-        a.m2[p] = (int)v;
-        any = true;
-      }
-    }
-    if (any) changed[round % 3] = 1;
-    if (!barrier()) return;
-    if (__ldcg(changed + round % 3) == 0) break;
+__device__ void handshake_rounds(const MatchArgs &a, int gw, int nw, B barrier) {
+  constexpr unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, n = a.n;
+  const unsigned below = (1u << lane) - 1u;
+  // the proposals' scratch is free: targets, the round of the last listing, the lists
+  int *ptr = a.slot[0].big_base, *stamp = a.slot[0].big_done, *count = a.odd + 2;  // count[3], by round
+  int *lists[2] = {reinterpret_cast<int *>(a.slot[0].desc), reinterpret_cast<int *>(a.slot[1].desc)};
+  const long long step = (long long)nw * 32;
+  for (long long v = (long long)gw * 32 + lane; v < n; v += step) {
+    a.m2[v] = -1;
+    ptr[v] = -1;
+    stamp[v] = 0;
+    lists[0][v] = (int)v;
   }
-  for (long long v = (long long)gw * 32 + lane; v < n; v += (long long)nw * 32)
-    if (a.m2[v] < 0) a.m2[v] = (int)v;
+  if (gw == 0 && lane == 0) {
+    count[0] = n;
+    count[1] = count[2] = 0;
+  }
+  if (!barrier()) return;
+  bool searched = false;  // the last round was a pass over all vertices
+  for (int round = 0;; ++round) {
+    const int k = ld_fresh(count + round % 3);
+    const int *list = lists[round & 1];
+    int *more = lists[~round & 1], *nmore = count + (round + 1) % 3;
+    if (gw == 0 && lane == 0) count[(round + 2) % 3] = 0;
+    if ((long long)round > 2ll * n + 4) {
+      if (gw == 0 && lane == 0) record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
+      return;
+    }
+    auto append = [&](bool take, int v) {  // convergent
+      const unsigned who = __ballot_sync(full, take);
+      if (!who) return;
+      int base = 0;
+      if (lane == 0) base = atomicAdd(nmore, __popc(who));
+      base = __shfl_sync(full, base, 0);
+      if (take) more[base + __popc(who & below)] = v;
+    };
+    if (k == 0) {
+      if (searched) break;
+      for (long long b = (long long)gw * 32; b < n; b += step) {
+        const long long v = b + lane;
+        bool stale = false;
+        if (v < n && ld_fresh(a.m2 + v) < 0) {
+          const int p = ld_fresh(ptr + v);
+          stale = p >= 0 && ld_fresh(a.m2 + p) >= 0;
+        }
+        if (stale) stamp[v] = round + 1;
+        append(stale, (int)v);
+      }
+      searched = true;
+      if (!barrier()) return;
+      continue;
+    }
+    searched = false;
+
+    // ---- point
+    for (long long b = (long long)gw * 32; b < k; b += step) {
+      const int v = b + lane < k ? ld_fresh(list + b + lane) : -1;
+      int p = kNone;
+      if (v >= 0 && a.xadj[v + 1] > a.xadj[v]) {
+        const int4 q = reinterpret_cast<const int4 *>(a.top)[v];
+        const int c[kTop] = {q.x, q.y, q.z, q.w};
+        p = kUnknown;
+#pragma unroll
+        for (int t = kTop - 1; t >= 0; --t) {
+          if (c[t] < 0) p = c[t];
+          else if (ld_fresh(a.m2 + c[t]) < 0) p = c[t];
+        }
+      }
+      unsigned rows = __ballot_sync(full, p == kUnknown);  // lists used up: the whole row
+      while (rows) {
+        const int src = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const int x = __shfl_sync(full, v, src), hb = hash_base(a, x);
+        const long long vw = a.vwgt[x], cap = weight_cap(a, x);
+        Cand<H> best;
+        for (int j = a.xadj[x] + lane; j < a.xadj[x + 1]; j += 32) {
+          const int y = a.adjncy[j];
+          if (y == x || ld_fresh(a.m2 + y) >= 0 || !pair_fits(cap, vw, a.vwgt[y])) continue;
+          const Cand<H> e = Cand<H>::make(x, y, a.adjwgt[j], hb);
+          if (e.better(best)) best = e;
+        }
+        const int id = best.warp_best().id();
+        if (lane == src) p = id;
+      }
+      if (v >= 0) ptr[v] = p;
+    }
+    if (!barrier()) return;
+
+    // ---- commit (by either end that is listed: the same words)
+    for (long long i = (long long)gw * 32 + lane; i < k; i += step) {
+      const int v = ld_fresh(list + i), p = ld_fresh(ptr + v);
+      if (p >= 0 && ld_fresh(ptr + p) == v) {
+        a.m2[v] = p;
+        a.m2[p] = v;
+      }
+    }
+    if (!barrier()) return;
+
+    // ---- wake
+    for (long long b = (long long)gw * 32; b < k; b += step) {
+      const int v = b + lane < k ? ld_fresh(list + b + lane) : -1;
+      const int u = v >= 0 ? ld_fresh(a.m2 + v) : -1;
+      const bool both = u >= 0 && ld_fresh(stamp + u) != round;  // u is not listed: its row is left to v
+      const unsigned other = __ballot_sync(full, both);
+      unsigned rows = __ballot_sync(full, u >= 0);
+      while (rows) {
+        const int src = __ffs(rows) - 1;
+        rows &= rows - 1;
+        for (int end = 0; end < 1 + (int)(other >> src & 1u); ++end) {
+          const int x = __shfl_sync(full, end ? u : v, src);
+          const int xe = a.xadj[x + 1];
+          for (int j0 = a.xadj[x]; j0 < xe; j0 += 32) {
+            const int y = j0 + lane < xe ? a.adjncy[j0 + lane] : -1;
+            const bool wake = y >= 0 && ld_fresh(ptr + y) == x && ld_fresh(a.m2 + y) < 0 &&
+                              atomicExch(stamp + y, round + 1) != round + 1;  // a row can name y twice
+            append(wake, y);
+          }
+        }
+      }
+    }
+    if (!barrier()) return;
+  }
+  for (long long v = (long long)gw * 32 + lane; v < n; v += step)
+    if (ld_fresh(a.m2 + v) < 0) a.m2[v] = (int)v;
 }
 
 // match[v] from best[]; a proposal that is not returned sets odd[0].  With
@@ -353,7 +448,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int 
   if (threadIdx.x == 0) s_last = atomicAdd(a.odd + 1, 1) == (int)gridDim.x - 1;
   __syncthreads();
   if (!s_last || __ldcg(a.odd) == 0) return;
-  handshake_rounds<H>(a, a.top, a.odd + 2, threadIdx.x >> 5, blockDim.x >> 5, [&] {
+  handshake_rounds<H>(a, threadIdx.x >> 5, blockDim.x >> 5, [&] {
     __threadfence();
     __syncthreads();
     return true;
@@ -364,8 +459,8 @@ __global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int 
 template <bool H>
 __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_handshake(MatchArgs a) {
   if (__ldcg(a.odd) == 0) return;
-  handshake_rounds<H>(a, a.top, a.odd + 2, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5),
-                      (int)((gridDim.x * blockDim.x) >> 5), [&] { return grid_barrier(a.st, gridDim.x); });
+  handshake_rounds<H>(a, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), (int)((gridDim.x * blockDim.x) >> 5),
+                      [&] { return grid_barrier(a.st, gridDim.x); });
 }
 
 // ---------------------------------------------------------------------------

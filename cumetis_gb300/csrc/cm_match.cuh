@@ -43,7 +43,7 @@ struct MatchArgs {
   unsigned long long *big;       // [3] = (rows << 32 | chunks) of the slots, by round
   int *tick;                     // [3] work tickets of the round kernel, by round
   int *vmax;                     // largest vertex weight (zeroed before the launch)
-  int *odd;                      // [2]: an offer was not returned; blocks of k_match_finish done
+  int *odd;                      // [5]: an offer was not returned; blocks of k_match_finish done; handshakes' list lengths
   int *part;                     // per chunk: kTop x (w, h, k)
   long long max_rounds;
   DevStatus *st;

@@ -269,8 +269,9 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
       unsigned long long sum = 0ull;
       int longest = 0;
       for (int v = r0 + (int)threadIdx.x; v < r1; v += kLvThreads) {
-        const int h = best_holder(ld_best(a, v));
-        const bool mutual = h >= 0 && best_holder(ld_best(a, h)) == v;
+        const unsigned long long b = ld_best(a, v);
+        const int h = best_holder(b);
+        const bool mutual = h >= 0 && best_mutual(b, ld_best(a, h), v);
         unfit |= h >= 0 && !mutual;
         const int u = mutual ? h : v;
         match[v] = u;

@@ -39,9 +39,10 @@
 //   k_match_finish   match[v] = the partner, or v.
 //
 // Only an adjacency that is not symmetric can end with an offer that is not
-// returned (best[u] = v, best[v] != u).  k_match_finish sees that and the
-// matching is then computed again by handshakes (handshake_rounds), whose
-// result is defined for such inputs too.
+// returned (best[u] = v, best[v] != u), or returned with another weight (the two
+// entries of an edge differ).  k_match_finish sees that and the matching is then
+// computed again by handshakes (handshake_rounds), whose result is defined for
+// such inputs too.
 #include <climits>
 
 #include <algorithm>
@@ -428,15 +429,16 @@ __device__ void handshake_rounds(const MatchArgs &a, int gw, int nw, B barrier) 
     if (ld_fresh(a.m2 + v) < 0) a.m2[v] = (int)v;
 }
 
-// match[v] from best[]; a proposal that is not returned sets odd[0].  With
+// match[v] from best[]; a proposal that is not returned alike sets odd[0].  With
 // `alone` the last block then computes the matching by handshakes itself.
 template <bool H>
 __global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int alone) {
   bool odd = false;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < a.n;
        v += (long long)gridDim.x * blockDim.x) {
-    const int h = best_holder(a.best[v]);
-    const bool mutual = h >= 0 && best_holder(a.best[h]) == (int)v;
+    const unsigned long long b = a.best[v];
+    const int h = best_holder(b);
+    const bool mutual = h >= 0 && best_mutual(b, a.best[h], (int)v);
     a.m2[v] = mutual ? h : (int)v;
     odd |= h >= 0 && !mutual;
   }

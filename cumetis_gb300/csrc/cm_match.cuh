@@ -176,6 +176,14 @@ __device__ __forceinline__ unsigned long long best_key(int v, int w) {
   return ((unsigned long long)((unsigned)w ^ 0x80000000u) << 32) | (unsigned)~(unsigned)v;
 }
 __device__ __forceinline__ int best_holder(unsigned long long b) { return b == 0ull ? -1 : (int)~(unsigned)b; }
+// Whether v and h hold each other's proposals, over entries of equal weight.  With
+// every pair so, no two vertices prefer each other to their partners, each by its
+// own row: v's proposal was refused for a better one, whose weight the row of the
+// vertex that refused holds too.  The matching is then that of mutual proposals,
+// whatever the other entries are.
+__device__ __forceinline__ bool best_mutual(unsigned long long bv, unsigned long long bh, int v) {
+  return best_holder(bh) == v && (bv >> 32) == (bh >> 32);
+}
 __device__ __forceinline__ unsigned long long ld_best(const MatchArgs &a, int k) { return ld_fresh(a.best + k); }
 
 // v's proposal (key) to c beats the proposal b that c holds.

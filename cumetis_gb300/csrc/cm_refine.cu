@@ -285,13 +285,14 @@ k_boundary_list(const int *__restrict__ flags, const int *__restrict__ target, i
 }
 
 // Prefix of every part's counts over the blocks (one warp a part), then by the
-// last block to finish: pstart[t], the exclusive prefix of the parts' totals, and
-// the parts' balance windows from the total vertex weight (Sum_maxmin_pwgts).
+// last block to finish: pstart[t], the exclusive prefix of the parts' totals, a
+// second count of the parts' weights (k_moves), and the parts' balance windows from
+// the total vertex weight (Sum_maxmin_pwgts).
 constexpr int kOffsetThreads = 256;
 __global__ void __launch_bounds__(kOffsetThreads)
 k_sort_offsets(const int *__restrict__ d_nb, int nparts, float tp, const int *__restrict__ pwgts,
                int *__restrict__ bhist, int *pcount, int *__restrict__ pstart, int *__restrict__ maxw,
-               int *__restrict__ minw, unsigned *done) {
+               int *__restrict__ minw, int *__restrict__ left, unsigned *done) {
   __shared__ int scan[kOffsetThreads / 32 + 1];
   __shared__ bool s_last;
   __shared__ unsigned long long s_tot;
@@ -326,6 +327,7 @@ k_sort_offsets(const int *__restrict__ d_nb, int nparts, float tp, const int *__
     const int ex = block_exclusive_scan<kOffsetThreads>(c, scan, &tot);
     if (t < nparts) {
       pstart[t] = carry + ex;
+      left[t] = pwgts[t];  // the moves' second count
       wt += pwgts[t];
     }
     carry += tot;
@@ -406,26 +408,52 @@ k_sort_scatter(const int *__restrict__ d_nb, const int *__restrict__ bnd_v, cons
 // by row length it takes 0.28 and 0.13), although most
 // stretches of a group are moved or refused as a whole.  So the block takes
 // kMoveThreads records at a time and settles them together when it can:
-//   - everyone moves: the weights leave their parts by atomics that return what
-//     was left; if every part stayed above its lower limit (and was not above
-//     its upper one before) and the sum fits part to, each vertex alone was
-//     allowed in order, for weights >= 0;
+//   - everyone moves: the records' weights are added up by part, in a table of the
+//     block; if every part stays above its lower limit (and was not above its upper
+//     one before) and the sum fits part to, each vertex alone was allowed in order,
+//     for weights >= 0;
 //   - everyone is refused: nobody fits as the weights are now, and refusals
 //     change no weight.
 // Else the first warp settles the records in order, 32 at a time, by stretches:
 // the longest prefix that moves, then the longest that is refused.  Either way
-// the outcome for two parts is that of the walk; with more parts the blocks
-// race as the reference's threads do, but a lower limit is never crossed, since
-// a weight that would cross it is put back.
-constexpr int kMoveThreads = 512;
+// the outcome for two parts is that of the walk.  With more parts the blocks race
+// as the reference's threads do, but no limit is crossed.  Weight is first taken
+// from a second count of the part (left), where it is put back if that falls below
+// the lower limit, and only then from its weight: pwgts never shows room that may
+// go again, and left never exceeds it.  Only the part's own block adds to it, after a
+// look at its weight, which the others can only lower.  A part that another block
+// took from first leaves its records to the walk.  (Compare-and-swap on pwgts alone
+// keeps the limits too, but 64 blocks that take from the same parts wait for one
+// another: projection and pass of a 1000 x 1000 grid in 64 parts 170 us.)
+constexpr int kMoveThreads = 512, kMoveSlots = 2 * kMoveThreads;
+
+// Takes w out of part p while it keeps at least lo; whether it did.  left: null
+// where no other block takes from the part, and the caller has looked already.
+__device__ __forceinline__ bool take_weight(int *pwgts, int *left, int p, int w, int lo) {
+  if (left && atomicSub(left + p, w) - w < lo) {
+    atomicAdd(left + p, w);
+    return false;
+  }
+  atomicSub(pwgts + p, w);
+  return true;
+}
+// Adds w to part p: to its weight first.
+__device__ __forceinline__ void give_weight(int *pwgts, int *left, int p, int w) {
+  atomicAdd(pwgts + p, w);
+  if (!left) return;
+  __threadfence();
+  atomicAdd(left + p, w);
+}
+
 template <bool kUp>
 __global__ void __launch_bounds__(kMoveThreads)
 k_moves(const int *__restrict__ pstart, const int4 *__restrict__ sorted, const int *__restrict__ maxw,
-        const int *__restrict__ minw, int *pwgts, int *where, unsigned long long *moves) {
+        const int *__restrict__ minw, int *pwgts, int *left, int *where, unsigned long long *moves) {
   __shared__ int4 s_rec[kMoveThreads];
-  __shared__ int s_warp[kMoveThreads / 32], s_sum, s_pto;
+  __shared__ int s_part[kMoveSlots], s_out[kMoveSlots];  // by slot: a source part, the weight that leaves it
+  __shared__ int s_sum, s_pto;
   const int to = blockIdx.x;
-  const bool racing = gridDim.x > 2;  // other blocks may take from the same parts
+  if (gridDim.x <= 2) left = nullptr;  // two parts: nobody else takes from the same part
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int tomax = maxw[to], tomin = minw[to];
   const int i0 = pstart[to], i1 = pstart[to + 1];
@@ -434,7 +462,7 @@ k_moves(const int *__restrict__ pstart, const int4 *__restrict__ sorted, const i
   const int4 none = make_int4(-1, 0, to, 0);
   int4 next = i0 + (int)threadIdx.x < i1 ? sorted[i0 + threadIdx.x] : none;
   for (int b = i0; b < i1; b += kMoveThreads) {
-    const int4 r = next;
+    int4 r = next;
     next = b + kMoveThreads + (int)threadIdx.x < i1 ? sorted[b + kMoveThreads + threadIdx.x] : none;
     const int me = r.z, vw = r.y;
     // me == to would add and remove the same weight: a no-op move, skipped
@@ -446,32 +474,55 @@ k_moves(const int *__restrict__ pstart, const int4 *__restrict__ sorted, const i
     const int lo = cand ? minw[me] : 0, hi = cand ? maxw[me] : 0;
     const bool fits = cand && pto + vw >= tomin && pto + vw <= tomax && pme - vw >= lo && pme - vw <= hi;
     if (!__syncthreads_or(fits)) continue;  // everyone is refused
-    const int total = __reduce_add_sync(0xffffffffu, cand ? vw : 0);
-    if (lane == 0) s_warp[warp] = total;
     const bool plain = !cand || (vw >= 0 && vw < (1 << 20) && fits && pme <= hi);
     if (__syncthreads_and(plain)) {
-      if (threadIdx.x == 0) {
-        int t = 0;
-        for (int w = 0; w < kMoveThreads / 32; ++w) t += s_warp[w];
-        s_sum = t;  // below 2^29
+      for (int i = threadIdx.x; i < kMoveSlots; i += kMoveThreads) {
+        s_part[i] = -1;
+        s_out[i] = 0;
       }
+      if (threadIdx.x == 0) s_sum = 0;
       __syncthreads();
-      const int sum = s_sum;
-      if ((long long)pto + sum <= tomax) {
-        const bool ok = !cand || atomicSub(&pwgts[me], vw) - vw >= lo;
-        if (__syncthreads_and(ok)) {
-          if (cand) {
-            where[r.x] = to;
-            ++nm;
-          }
-          if (threadIdx.x == 0) {
-            atomicAdd(&pwgts[to], sum);
-            __threadfence();
-          }
-          __syncthreads();
-          continue;
+      // The record's part's slot: at most kMoveThreads parts in twice as many slots.
+      // The records of a warp whose source is one part come together (with two parts
+      // all do).
+      int slot = me & (kMoveSlots - 1);
+      const int sum = __reduce_add_sync(0xffffffffu, cand ? vw : 0);  // below 2^29 for the whole block
+      const unsigned some = __ballot_sync(0xffffffffu, cand);
+      const int first = __ffs(some) - 1, part = __shfl_sync(0xffffffffu, me, first & 31);
+      const bool alike = __all_sync(0xffffffffu, !cand || me == part);
+      if (cand && (!alike || lane == first)) {
+        for (;;) {
+          const int p = atomicCAS(&s_part[slot], -1, me);
+          if (p == -1 || p == me) break;
+          slot = (slot + 1) & (kMoveSlots - 1);
         }
-        if (cand) atomicAdd(&pwgts[me], vw);
+        atomicAdd(&s_out[slot], alike ? sum : vw);
+      }
+      if (lane == first) atomicAdd(&s_sum, sum);
+      if (alike) slot = __shfl_sync(0xffffffffu, slot, first & 31);
+      __syncthreads();
+      bool room = (long long)pto + s_sum <= tomax;
+      for (int i = threadIdx.x; i < kMoveSlots; i += kMoveThreads)
+        if (s_part[i] >= 0) room = room && pw[s_part[i]] - s_out[i] >= minw[s_part[i]];
+      if (__syncthreads_and(room)) {
+        for (int i = threadIdx.x; i < kMoveSlots; i += kMoveThreads) {
+          if (s_part[i] >= 0 && !take_weight(pwgts, left, s_part[i], s_out[i], minw[s_part[i]])) {
+            atomicSub(&s_sum, s_out[i]);
+            s_out[i] = -1;  // another block came first
+          }
+        }
+        __syncthreads();
+        const bool moved = cand && s_out[slot] >= 0;
+        if (moved) {
+          where[r.x] = to;
+          ++nm;
+          r.z = to;  // settled
+        }
+        if (threadIdx.x == 0) {
+          give_weight(pwgts, left, to, s_sum);
+          __threadfence();
+        }
+        if (__syncthreads_and(!cand || moved)) continue;
       }
     }
     s_rec[threadIdx.x] = r;
@@ -480,16 +531,16 @@ k_moves(const int *__restrict__ pstart, const int4 *__restrict__ sorted, const i
     if (warp == 0) {
       for (int c = 0; c < kMoveThreads && b + c < i1; c += 32) {
         const int4 x = s_rec[c + lane];
-        unsigned left = __ballot_sync(0xffffffffu, kUp ? x.z < to : x.z > to);
-        while (left) {
-          const bool mine = left >> lane & 1u;
+        unsigned open = __ballot_sync(0xffffffffu, kUp ? x.z < to : x.z > to);
+        while (open) {
+          const bool mine = open >> lane & 1u;
           const int p = pw[to], q = mine ? pw[x.z] : 0;
           const int qlo = mine ? minw[x.z] : 0, qhi = mine ? maxw[x.z] : 0;
-          // weights before each vertex if all of `left` move
+          // weights before each vertex if all of `open` move
           int before = 0, gone = 0;
           for (int j = 0; j < 32; ++j) {
             const int wj = __shfl_sync(0xffffffffu, x.y, j), mj = __shfl_sync(0xffffffffu, x.z, j);
-            if ((left >> j & 1u) && j < lane) {
+            if ((open >> j & 1u) && j < lane) {
               before += wj;
               if (mj == x.z) gone += wj;
             }
@@ -497,27 +548,27 @@ k_moves(const int *__restrict__ pstart, const int4 *__restrict__ sorted, const i
           const int pt = p + before + x.y, pm = q - gone - x.y;
           const bool ok = pt >= tomin && pt <= tomax && pm >= qlo && pm <= qhi;
           const unsigned bad = __ballot_sync(0xffffffffu, mine && !ok);
-          const unsigned go = bad ? left & ((1u << (__ffs(bad) - 1)) - 1u) : left;
+          const unsigned go = bad ? open & ((1u << (__ffs(bad) - 1)) - 1u) : open;
           if (go) {
             bool moved = go >> lane & 1u;
-            if (moved && atomicSub(&pwgts[x.z], x.y) - x.y < qlo && racing && x.y > 0) {  // another block came first
-              atomicAdd(&pwgts[x.z], x.y);
-              moved = false;
+            if (moved) {
+              // (false: another block came first)
+              moved = take_weight(pwgts, left, x.z, x.y, x.y > 0 ? qlo : INT_MIN);
             }
             const int sum = __reduce_add_sync(0xffffffffu, moved ? x.y : 0);
-            if (lane == 0 && sum) atomicAdd(&pwgts[to], sum);
+            if (lane == 0 && sum) give_weight(pwgts, left, to, sum);
             if (moved) {
               where[x.x] = to;
               ++nm;
             }
-            left &= ~go;
+            open &= ~go;
             __threadfence();
             __syncwarp();
           } else {
             // the first is refused, and with it everyone up to the next that fits as things are
             const bool fit = mine && p + x.y >= tomin && p + x.y <= tomax && q - x.y >= qlo && q - x.y <= qhi;
-            const unsigned yes = __ballot_sync(0xffffffffu, fit) & ~(left & (0u - left));
-            left = yes ? left & ~((1u << (__ffs(yes) - 1)) - 1u) : 0u;
+            const unsigned yes = __ballot_sync(0xffffffffu, fit) & ~(open & (0u - open));
+            open = yes ? open & ~((1u << (__ffs(yes) - 1)) - 1u) : 0u;
           }
         }
       }
@@ -552,7 +603,7 @@ __global__ void k_cut(int n, const int *__restrict__ xadj, const int *__restrict
 }
 
 struct RefineWs {
-  int *pwgts, *maxw, *minw, *flag, *target, *bnd_v, *bnd_t, *bhist, *pcount, *pstart, *acc;
+  int *pwgts, *left, *maxw, *minw, *flag, *target, *bnd_v, *bnd_t, *bhist, *pcount, *pstart, *acc;
   int4 *sorted;  // boundary records (vertex, weight, part, 0) by target part
   unsigned long long *counters;  // [0] = moves, [1] = cut
   // cleared at the start of a pass, as one block: part weights, the list's
@@ -576,7 +627,7 @@ size_t clear_bytes(int64_t n, int nparts) {
 
 size_t refine_ws_bytes(cm_ctx *ctx, int64_t n, int nparts) {
   size_t b = 0;
-  b += (size_t)(2 * nparts + 2 * (nparts + 1)) * 4 + 5 * 256;
+  b += (size_t)(3 * nparts + 2 * (nparts + 1)) * 4 + 6 * 256;
   b += (size_t)(8 * n + 8) * 4 + 6 * 256;
   b += clear_bytes(n, nparts) + 256;
   if (nparts > kSmemParts) b += (size_t)grid_warps(ctx) * nparts * 4 + 256;
@@ -586,6 +637,7 @@ size_t refine_ws_bytes(cm_ctx *ctx, int64_t n, int nparts) {
 int take_refine_ws(cm_ctx *ctx, int64_t n, int nparts, RefineWs &w) {
   w.maxw = (int *)ws_take(ctx, (size_t)nparts * 4);
   w.minw = (int *)ws_take(ctx, (size_t)nparts * 4);
+  w.left = (int *)ws_take(ctx, (size_t)nparts * 4);
   w.pcount = (int *)ws_take(ctx, (size_t)(nparts + 1) * 4);
   w.pstart = (int *)ws_take(ctx, (size_t)(nparts + 1) * 4);
   w.flag = (int *)ws_take(ctx, (size_t)n * 4 + 4);
@@ -597,7 +649,7 @@ int take_refine_ws(cm_ctx *ctx, int64_t n, int nparts, RefineWs &w) {
   w.acc_ints = nparts > kSmemParts ? (size_t)grid_warps(ctx) * nparts : 0;
   w.acc = w.acc_ints ? (int *)ws_take(ctx, w.acc_ints * 4) : nullptr;
   w.counters = (unsigned long long *)ws_take(ctx, 64);
-  if (!w.maxw || !w.minw || !w.pcount || !w.pstart || !w.flag || !w.target || !w.bnd_v || !w.bnd_t || !w.sorted ||
+  if (!w.maxw || !w.minw || !w.left || !w.pcount || !w.pstart || !w.flag || !w.target || !w.bnd_v || !w.bnd_t || !w.sorted ||
       !w.clear || (w.acc_ints && !w.acc) || !w.counters)
     return cm_fail(CM_ERR_NOMEM, "refine: workspace too small");
   return CM_OK;
@@ -645,11 +697,13 @@ int refine_pass(cm_ctx *ctx, const cm_graph &g, int nparts, int32_t *where, Refi
   const int sort_blocks = (n + kSortBlock - 1) / kSortBlock;
   // tpwgts = 1.0 / nparts rounded to float, as cuMetis_set_graph_admin stores it (cu:384)
   k_sort_offsets<<<std::min(sms, (nparts + 7) / 8), kOffsetThreads, 0, s>>>(
-      w.nb, nparts, (float)(1.0 / nparts), w.pwgts, w.bhist, w.pcount, w.pstart, w.maxw, w.minw, w.done);
+      w.nb, nparts, (float)(1.0 / nparts), w.pwgts, w.bhist, w.pcount, w.pstart, w.maxw, w.minw, w.left, w.done);
   k_sort_scatter<<<sort_blocks, 32, nparts <= kSmemParts ? nparts * 4 : 0, s>>>(
       w.nb, w.bnd_v, w.bnd_t, nparts, w.bhist, w.pstart, g.vwgt, where, w.sorted);
-  k_moves<true><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, where, w.counters);
-  k_moves<false><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, where, w.counters);
+  k_moves<true><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, w.left, where,
+                                                w.counters);
+  k_moves<false><<<nparts, kMoveThreads, 0, s>>>(w.pstart, w.sorted, w.maxw, w.minw, w.pwgts, w.left, where,
+                                                 w.counters);
   ctx->launches += 8;
   return check_launch(ctx, "refine");
 }

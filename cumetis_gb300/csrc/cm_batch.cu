@@ -214,8 +214,7 @@ int BatchCoarsener::add(int32_t count, const cm_graph *graphs, const cm_coarsen_
       tvwgt += g.vwgt[v];
       maxdeg = std::max<int64_t>(maxdeg, (int64_t)g.xadj[v + 1] - g.xadj[v]);
     }
-    // maxvwgt = (int)(1.5 * tvwgt / Coarsen_threshold), cuMetis.cu:1828
-    a.h->maxvwgt = a.p.maxvwgt > 0 ? a.p.maxvwgt : (int32_t)(1.5 * (double)tvwgt / a.p.coarsen_to);
+    a.h->maxvwgt = a.p.maxvwgt > 0 ? a.p.maxvwgt : cm_weight_limit(tvwgt, a.p.coarsen_to);
     a.row_bound = 2 * maxdeg;
     if (n == 0) {  // nothing to coarsen: an empty coarse level, as cm_coarsen makes
       char *q = nullptr;

@@ -644,8 +644,7 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
     row_bound = 2 * maxdeg;
   }
   h->levels.push_back(L0);
-  // maxvwgt = (int)(1.5 * tvwgt / Coarsen_threshold), cuMetis.cu:1828
-  h->maxvwgt = params->maxvwgt > 0 ? params->maxvwgt : (int32_t)(1.5 * (double)tvwgt / params->coarsen_to);
+  h->maxvwgt = params->maxvwgt > 0 ? params->maxvwgt : cm_weight_limit(tvwgt, params->coarsen_to);
   int32_t *sizes = (int32_t *)ws_take(ctx, 64);
   const size_t level_ws_off = ctx->ws_used;
 

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
     }
     if (!level_barrier(A.bar, target, gridDim.x, st)) return;
     if (__ldcg(stats + 1) > kMatchChunk) return;  // the separate kernels' graph
-    if (A.derive_cap) a.maxvwgt = (int)(1.5 * (double)(long long)__ldcg(stats) / A.coarsen_to);
+    if (A.derive_cap) a.maxvwgt = cm_weight_limit((int64_t)__ldcg(stats), A.coarsen_to);
   }
   for (int level = 0;; ++level) {
     const int nb = min((int)gridDim.x, 1 + (n + m) / kLvWork);
@@ -515,7 +515,7 @@ int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaS
   if (measure) {
     long long stats[2];
     memcpy(stats, r->result + 2, sizeof stats);
-    if (p->maxvwgt <= 0) h->maxvwgt = (int32_t)(1.5 * (double)stats[0] / p->coarsen_to);
+    if (p->maxvwgt <= 0) h->maxvwgt = cm_weight_limit(stats[0], p->coarsen_to);
     *row_bound = 2 * stats[1];
   }
   if (*produced > 0) h->slabs.push_back(slab);

@@ -156,6 +156,7 @@ int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s) {
   Copies U;
   U.count = 0;
   U.first[0] = 0;
+  cudaError_t refused = cudaSuccess;
   auto flush = [&] {
     if (U.count == 0) return;
     const int parts = U.first[U.count];
@@ -166,18 +167,18 @@ int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s) {
   for (int i = 0; i < count; ++i) {
     if (a[i].bytes == 0) continue;
     bool copy = ((size_t)a[i].src & 3) != 0;  // the kernel moves whole words
-    if (!copy && a[i].bytes >= kPinnedCopyBytes) {
+    if (!copy) {
       cudaPointerAttributes at{};
       if (cudaPointerGetAttributes(&at, a[i].src) != cudaSuccess) cudaGetLastError();
-      else copy = at.type == cudaMemoryTypeHost;
+      else copy = at.type == cudaMemoryTypeDevice ||  // not the host's: as the copy call takes it
+                  (at.type == cudaMemoryTypeHost && a[i].bytes >= kPinnedCopyBytes);
     }
     if (copy) {
-      cudaMemcpyAsync(a[i].dst, a[i].src, a[i].bytes, cudaMemcpyHostToDevice, s);
+      const cudaError_t e = cudaMemcpyAsync(a[i].dst, a[i].src, a[i].bytes, cudaMemcpyHostToDevice, s);
+      if (e != cudaSuccess) refused = e;
       continue;
     }
-    const volatile char *c = (const volatile char *)a[i].src;
-    (void)c[0];  // a bad address fails here, on the host
-    (void)c[a[i].bytes - 1];
+    cm_touch_pages(a[i].src, a[i].bytes);
     U.src[U.count] = (const char *)a[i].src;
     U.dst[U.count] = (char *)a[i].dst;
     U.bytes[U.count] = a[i].bytes;
@@ -185,6 +186,10 @@ int upload_arrays(cm_ctx *ctx, const HostArray *a, int count, cudaStream_t s) {
     if (++U.count == kPieces) flush();
   }
   flush();
+  if (refused != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_status(refused, "upload");
+  }
   return check_launch(ctx, "upload");
 }
 

@@ -24,6 +24,8 @@
 #include <utility>
 #include <vector>
 
+#include <unistd.h>
+
 #ifdef _OPENMP
 #include <omp.h>
 #endif
@@ -87,6 +89,14 @@ void radix_sort_u64(std::vector<uint64_t> &a, int bits) {
 }
 
 }  // namespace
+
+void cm_touch_pages(const void *p, size_t bytes) {
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  if (bytes == 0) return;
+  const volatile char *c = (const volatile char *)p;
+  for (size_t at = 0; at < bytes; at += page) (void)c[at];
+  (void)c[bytes - 1];
+}
 
 int cm_fail(int code, const char *fmt, ...) {
   va_list ap;

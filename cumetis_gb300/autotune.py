@@ -8,11 +8,11 @@ contraction sorts in one-warp batches and its chunk size, the block shapes of
 their kernels, the resident blocks per SM each size-class shape is compiled
 for).  The search is coordinate descent from the current tuning file (or
 the compiled-in defaults): for each parameter in turn every other candidate
-value is built as a library variant (only the source it belongs to is
+value is built as a library variant (only the sources that read the macro are
 recompiled), timed with bench.py in a fresh process on the same workload,
 and kept when it is at least --min-gain faster than the incumbent.  The
-winner must then pass a parity subset of the GPU tests before the tuning
-file is written; `build()` compiles it in from then on.  Needs a GPU.
+winner must then pass a subset of the GPU tests, on the kernels of whole levels
+and on the separate ones, before the tuning file is written; `build()` compiles it in from then on.  Needs a GPU.
 """
 import argparse
 import json
@@ -25,7 +25,8 @@ from . import build as B
 
 ROOT = os.path.dirname(B.HERE)
 
-# (macro, compiled-in default, candidates, source it belongs to)
+# (macro, compiled-in default, candidates, source it belongs to; a macro that a header
+# reads reaches the header's other sources too, build.variant_defines)
 PARAMS = [
     ("CM_SERIAL_DEG", 16, [8, 16], "cm_match.cu"),          # rows scanned by one lane (warp-per-vertex threshold)
     ("CM_MATCH_CHUNK", 256, [128, 256, 512], "cm_match.cu"),  # entries per warp work item
@@ -40,7 +41,9 @@ PARAMS = [
 ]
 DEFAULTS = {name: d for name, d, _, _ in PARAMS}
 SOURCE = {name: src for name, _, _, src in PARAMS}
-CHECK_TESTS = "test_long_rows or test_contract_bitexact or test_coarsen_hierarchy or test_match_bitexact_synthetic"
+CHECK_FILES = ["tests/test_parity_gpu.py", "tests/test_levels_gpu.py", "tests/test_match_paths_gpu.py"]
+CHECK_TESTS = ("test_long_rows or test_contract_bitexact or test_coarsen_hierarchy or test_match_bitexact_synthetic"
+               " or test_levels_equal_the_separate_kernels or test_rows_at_the_scan_boundaries")
 
 
 def valid(cfg):
@@ -129,7 +132,7 @@ def main(argv=None):
     cfg, best, trials = search(start, measure, args.min_gain)
     lib = os.path.join(variant_dir(cfg), "libcm.so")
     if not args.no_check:
-        r = subprocess.run([sys.executable, "-m", "pytest", "tests/test_parity_gpu.py", "-x", "-q", "-k", CHECK_TESTS],
+        r = subprocess.run([sys.executable, "-m", "pytest", *CHECK_FILES, "-x", "-q", "-k", CHECK_TESTS],
                            env=dict(os.environ, CUMETIS_LIB=lib), cwd=ROOT, stdout=subprocess.PIPE,
                            stderr=subprocess.STDOUT, text=True)
         if r.returncode != 0:

@@ -12,6 +12,7 @@ import concurrent.futures as cf
 import hashlib
 import json
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -115,10 +116,36 @@ def build(force=False, verbose=False):
     return LIB
 
 
+def _headers(src):
+    """Names of the headers that a source of CSRC includes, also through others."""
+    seen, todo = set(), [src]
+    while todo:
+        with open(os.path.join(CSRC, todo.pop())) as f:
+            found = re.findall(r'^\s*#include "([^"/]+)"', f.read(), re.M)
+        todo += [h for h in found if h not in seen and os.path.exists(os.path.join(CSRC, h))]
+        seen.update(found)
+    return seen
+
+
+def variant_defines(defines_by_source):
+    """The flags of every source of a variant: a macro that a header reads goes to
+    all sources that include that header, so that no two parts of one library are
+    built with different values."""
+    out = {k: list(v) for k, v in defines_by_source.items()}
+    flags = {d for v in defines_by_source.values() for d in v}
+    for f in CU_SOURCES:
+        headers = [h for h in _headers(f) if os.path.exists(os.path.join(CSRC, h))]
+        text = "\n".join(open(os.path.join(CSRC, h)).read() for h in headers)
+        for d in flags:
+            if d not in out.get(f, []) and re.search(r"\b%s\b" % d[2:].split("=")[0], text):
+                out.setdefault(f, []).append(d)
+    return {k: sorted(v) for k, v in out.items()}
+
+
 def build_variant(defines_by_source, out_dir):
     """Builds a libcm.so variant into out_dir: each CUDA source compiled with
-    its own -D flags (defines_by_source: {"cm_match.cu": ["-DCM_X=1"], ...};
-    sources not named get none), linked with the main build's C++ objects.
+    its own -D flags (defines_by_source: {"cm_match.cu": ["-DCM_X=1"], ...},
+    completed by variant_defines), linked with the main build's C++ objects.
     Objects are cached under _build/variants by source and flags, so a
     variant that changes one source recompiles only that one.  Returns the
     library path."""
@@ -128,10 +155,11 @@ def build_variant(defines_by_source, out_dir):
     os.makedirs(cache, exist_ok=True)
     os.makedirs(out_dir, exist_ok=True)
     deps = _deps()
+    defines = variant_defines(defines_by_source)
     jobs, objs = [], []
     for f in CU_SOURCES:
         src = os.path.join(CSRC, f)
-        defs = list(defines_by_source.get(f, []))
+        defs = defines.get(f, [])
         key = hashlib.sha1((f + "|" + " ".join(defs)).encode()).hexdigest()[:16]
         obj = os.path.join(cache, "%s.%s.o" % (f, key))
         objs.append(obj)

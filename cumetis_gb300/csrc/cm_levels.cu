@@ -420,7 +420,7 @@ bool fused_fits(const cm_ctx *ctx, int64_t n, int64_t m, int64_t max_deg, int32_
 
 int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaStream_t s, int *produced, int *stopped,
                  int64_t *row_bound, bool measure) {
-  static_assert(kFusedWork <= 1 << kCountBits, "packed scan");
+  static_assert(kFusedWork < 1 << kCountBits, "packed scan: counts of isolated vertices, too, stay below 2^kCountBits");
   *produced = 0;
   *stopped = 0;
   const cm_level F = h->levels.back();

@@ -30,8 +30,7 @@
 // one warp per row moves the entries to their final place.
 #include <algorithm>
 
-// Rows of at most CM_TINY_MAX expanded entries are sorted many per warp (a
-// tuning parameter, set through the build).
+// The rows' header's limit of tiny rows, which the tuner searches as this source's.
 #ifndef CM_TINY_MAX
 #define CM_TINY_MAX 64
 #endif

@@ -47,8 +47,7 @@
 
 #include <algorithm>
 
-// Rows of at most kSerialDeg entries are scanned by one lane, longer rows in
-// kMatchChunk-entry warp work items (tuning parameters, set through the build).
+// The header's row thresholds, which the tuner searches as this source's.
 #ifndef CM_SERIAL_DEG
 #define CM_SERIAL_DEG 16
 #endif
@@ -588,8 +587,7 @@ int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, 
   MatchArgs a;
   a.n = n;
   a.xadj = g->xadj; a.adjncy = g->adjncy; a.adjwgt = g->adjwgt; a.vwgt = g->vwgt;
-  a.maxvwgt = maxvwgt;  // with graphs side by side: the smallest cap (it gates the all-eligible first round)
-  a.mode = mode;
+  a.maxvwgt = maxvwgt;  // with graphs side by side: the smallest cap (all_eligible)
   a.m2 = d_match;
   a.vgid = vgid;
   a.gbase = gbase;

@@ -7,8 +7,7 @@
 #include "cm_ctx.h"
 
 // Rows of at most kSerialDeg entries are scanned by one lane, longer rows in
-// kMatchChunk-entry warp work items (tuning parameters,
-// set through the build; cm_match.cu).
+// kMatchChunk-entry warp work items (tuning parameters, set through the build).
 #ifndef CM_SERIAL_DEG
 #define CM_SERIAL_DEG 16
 #endif
@@ -35,7 +34,6 @@ struct MatchArgs {
   int n, span;                   // span: vertices a warp takes at a time (multiple of 32, at most kSpan)
   const int *xadj, *adjncy, *adjwgt, *vwgt;
   long long maxvwgt;
-  int mode;
   int *m2;                       // the matching (output)
   unsigned long long *best;      // best proposal received: (weight, proposer), 0 = none (best_key)
   int *top, *topw;               // kTop listed candidates per vertex: ids, weights

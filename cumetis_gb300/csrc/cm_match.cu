@@ -276,8 +276,7 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
       if (!grid_barrier(st, gridDim.x)) return;
     } else {
       __threadfence();
-      __syncthreads();
-      if (ld_relaxed(&st->error) != 0) return;
+      if (__syncthreads_or(ld_relaxed(&st->error) != 0)) return;  // one answer for the block
     }
   }
   if (first_thread) st->rounds = round;
@@ -289,44 +288,104 @@ __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_rounds
 // pair forms.  Every unmatched vertex points at its most preferred unmatched
 // neighbour, and vertices that point at each other are matched; whichever pairs
 // are matched first, the outcome is the same.  Rounds over a list of the vertices
-// that have to point anew (at first all), in three phases:
-//   point   the first unmatched of the vertex's listed candidates, or of its row;
+// that have to point anew (at first all):
+//   point   the first unmatched of the vertex's listed candidates; with none left a
+//           lane scans a row of up to kSerialDeg entries, longer rows are queued;
+//   scan    the queued rows, by chunks, a new list for each;
 //   commit  the pairs;
 //   wake    neighbours that point at a vertex matched now go on the next list.
-// A vertex is woken through the matched one's row, so it can be missed where its own
-// entry has no counterpart: when the list is empty, one pass over all vertices
-// finds those.  The work is that of the rows looked at, not rounds times vertices:
-// a path in order takes n / 2 rounds of a few vertices each.  At most 2 n + 4
-// rounds: all but every second match a pair.
-// Over the warps gw, gw + nw, ...; barrier() separates the phases and returns false
-// to give up.  What other warps write is read fresh.
-template <bool H, typename B>
-__device__ void handshake_rounds(const MatchArgs &a, int gw, int nw, B barrier) {
+// A vertex is woken through the matched one's row, of up to kMatchChunk entries while
+// lists are short and up to kSerialDeg (a lane each) while they are long.  It is missed
+// where that row is longer or its own entry has no counterpart: a pass over all
+// vertices finds those, in the round after such a row, in every kPassRounds-th (else
+// chains that wait for a vertex run one after another: a 1000 x 1000 grid without 0.1%
+// of its entries 162 ms, so 43) and when the list is empty.  The work is that of the rows looked at, not rounds times vertices: a
+// path in order takes n / 2 rounds of a few vertices each.  Latency: three barriers a
+// round, four with queued rows, each phase some dependent trips to L2.  At most
+// 4 n + 8 rounds: of any four before the last one matches a pair.
+// With GRID all blocks work together (a cooperative launch), and block 0 goes on alone,
+// with block barriers, while lists are short (kSoloEntries; the others wait at a grid
+// barrier, for kSoloRounds at most); else the calling block is the only one.
+// wbuf: the warp's 32 int2 of shared memory.  What other warps write is read fresh.
+constexpr int kSoloEntries = 1024, kSoloRounds = 4096, kPassRounds = 6;
+constexpr int kSoloPass = 16384;  // vertices that one block passes over
+template <bool H, bool GRID>
+__device__ void handshake_rounds(const MatchArgs &a, int2 *wbuf) {
   constexpr unsigned full = 0xffffffffu;
+  constexpr int kHalf = 8;
   const int lane = threadIdx.x & 31, n = a.n;
   const unsigned below = (1u << lane) - 1u;
-  // the proposals' scratch is free: targets, the round of the last listing, the lists
-  int *ptr = a.slot[0].big_base, *stamp = a.slot[0].big_done, *count = a.odd + 2;  // count[3], by round
-  int *lists[2] = {reinterpret_cast<int *>(a.slot[0].desc), reinterpret_cast<int *>(a.slot[1].desc)};
-  const long long step = (long long)nw * 32;
-  for (long long v = (long long)gw * 32 + lane; v < n; v += step) {
+  // the proposals' scratch is free: targets, the round of the last listing, the
+  // lists; slot 1 for the queued rows
+  int *ptr = reinterpret_cast<int *>(a.best), *stamp = ptr + n;
+  int *lists[2] = {reinterpret_cast<int *>(a.slot[0].desc), reinterpret_cast<int *>(a.slot[0].desc) + n};
+  int *count = a.odd + 2, *search = a.odd + 5;  // [3] each, by round: the list's length, a pass over all is due
+  int *solo_end = a.odd + 8;  // the round in which block 0 has stopped to work alone
+  const Slot &S = a.slot[1];
+  const int block_warps = (int)(blockDim.x >> 5), warp = (int)(threadIdx.x >> 5);
+  int gw = warp, nw = block_warps;
+  if (GRID) {
+    gw += (int)blockIdx.x * block_warps;
+    nw *= (int)gridDim.x;
+  }
+  bool solo = !GRID;
+  int alone = 0;  // rounds of block 0 alone
+  auto barrier = [&]() -> bool {
+    if (!solo) return grid_barrier(a.st, gridDim.x);
+    __threadfence();
+    return !__syncthreads_or(ld_relaxed(&a.st->error) != 0);  // one answer for the block
+  };
+  for (long long v = (long long)gw * 32 + lane, step = (long long)nw * 32; v < n; v += step) {
     a.m2[v] = -1;
-    ptr[v] = -1;
+    ptr[v] = kNone;
     stamp[v] = 0;
     lists[0][v] = (int)v;
   }
   if (gw == 0 && lane == 0) {
     count[0] = n;
     count[1] = count[2] = 0;
+    search[0] = search[1] = search[2] = 0;
+    a.big[0] = 0;
+    a.tick[0] = 0;
   }
   if (!barrier()) return;
-  bool searched = false;  // the last round was a pass over all vertices
+  bool searched = false;  // the last round only made a pass over all vertices
   for (int round = 0;; ++round) {
     const int k = ld_fresh(count + round % 3);
+    const bool pass = k == 0 || ld_fresh(search + round % 3) != 0 || round % kPassRounds == kPassRounds - 1;
+    if (GRID) {
+      const bool small = k > 0 && k <= kSoloEntries && (!pass || n <= kSoloPass);
+      if (!solo && small) {  // all have read the counters before block 0 goes on
+        if (!barrier()) return;
+        if (blockIdx.x != 0) {
+          if (!barrier()) return;
+          round = ld_fresh(solo_end) - 1;
+          searched = false;
+          continue;
+        }
+        solo = true;
+        gw = warp;
+        nw = block_warps;
+        alone = 0;
+      } else if (solo && (!small || alone > kSoloRounds)) {
+        if (threadIdx.x == 0) *solo_end = round;
+        solo = false;
+        nw = block_warps * (int)gridDim.x;
+        if (!barrier()) return;
+        --round;  // this round, together
+        continue;
+      }
+      alone += 1;
+    }
+    const long long step = (long long)nw * 32;
     const int *list = lists[round & 1];
     int *more = lists[~round & 1], *nmore = count + (round + 1) % 3;
-    if (gw == 0 && lane == 0) count[(round + 2) % 3] = 0;
-    if ((long long)round > 2ll * n + 4) {
+    if (gw == 0 && lane == 0) {
+      count[(round + 2) % 3] = 0;
+      search[(round + 2) % 3] = 0;
+    }
+    if (k == 0 && searched) break;
+    if ((long long)round > 4ll * n + 8) {
       if (gw == 0 && lane == 0) record_error(a.st, CM_ERR_LIMIT, ERR_SITE_ROUNDS);
       return;
     }
@@ -338,59 +397,108 @@ __device__ void handshake_rounds(const MatchArgs &a, int gw, int nw, B barrier) 
       base = __shfl_sync(full, base, 0);
       if (take) more[base + __popc(who & below)] = v;
     };
-    if (k == 0) {
-      if (searched) break;
+    if (pass) {  // those whose target is matched, unless they point anew in this round
       for (long long b = (long long)gw * 32; b < n; b += step) {
         const long long v = b + lane;
         bool stale = false;
-        if (v < n && ld_fresh(a.m2 + v) < 0) {
+        if (v < n && ld_fresh(a.m2 + v) < 0 && ld_fresh(stamp + v) != round) {
           const int p = ld_fresh(ptr + v);
           stale = p >= 0 && ld_fresh(a.m2 + p) >= 0;
         }
         if (stale) stamp[v] = round + 1;
         append(stale, (int)v);
       }
-      searched = true;
+    }
+    searched = k == 0;
+    if (searched) {
       if (!barrier()) return;
       continue;
     }
-    searched = false;
+    // entries of the list a warp takes at a time: few where there are few
+    const int per = (int)min(32ll, max(1ll, ((long long)k + nw - 1) / nw));
+    const long long stride = (long long)nw * per;
+    const int wake_deg = k <= n >> 6 ? kMatchChunk : kSerialDeg;  // longest row that wakes
 
     // ---- point
-    for (long long b = (long long)gw * 32; b < k; b += step) {
-      const int v = b + lane < k ? ld_fresh(list + b + lane) : -1;
-      int p = kNone;
-      if (v >= 0 && a.xadj[v + 1] > a.xadj[v]) {
-        const int4 q = reinterpret_cast<const int4 *>(a.top)[v];
+    for (long long b = (long long)gw * per; b < k; b += stride) {
+      const int v = lane < per && b + lane < k ? ld_fresh(list + b + lane) : -1;
+      int p = kNone, xs = 0, deg = 0;
+      if (v >= 0) {
+        xs = a.xadj[v];
+        deg = a.xadj[v + 1] - xs;
+      }
+      if (deg > 0) {
+        const int4 q = __ldcg(reinterpret_cast<const int4 *>(a.top) + v);
         const int c[kTop] = {q.x, q.y, q.z, q.w};
         p = kUnknown;
 #pragma unroll
-        for (int t = kTop - 1; t >= 0; --t) {
-          if (c[t] < 0) p = c[t];
-          else if (ld_fresh(a.m2 + c[t]) < 0) p = c[t];
-        }
+        for (int t = kTop - 1; t >= 0; --t)
+          if (c[t] < 0 || ld_fresh(a.m2 + c[t]) < 0) p = c[t];
       }
-      unsigned rows = __ballot_sync(full, p == kUnknown);  // lists used up: the whole row
-      while (rows) {
-        const int src = __ffs(rows) - 1;
-        rows &= rows - 1;
-        const int x = __shfl_sync(full, v, src), hb = hash_base(a, x);
-        const long long vw = a.vwgt[x], cap = weight_cap(a, x);
+      const bool queue = p == kUnknown && deg > kSerialDeg;
+      if (p == kUnknown && !queue) {
+        const int hb = hash_base(a, v);
+        const long long vw = a.vwgt[v], cap = weight_cap(a, v);
         Cand<H> best;
-        for (int j = a.xadj[x] + lane; j < a.xadj[x + 1]; j += 32) {
-          const int y = a.adjncy[j];
-          if (y == x || ld_fresh(a.m2 + y) >= 0 || !pair_fits(cap, vw, a.vwgt[y])) continue;
-          const Cand<H> e = Cand<H>::make(x, y, a.adjwgt[j], hb);
-          if (e.better(best)) best = e;
+        for (int j = 0; j < deg; j += kHalf) {  // 8 entries in flight
+          int y[kHalf], w[kHalf], yw[kHalf], ym[kHalf];
+#pragma unroll
+          for (int t = 0; t < kHalf; ++t) {
+            y[t] = j + t < deg ? a.adjncy[xs + j + t] : v;
+            w[t] = j + t < deg ? a.adjwgt[xs + j + t] : 0;
+          }
+#pragma unroll
+          for (int t = 0; t < kHalf; ++t) {
+            yw[t] = a.vwgt[y[t]];
+            ym[t] = y[t] != v ? ld_fresh(a.m2 + y[t]) : 0;
+          }
+#pragma unroll
+          for (int t = 0; t < kHalf; ++t) {
+            if (ym[t] >= 0 || !pair_fits(cap, vw, yw[t])) continue;
+            const Cand<H> e = Cand<H>::make(v, y[t], w[t], hb);
+            if (e.better(best)) best = e;
+          }
         }
-        const int id = best.warp_best().id();
-        if (lane == src) p = id;
+        p = best.id();
       }
-      if (v >= 0) ptr[v] = p;
+      append_scan(a, 1, 0, queue, v, xs, deg);
+      if (v >= 0 && !queue) ptr[v] = p;
     }
     if (!barrier()) return;
 
+    // ---- scan
+    const int nchunks = (int)(ld_fresh(a.big) & 0xffffffffu);
+    alone += nchunks / 32;  // (their time)
+    if (nchunks > 0) {
+      for (;;) {
+        int q = 0;
+        if (lane == 0) q = atomicAdd(a.tick, 1);
+        q = __shfl_sync(full, q, 0);
+        if (q >= nchunks) break;
+        const int4 d = __ldcg(S.desc + q);
+        TopK<H, kTop> r = chunk_best<H, kTop, kOpen>(a, d.x, d.y, d.z, false, wbuf);
+        bool mine = true;
+        if (d.w >= 0) {
+          const int nch = (a.xadj[d.x + 1] - a.xadj[d.x] + kMatchChunk - 1) / kMatchChunk;
+          mine = part_done<H, kTop>(a, S, q, d, nch, r);
+          if (mine) {
+            const int base = ld_fresh(S.big_base + d.w);
+            r = merge_parts<H, kTop>(a, nch * kTop, [&](int t) { return (size_t)base * kTop + t; });
+          }
+        }
+        if (mine && lane == 0) {
+          store_top(a, d.x, r);
+          ptr[d.x] = r.c[0].id();
+        }
+      }
+      if (!barrier()) return;
+    }
+
     // ---- commit (by either end that is listed: the same words)
+    if (gw == 0 && lane == 0) {
+      a.big[0] = 0;
+      a.tick[0] = 0;
+    }
     for (long long i = (long long)gw * 32 + lane; i < k; i += step) {
       const int v = ld_fresh(list + i), p = ld_fresh(ptr + v);
       if (p >= 0 && ld_fresh(ptr + p) == v) {
@@ -401,30 +509,52 @@ __device__ void handshake_rounds(const MatchArgs &a, int gw, int nw, B barrier) 
     if (!barrier()) return;
 
     // ---- wake
-    for (long long b = (long long)gw * 32; b < k; b += step) {
-      const int v = b + lane < k ? ld_fresh(list + b + lane) : -1;
+    for (long long b = (long long)gw * per; b < k; b += stride) {
+      const int v = lane < per && b + lane < k ? ld_fresh(list + b + lane) : -1;
       const int u = v >= 0 ? ld_fresh(a.m2 + v) : -1;
-      const bool both = u >= 0 && ld_fresh(stamp + u) != round;  // u is not listed: its row is left to v
-      const unsigned other = __ballot_sync(full, both);
-      unsigned rows = __ballot_sync(full, u >= 0);
-      while (rows) {
-        const int src = __ffs(rows) - 1;
-        rows &= rows - 1;
-        for (int end = 0; end < 1 + (int)(other >> src & 1u); ++end) {
-          const int x = __shfl_sync(full, end ? u : v, src);
-          const int xe = a.xadj[x + 1];
-          for (int j0 = a.xadj[x]; j0 < xe; j0 += 32) {
-            const int y = j0 + lane < xe ? a.adjncy[j0 + lane] : -1;
-            const bool wake = y >= 0 && ld_fresh(ptr + y) == x && ld_fresh(a.m2 + y) < 0 &&
-                              atomicExch(stamp + y, round + 1) != round + 1;  // a row can name y twice
-            append(wake, y);
+      // v's row, and u's where u is not listed
+      int xx[2] = {u >= 0 ? v : -1, u >= 0 && ld_fresh(stamp + u) != round ? u : -1}, xxs[2], xdeg[2];
+#pragma unroll
+      for (int end = 0; end < 2; ++end) {
+        xxs[end] = xx[end] >= 0 ? a.xadj[xx[end]] : 0;
+        xdeg[end] = xx[end] >= 0 ? a.xadj[xx[end] + 1] - xxs[end] : 0;
+      }
+      // (the stamp: once on a list, though a row may name a vertex twice)
+      auto listed = [&](int y) { return atomicExch(stamp + y, round + 1) == round + 1; };
+#pragma unroll 1
+      for (int end = 0; end < 2; ++end) {
+        const int x = end ? xx[1] : xx[0], xs = end ? xxs[1] : xxs[0], deg = end ? xdeg[1] : xdeg[0];
+        if (deg > wake_deg) search[(round + 1) % 3] = 1;
+        for (int j = 0; deg <= kSerialDeg && j < deg; j += kHalf) {
+          int y[kHalf];
+          bool waits[kHalf];
+#pragma unroll
+          for (int t = 0; t < kHalf; ++t) y[t] = j + t < deg ? a.adjncy[xs + j + t] : x;
+#pragma unroll
+          for (int t = 0; t < kHalf; ++t) {
+            const int yp = ld_fresh(ptr + y[t]), ym = ld_fresh(a.m2 + y[t]);
+            waits[t] = yp == x && ym < 0;  // (x is matched)
+          }
+#pragma unroll
+          for (int t = 0; t < kHalf; ++t)
+            if (waits[t] && !listed(y[t])) more[atomicAdd(nmore, 1)] = y[t];
+        }
+        unsigned rows = __ballot_sync(full, deg > kSerialDeg && deg <= wake_deg);
+        while (rows) {
+          const int src = __ffs(rows) - 1;
+          rows &= rows - 1;
+          const int on = __shfl_sync(full, x, src), s0 = __shfl_sync(full, xs, src), e0 = s0 + __shfl_sync(full, deg, src);
+          for (int j0 = s0; j0 < e0; j0 += 32) {
+            const int y = j0 + lane < e0 ? a.adjncy[j0 + lane] : on;
+            const int yp = ld_fresh(ptr + y), ym = ld_fresh(a.m2 + y);
+            append(yp == on && ym < 0 && !listed(y), y);
           }
         }
       }
     }
     if (!barrier()) return;
   }
-  for (long long v = (long long)gw * 32 + lane; v < n; v += step)
+  for (long long v = (long long)gw * 32 + lane, step = (long long)nw * 32; v < n; v += step)
     if (ld_fresh(a.m2 + v) < 0) a.m2[v] = (int)v;
 }
 
@@ -449,19 +579,16 @@ __global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int 
   if (threadIdx.x == 0) s_last = atomicAdd(a.odd + 1, 1) == (int)gridDim.x - 1;
   __syncthreads();
   if (!s_last || __ldcg(a.odd) == 0) return;
-  handshake_rounds<H>(a, threadIdx.x >> 5, blockDim.x >> 5, [&] {
-    __threadfence();
-    __syncthreads();
-    return true;
-  });
+  __shared__ int2 sh_q[kPrepThreads / 32][32];
+  handshake_rounds<H, false>(a, sh_q[threadIdx.x >> 5]);
 }
 
 // The same for large graphs, with every resident block.
 template <bool H>
 __global__ void __launch_bounds__(kMatchThreads, kMatchMinBlocks) k_match_handshake(MatchArgs a) {
   if (__ldcg(a.odd) == 0) return;
-  handshake_rounds<H>(a, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), (int)((gridDim.x * blockDim.x) >> 5),
-                      [&] { return grid_barrier(a.st, gridDim.x); });
+  __shared__ int2 sh_q[kMatchThreads / 32][32];
+  handshake_rounds<H, true>(a, sh_q[threadIdx.x >> 5]);
 }
 
 // ---------------------------------------------------------------------------
@@ -549,10 +676,11 @@ size_t match_ws_bytes(int64_t n, int64_t m) {
   return b + 64 * 256;
 }
 
-// Graphs above this many vertices + entries get the handshake kernel with
-// every block behind k_match_finish (a launch that returns at once costs a few
-// us, under 5% there); below it the last block of k_match_finish does the work.
-constexpr int64_t kAloneWork = 1 << 21;
+// Graphs above this many vertices + entries get the handshake kernel behind
+// k_match_finish (a launch that returns at once costs 3 us); below it, where that
+// kernel would be one block, the last block of k_match_finish does the work (a grid of
+// 900 vertices 50 instead of 55 us).
+constexpr int64_t kAloneWork = kWorkPerBlock;
 
 int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, int32_t *d_match, cudaStream_t s,
                  const int32_t *vgid, const int32_t *gbase, const int32_t *gcap, int64_t max_deg) {

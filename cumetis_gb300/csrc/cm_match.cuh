@@ -41,7 +41,7 @@ struct MatchArgs {
   unsigned long long *big;       // [3] = (rows << 32 | chunks) of the slots, by round
   int *tick;                     // [3] work tickets of the round kernel, by round
   int *vmax;                     // largest vertex weight (zeroed before the launch)
-  int *odd;                      // [5]: an offer was not returned; blocks of k_match_finish done; handshakes' list lengths
+  int *odd;                      // [8]: an offer was not returned; blocks of k_match_finish done; handshake_rounds' counters
   int *part;                     // per chunk: kTop x (w, h, k)
   long long max_rounds;
   DevStatus *st;
@@ -263,8 +263,9 @@ __device__ __forceinline__ TopK<H, KK> merge_parts(const MatchArgs &a, int cnt, 
 // b + lane + 32 u, all loads issued before any is used, and marks with
 // k[u] = -1 those that are no candidates: the vertex itself, pairs that do not
 // fit (`all`: every pair fits), and neighbours that hold a proposal v cannot
-// beat: by its weight alone (kWeak), or at all (kExact).
-enum : int { kStatic = 0, kWeak = 1, kExact = 2 };
+// beat: by its weight alone (kWeak), or at all (kExact); or those matched (kOpen,
+// for the handshakes).
+enum : int { kStatic = 0, kWeak = 1, kExact = 2, kOpen = 3 };
 template <bool H, int FILTER>
 __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, int e, bool all, int hb,
                                              int (&k)[kMatchChunk / 32], int (&w)[kMatchChunk / 32]) {
@@ -298,6 +299,14 @@ __device__ __forceinline__ void load_entries(const MatchArgs &a, int v, int b, i
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (((unsigned)w[u] ^ 0x80000000u) < bw[u]) k[u] = -1;
+  }
+  if constexpr (FILTER == kOpen) {
+    int mk[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) mk[u] = (u < nu && k[u] >= 0) ? ld_fresh(a.m2 + k[u]) : 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (mk[u] >= 0) k[u] = -1;
   }
   if constexpr (FILTER == kExact) {
     unsigned long long bk[U];
@@ -335,9 +344,9 @@ constexpr int kLaneRefusals = kSerialDeg + kTop, kWarpRefusals = kMatchChunk + k
 #endif
 constexpr unsigned kChainSteps = CM_CHAIN_STEPS;
 
-// The warp's best KK candidates over entries [b, e), e - b <= 64, of v's row,
-// with FILTER among those that v beats the proposal of; every lane gets the list.
-template <bool H, int KK, bool FILTER>
+// The warp's best KK candidates over entries [b, e), e - b <= 64, of v's row, among
+// those that FILTER leaves (kWeak: as kExact); every lane gets the list.
+template <bool H, int KK, int FILTER>
 __device__ __forceinline__ TopK<H, KK> pair_best(const MatchArgs &a, int v, int b, int e, bool all, int hb) {
   const int lane = threadIdx.x & 31, j0 = b + lane, j1 = j0 + 32;
   int k0 = -1, k1 = -1, w0 = 0, w1 = 0;
@@ -357,7 +366,10 @@ __device__ __forceinline__ TopK<H, KK> pair_best(const MatchArgs &a, int v, int 
     if (!pair_fits(cap, vw, x0)) k0 = -1;
     if (!pair_fits(cap, vw, x1)) k1 = -1;
   }
-  if (FILTER) {
+  if (FILTER == kOpen) {
+    if (k0 >= 0 && ld_fresh(a.m2 + k0) >= 0) k0 = -1;
+    if (k1 >= 0 && ld_fresh(a.m2 + k1) >= 0) k1 = -1;
+  } else if (FILTER != kStatic) {
     const unsigned long long y0 = k0 >= 0 ? ld_best(a, k0) : 0ull, y1 = k1 >= 0 ? ld_best(a, k1) : 0ull;
     if (k0 >= 0 && !beats<H>(best_key(v, w0), y0, v, k0, hb)) k0 = -1;
     if (k1 >= 0 && !beats<H>(best_key(v, w1), y1, v, k1, hb)) k1 = -1;
@@ -404,7 +416,7 @@ __device__ __forceinline__ TopK<H, KK> chunk_best(const MatchArgs &a, int v, int
   const int hb = hash_base(a, v);
   // Rows and last chunks of up to 64 entries (most of a skewed graph's): two
   // entries a lane, every one compared in full, against a proposal too.
-  if (nu <= 2) return pair_best<H, KK, FILTER != kStatic>(a, v, b, e, all, hb);
+  if (nu <= 2) return pair_best<H, KK, FILTER>(a, v, b, e, all, hb);
   int k[U], w[U];
   load_entries<H, FILTER>(a, v, b, e, all, hb, k, w);
   if constexpr (!H) {

@@ -653,13 +653,14 @@ extern "C" int cm_coarsen(cm_ctx *ctx, const cm_graph *g, int input_on_device, c
   int32_t *sizes = (int32_t *)ws_take(ctx, 64);
   const size_t level_ws_off = ctx->ws_used;
 
+  bool odd = false;  // a level was not symmetric: the separate kernels from there on
   for (;;) {
     cm_level &F = h->levels.back();
     const int64_t n = F.g.nvtxs, m = F.g.nedges;
-    if (measure || fused_fits(ctx, n, m, row_bound / 2, params->match_mode)) {
+    if (measure || (!odd && fused_fits(ctx, n, m, row_bound / 2, params->match_mode))) {
       int produced = 0, stopped = 0;
       ctx->ws_used = level_ws_off;
-      if ((rc = launch_fused(ctx, h, params, s, &produced, &stopped, &row_bound, measure))) return fail(rc);
+      if ((rc = launch_fused(ctx, h, params, s, &produced, &stopped, &row_bound, measure, &odd))) return fail(rc);
       measure = false;
       if (stopped) break;
       if (produced > 0) continue;

@@ -186,8 +186,9 @@ int launch_contract(cm_ctx *ctx, const cm_graph *fine, const int32_t *match, int
 // with 0.6 M, 1198 with 1.2 M, 1191 with 2 M; a 101^3 grid 2571, 2498, 2456, 2445;
 // larger graphs fill the chip in every kernel anyway).  launch_fused coarsens
 // h->levels.back() by the params' rules as far as the kernel can, appends the
-// levels (*produced; *stopped = 1 when the stop rule ended the coarsening) and
-// updates *row_bound; it waits for the stream.
+// levels (*produced; *stopped = 1 when the stop rule ended the coarsening; *odd: it
+// ended before a level that is not symmetric, and the next will hardly be) and updates
+// *row_bound; it waits for the stream.
 #ifndef CM_FUSED_WORK
 #define CM_FUSED_WORK 1200000
 #endif
@@ -198,7 +199,7 @@ size_t fused_ws_bytes(int64_t n, int64_t m);
 // (where the parameters leave it open) the hierarchy's maxvwgt are set.
 bool fused_fits(const cm_ctx *ctx, int64_t n, int64_t m, int64_t max_deg, int32_t mode);
 int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaStream_t s, int *produced, int *stopped,
-                 int64_t *row_bound, bool measure);
+                 int64_t *row_bound, bool measure, bool *odd);
 
 }  // namespace cm
 

@@ -49,6 +49,10 @@ constexpr int kLvItems = 8, kMaxRow = 32 * kLvItems;  // longest expanded row: o
 // a barrier.  A level with a longer chain is left to the separate kernels, where
 // nobody waits for it.
 constexpr unsigned kFusedSteps = 1u << 18;
+// Why a level is not handled: a row of more than kMatchChunk entries; an adjacency
+// that is not symmetric, or a long chain.  The levels behind an odd one are most likely
+// odd too and are not tried.
+enum : int { kRowTooLong = 1, kOdd = 2 };
 constexpr int kMaxFused = 64;                         // levels of one launch
 constexpr int kCountBits = 21;                        // vertices and entries stay below 2^21 (packed scan)
 static_assert(kTinyMax < kMaxRow, "row lengths");
@@ -71,10 +75,10 @@ struct LevelArgs {
   int4 *row_meta;
   int2 *cplace, *stage;
   unsigned long long *sums;  // [2][gridDim.x]: the blocks' vertices, the blocks' coarse entries
-  int *flags;                // [kMaxFused][4]: not handled, longest expanded row, longer rows, -
+  int *flags;                // [kMaxFused][4]: not handled (kRowTooLong, kOdd), longest expanded row, longer rows, -
   unsigned *bar;             // barrier arrivals
   FusedLevel *out;           // [kMaxFused]
-  int *result;               // [0] levels produced, [1] 1 if the stop rule ended the coarsening
+  int *result;               // [0] levels produced, [1] 1 if the stop rule ended the coarsening, [6] kOdd: see there
   // First level not measured yet: take the sum of its weights and its longest row
   // into result[2..5] and, with derive_cap, the weight limit from them.
   int measure, derive_cap;
@@ -238,9 +242,10 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
         if (lane == 0) store_top(a, x, r);
       }
     }
-    if (unfit) flags[0] = 1;
+    if (unfit) flags[0] = kRowTooLong;
     if (!level_barrier(A.bar, target, nb, st)) return;
     if (__ldcg(flags) != 0) return;
+    unfit = false;
 
     // ---- proposals
     unsigned steps = kFusedSteps;
@@ -286,11 +291,15 @@ __global__ void __launch_bounds__(kLvThreads, 1) k_levels(LevelArgs A) {
       if (threadIdx.x == 0) A.sums[blockIdx.x] = total;
       longest = __reduce_max_sync(0xffffffffu, longest);
       if (lane == 0 && longest > 0) atomicMax(flags + 1, longest);
-      if (unfit) flags[0] = 1;
+      if (unfit) flags[0] = kOdd;
     }
     if (!level_barrier(A.bar, target, nb, st)) return;
     const int longest = __ldcg(flags + 1);
-    if (__ldcg(flags) != 0 || longest > kMaxRow) return;
+    const int odd = __ldcg(flags);
+    if (odd != 0 || longest > kMaxRow) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) A.result[6] = odd;
+      return;
+    }
 
     // ---- vertices
     unsigned long long total;
@@ -419,7 +428,7 @@ bool fused_fits(const cm_ctx *ctx, int64_t n, int64_t m, int64_t max_deg, int32_
 }
 
 int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaStream_t s, int *produced, int *stopped,
-                 int64_t *row_bound, bool measure) {
+                 int64_t *row_bound, bool measure, bool *odd) {
   static_assert(kFusedWork < 1 << kCountBits, "packed scan: counts of isolated vertices, too, stay below 2^kCountBits");
   *produced = 0;
   *stopped = 0;
@@ -512,6 +521,7 @@ int launch_fused(cm_ctx *ctx, cm_hierarchy *h, const cm_coarsen_params *p, cudaS
   }
   *produced = r->result[0];
   *stopped = r->result[1];
+  *odd = r->result[6] == kOdd;
   if (measure) {
     long long stats[2];
     memcpy(stats, r->result + 2, sizeof stats);

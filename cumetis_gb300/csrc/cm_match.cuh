@@ -739,6 +739,7 @@ __device__ __forceinline__ ChainEnd propose_span(const MatchArgs &a, long long b
       --*steps;
     }
     const unsigned idle = __ballot_sync(0xffffffffu, cur < 0);
+    const bool first = taken == 0;
     if (taken < cnt && idle) {
       const int at = taken + __popc(idle & below);
       if (cur < 0 && at < cnt) {
@@ -749,6 +750,15 @@ __device__ __forceinline__ ChainEnd propose_span(const MatchArgs &a, long long b
       taken += __popc(idle);
     } else if (idle == 0xffffffffu) {
       break;
+    }
+    if (first) {
+      // A hub's leaves all want the hub: of a warp's first vertices only the best offers
+      // itself, the others are refused by it or with it (a star of 1 M leaves: the
+      // matching 171 -> 143 us with ties to the lower id, 243 -> 200 with hashed ones).
+      const int c = cur >= 0 ? L.id[0] : kNone, hub = __shfl_sync(0xffffffffu, c, 0);
+      if (__all_sync(0xffffffffu, c >= 0 && c == hub) &&
+          Cand<H>::make(hub, cur, L.w[0], hb).warp_best().id() != cur)
+        L.drop();
     }
     int qv = -1, qx = 0, qdeg = 0;
     if (cur >= 0) {

@@ -13,6 +13,10 @@
 // traffic per vertex: match (4 B), xadj (4 B), vwgt (4 B) read; cmap (4 B)
 // written; leader/cvwgt/eoff (12 B per coarse vertex) written.  Bound by latency
 // on all but the largest graphs (three dependent trips and the look-back).
+//
+// A vertex whose partner is out of range or does not point back is reported and taken
+// as a singleton: whatever the array holds, every vertex gets a coarse id and every
+// row is counted once, so the contraction stays within its arrays.
 #include "cm_ctx.h"
 
 namespace cm {
@@ -78,7 +82,11 @@ k_cmap(int n, const int *__restrict__ xadj, const int *__restrict__ vwgt, const 
     const long long v = wbase + it * 32 + lane;
     dv[it] -= xv[it];
     du[it] -= xu[it];
-    bad |= v < n && back[it] != (int)v;  // not an involution
+    if (v < n && back[it] != (int)v) {  // not an involution: a singleton too
+      bad = true;
+      u[it] = (int)v;
+      du[it] = 0;
+    }
     unsigned long long val = 0;
     if (v < n && v <= u[it]) val = (1ull << 31) | (unsigned long long)(dv[it] + du[it]);
     const unsigned long long x = warp_inclusive_scan_u64(val);

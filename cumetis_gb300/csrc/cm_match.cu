@@ -558,10 +558,11 @@ __device__ void handshake_rounds(const MatchArgs &a, int2 *wbuf) {
     if (ld_fresh(a.m2 + v) < 0) a.m2[v] = (int)v;
 }
 
-// match[v] from best[]; a proposal that is not returned alike sets odd[0].  With
-// `alone` the last block then computes the matching by handshakes itself.
-template <bool H>
-__global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int alone) {
+// match[v] from best[]; a proposal that is not returned alike sets odd[0].  With ALONE
+// the last block then computes the matching by handshakes itself (a form of its own:
+// the registers of that cost the large graphs' kernel occupancy, R-MAT 22 14 -> 31 us).
+template <bool H, bool ALONE>
+__global__ void __launch_bounds__(kPrepThreads, ALONE ? 0 : 8) k_match_finish(MatchArgs a) {
   bool odd = false;
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < a.n;
        v += (long long)gridDim.x * blockDim.x) {
@@ -572,15 +573,17 @@ __global__ void __launch_bounds__(kPrepThreads) k_match_finish(MatchArgs a, int 
     odd |= h >= 0 && !mutual;
   }
   if (odd) atomicOr(a.odd, 1);
-  if (!alone) return;
-  __threadfence();
-  __syncthreads();
-  __shared__ int s_last;
-  if (threadIdx.x == 0) s_last = atomicAdd(a.odd + 1, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (!s_last || __ldcg(a.odd) == 0) return;
-  __shared__ int2 sh_q[kPrepThreads / 32][32];
-  handshake_rounds<H, false>(a, sh_q[threadIdx.x >> 5]);
+  if constexpr (ALONE) {
+    __shared__ int s_last;
+    __shared__ int2 sh_q[kPrepThreads / 32][32];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(a.odd + 1, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (ld_fresh(a.odd) != 0) handshake_rounds<H, false>(a, sh_q[threadIdx.x >> 5]);
+  }
 }
 
 // The same for large graphs, with every resident block.
@@ -799,8 +802,13 @@ int launch_match(cm_ctx *ctx, const cm_graph *g, int32_t maxvwgt, int32_t mode, 
     ctx->launches++;
   }
   const unsigned vgrid = (unsigned)std::min<int64_t>((int64_t)ctx->num_sms * 8, n / kPrepThreads + 1);
-  if (hash) k_match_finish<true><<<vgrid, kPrepThreads, 0, s>>>(a, alone);
-  else k_match_finish<false><<<vgrid, kPrepThreads, 0, s>>>(a, alone);
+  if (alone) {
+    if (hash) k_match_finish<true, true><<<vgrid, kPrepThreads, 0, s>>>(a);
+    else k_match_finish<false, true><<<vgrid, kPrepThreads, 0, s>>>(a);
+  } else {
+    if (hash) k_match_finish<true, false><<<vgrid, kPrepThreads, 0, s>>>(a);
+    else k_match_finish<false, false><<<vgrid, kPrepThreads, 0, s>>>(a);
+  }
   ctx->launches++;
   if (e == cudaSuccess && !alone) {
     e = cudaLaunchCooperativeKernel(hfn, dim3(grid), dim3(kMatchThreads), args, 0, s);

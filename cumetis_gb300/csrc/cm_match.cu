@@ -329,7 +329,7 @@ __device__ void handshake_rounds(const MatchArgs &a, int2 *wbuf) {
     nw *= (int)gridDim.x;
   }
   bool solo = !GRID;
-  int alone = 0;  // rounds of block 0 alone
+  int alone = 0;  // rounds of block 0 alone, weighted by what a warp has in them: up to 30 us a unit
   auto barrier = [&]() -> bool {
     if (!solo) return grid_barrier(a.st, gridDim.x);
     __threadfence();
@@ -417,6 +417,7 @@ __device__ void handshake_rounds(const MatchArgs &a, int2 *wbuf) {
     // entries of the list a warp takes at a time: few where there are few
     const int per = (int)min(32ll, max(1ll, ((long long)k + nw - 1) / nw));
     const long long stride = (long long)nw * per;
+    alone += per;  // (a warp's rows one after another)
     const int wake_deg = k <= n >> 6 ? kMatchChunk : kSerialDeg;  // longest row that wakes
 
     // ---- point
@@ -468,7 +469,7 @@ __device__ void handshake_rounds(const MatchArgs &a, int2 *wbuf) {
 
     // ---- scan
     const int nchunks = (int)(ld_fresh(a.big) & 0xffffffffu);
-    alone += nchunks / 32;  // (their time)
+    alone += nchunks / 32;
     if (nchunks > 0) {
       for (;;) {
         int q = 0;
